@@ -173,6 +173,13 @@ __device__ __forceinline__ float rcbrt_nr(float x) {
   const float e = fmaf(-x, y * y * y, 1.0f);
   return fmaf(y * (1.0f / 3.0f), e, y);
 }
+// x^(-1/2): the third-order step y0 (1 + e/2 + 3 e^2 / 8), e = 1 - x y0^2.
+__device__ __forceinline__ double rsqrt_nr(double x) {
+  if (!(x > 1e-37 && x < 1e37)) return 1.0 / sqrt(x);
+  const double y = (double)ptx_rsqrt_approx((float)x);
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y, e * fma(e, 0.375, 0.5), y);
+}
 // sqrt(x) for x >= 0: one Newton step on y = 1/sqrt(x),
 // y <- y (3 - x y^2) / 2 (relative error ~2^-44), then s = x y and one
 // Newton step on s itself with the exact residual x - s^2 (an FMA),

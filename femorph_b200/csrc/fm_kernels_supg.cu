@@ -11,6 +11,8 @@
 // keeps the values compute_pressure sees (it runs before the zeroing).
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "fm_device.cuh"
 #include "fm_supg.cuh"
 
@@ -48,13 +50,16 @@ __device__ __forceinline__ void check_exit(const DevBatch& B, const DevProb& P, 
   if (status != FM_OK) B.pstate[pidx].status = status;
 }
 
-// MIXED: Gauss-point work in FP32 (supg_element_mixed).  All 128-thread
-// kernels are held to 168 registers a thread so that three CTAs fit an SM
-// (FP64 tet4: a small spill, 12% faster than two CTAs at 241 registers;
-// FP64 hexa8 with the stored geometry: ~500 bytes of spill, faster than two
-// CTAs at 255 registers, while forming the geometry in the kernel it spilled
-// 1 KB at three CTAs and ran 30% slower; mixed hexa8 with the stored
-// geometry: no spill, and 2% faster than four CTAs at 128 registers).
+// MIXED: Gauss-point work in FP32 (supg_element_mixed).  HISTORY: the batch
+// carries AB2 rates; without them the kernel holds fewer registers (mixed
+// tet4 154 -> 126, which lets four CTAs an SM run: 88 -> 80 us a step on
+// 663,552 tets), the arithmetic is the same.  The other 128-thread kernels
+// are held to 168 registers a thread so that three CTAs fit an SM: they are
+// bound by the latency of their FP64 chains and shared-memory reads, and
+// the spills this costs (FP64 tet4 24 bytes, hexa8 112) cost less than the
+// third CTA's warps bring (FP64 hexa8 at two CTAs and 255 registers 0.482,
+// at three with its coefficients in shared memory 0.438 ms; tet4 at four
+// CTAs 0.170, at three 0.164 ms).
 //
 // Accumulation of the element contributions into the tile's nodes, in the
 // order of the elements (colour-sorted) in both schemes, so both give the
@@ -71,23 +76,25 @@ __device__ __forceinline__ void check_exit(const DevBatch& B, const DevProb& P, 
 // from the geometry stored at placement (supg_geo_kernel; FP64, or rounded
 // to FP32 for the mixed form) instead of forming them from the staged
 // coordinates at every step, and stage no coordinates.
-template <int NPE, int THREADS, bool MIXED>
-__global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1)
+template <int NPE, int THREADS, bool MIXED, bool HISTORY>
+__global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED && !HISTORY ? 4 : 3) : 1)
     supg_tile_kernel(DevBatch B, int tn_max, int inc_max) {
   constexpr bool GATHER = NPE == 4;
   constexpr bool GEO = NPE == 8;
   extern __shared__ double sm[];
-  double* s_x = sm;
-  double* s_y = s_x + tn_max;
-  double* s_z = s_y + tn_max;
-  double* s_u = s_z + tn_max;
+  double* s_x = sm;  // coordinates: tet4 only
+  double* s_y = s_x + (GEO ? 0 : tn_max);
+  double* s_z = s_y + (GEO ? 0 : tn_max);
+  double* s_u = s_z + (GEO ? 0 : tn_max);
   double* s_v = s_u + tn_max;
   double* s_w = s_v + tn_max;
   double* s_a0 = s_w + tn_max;
   double* s_a1 = s_a0 + tn_max;
   double* s_a2 = s_a1 + tn_max;
-  double* R = s_a2 + tn_max;                                        // GATHER: [NPE * 3][THREADS]
-  int32_t* s_col = (int32_t*)(R + (GATHER ? NPE * 3 * THREADS : 0));  // colour offsets (<= 129)
+  // GATHER: [NPE * 3][THREADS] staged entries; hexa8: each thread's own
+  // column (supg_stage_doubles)
+  double* R = s_a2 + tn_max;
+  int32_t* s_col = (int32_t*)(R + supg_stage_doubles(NPE, MIXED, THREADS));  // colour offsets (<= 129)
   uint16_t* s_inc = (uint16_t*)(s_col + 130);                      // GATHER: incidence entries
   uint16_t* s_off = s_inc + (GATHER ? inc_max : 0);                // GATHER: per-node offsets
   uint16_t* s_cur = s_off + (GATHER ? tn_max + 1 : 0);             // GATHER: per-node cursors
@@ -101,7 +108,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1)
   if (st.iter >= B.target[pidx] || st.status != FM_OK) return;
   const DevProb& P = B.probs[pidx];
   const bool euler = (P.ex_mask & 1) || st.iter == 0;
-  const bool ab2 = !(P.ex_mask & 1);
+  const bool ab2 = HISTORY && !(P.ex_mask & 1);
   const int tid = threadIdx.x;
   for (int ln = tid; ln < tm.n_node; ln += THREADS) {
     const int g = B.tile_nodes[tm.node_begin + ln];
@@ -123,8 +130,10 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1)
     const int ninc = tm.n_elem * NPE;
     for (int i = tid; i < ninc; i += THREADS) s_inc[i] = B.tile_inc[tm.inc_begin + i];
   }
-  fill_shape_table<NPE, double>(&s_shape);
-  if (MIXED) fill_shape_table<NPE, float>(&s_shape_f);
+  if constexpr (MIXED) {
+    fill_shape_table<NPE, double>(&s_shape);
+    fill_shape_table<NPE, float>(&s_shape_f);
+  }
   __syncthreads();
   const int64_t E = B.E;
   // one lane asks L2 for a later tile's connectivity, incidence entries, AB2
@@ -154,18 +163,41 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1)
     }
   }
   int c_lo = 0;
+  using ConnRow = typename std::conditional<NPE == 4, uint2, uint4>::type;
+  const ConnRow* conn_g = reinterpret_cast<const ConnRow*>(B.conn) + tm.elem_begin;
+  // hexa8: the stored geometry of element le of this tile
+  using GeoT = typename std::conditional<MIXED, float, double>::type;
+  using Geo = typename std::conditional<MIXED, GeoStream32<THREADS>, GeoStream64<THREADS>>::type;
+  const bool bbar = (P.ex_mask & 2) != 0;
+  const int geo_passes = bbar ? 2 : 1;
+  auto geo_of = [&](int le) -> Geo {
+    const GeoT* g = MIXED ? reinterpret_cast<const GeoT*>(B.geo32) : reinterpret_cast<const GeoT*>(B.geo);
+    return Geo{reinterpret_cast<GeoT*>(R + (MIXED ? 0 : 24 * THREADS)) + tid, g + tm.elem_begin + le, E, geo_passes};
+  };
+  // corner ids loaded a chunk ahead (not in the mixed hexa8 kernel, where the
+  // four registers cost more, 0.0752 -> 0.0790 ms, than the wait for them)
+  constexpr bool AHEAD = !MIXED;
+  ConnRow next = {};
+  if (tid < tm.n_elem) {
+    if constexpr (AHEAD) next = __ldg(conn_g + tid);
+    if constexpr (GEO) geo_of(tid).start();
+  }
   for (int base = 0; base < tm.n_elem; base += THREADS) {
     const int le = base + tid;
     const bool active = le < tm.n_elem;
     double k[NPE][3];
     int ln[NPE];
+    ConnRow cw = next;
+    if constexpr (AHEAD) {
+      if (le + THREADS < tm.n_elem) next = __ldg(conn_g + le + THREADS);
+    } else {
+      if (active) cw = __ldg(conn_g + le);
+    }
     if (active) {
       const int64_t e = tm.elem_begin + le;
-      if (NPE == 4) {
-        const uint2 cw = __ldg(reinterpret_cast<const uint2*>(B.conn) + e);
+      if constexpr (NPE == 4) {
         ln[0] = cw.x & 0xffff; ln[1] = cw.x >> 16; ln[2] = cw.y & 0xffff; ln[3] = cw.y >> 16;
       } else {
-        const uint4 cw = __ldg(reinterpret_cast<const uint4*>(B.conn) + e);
         ln[0] = cw.x & 0xffff; ln[1] = cw.x >> 16; ln[2] = cw.y & 0xffff; ln[3] = cw.y >> 16;
         ln[4 % NPE] = cw.z & 0xffff; ln[5 % NPE] = cw.z >> 16; ln[6 % NPE] = cw.w & 0xffff; ln[7 % NPE] = cw.w >> 16;
       }
@@ -189,24 +221,45 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1)
         for (int a = 0; a < NPE; ++a) {
           Ud[a][0] = (float)(s_u[ln[a]] - u0); Ud[a][1] = (float)(s_v[ln[a]] - v0); Ud[a][2] = (float)(s_w[ln[a]] - w0);
         }
-        supg_element_mixed<NPE, GEO>(P, s_shape_f, s_shape, Xr, U0, Ud, precise, s_x, s_y, s_z, ln, k, lam, reg,
-                                     GEO ? B.geo32 + e : nullptr, E);
+        supg_element_mixed<NPE>(P, s_shape_f, s_shape, Xr, U0, Ud, precise, s_x, s_y, s_z, ln, k, lam, reg, geo_of(le));
       } else {
-        supg_element<NPE, GEO>(P, s_shape, s_x, s_y, s_z, s_u, s_v, s_w, ln, k, lam, reg, GEO ? B.geo + e : nullptr, E);
+        if constexpr (NPE == 4)
+          supg_element_tet(P, s_x, s_y, s_z, s_u, s_v, s_w, ln, k, lam, reg);
+        else if (bbar)
+          supg_element_hexa<THREADS, true>(P, s_u, s_v, s_w, ln, R + tid, k, lam, reg, geo_of(le));
+        else
+          supg_element_hexa<THREADS, false>(P, s_u, s_v, s_w, ln, R + tid, k, lam, reg, geo_of(le));
       }
       B.el_lam[e] = lam;
       B.el_reg[e] = reg;
       if (ab2) {
+        // four nodes' old rates are loaded before their new ones are stored:
+        // a load behind the store of another row would wait for it (the
+        // compiler cannot know that the rows differ)
+        double* h = B.sdus + e;
 #pragma unroll
-        for (int a = 0; a < NPE; ++a)
+        for (int a0 = 0; a0 < NPE; a0 += 4) {
+          double old[4][3];
+          if (!euler) {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            double* h = B.sdus + (int64_t)(a * 3 + c) * E + e;
-            const double kp = k[a][c];
-            if (!euler) k[a][c] = (3.0 / 2.0) * kp - (1.0 / 2.0) * __ldcs(h);
-            __stcs(h, kp);
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+              for (int c = 0; c < 3; ++c) old[a][c] = __ldcs(h + (int64_t)((a0 + a) * 3 + c) * E);
           }
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const double kp = k[a0 + a][c];
+              if (!euler) k[a0 + a][c] = (3.0 / 2.0) * kp - (1.0 / 2.0) * old[a][c];
+              __stcs(h + (int64_t)((a0 + a) * 3 + c) * E, kp);
+            }
+        }
       }
+    }
+    if constexpr (GEO) {
+      // the next chunk's first points on their way while this one is added up
+      if (le + THREADS < tm.n_elem) geo_of(le + THREADS).start();
     }
     if constexpr (GATHER) {
       // the barrier that frees R (owners of the previous chunk done) comes
@@ -435,9 +488,9 @@ __global__ void supg_pressure_kernel(DevBatch B, int tn_max, double* pres) {
   }
 }
 
-size_t supg_smem_bytes(int tn_max, int inc_max, int npe, int threads) {
+size_t supg_smem_bytes(int tn_max, int inc_max, int npe, int threads, bool mixed) {
   const bool gather = npe == 4;
-  return (size_t)tn_max * 9 * sizeof(double) + (gather ? (size_t)npe * 3 * threads * sizeof(double) : 0) +
+  return ((size_t)tn_max * (npe == 4 ? 9 : 6) + supg_stage_doubles(npe, mixed, threads)) * sizeof(double) +
          130 * sizeof(int32_t) + (gather ? ((size_t)inc_max + 2 * (size_t)tn_max + 1) * sizeof(uint16_t) : 0);
 }
 
@@ -451,6 +504,26 @@ static cudaError_t raise_dyn_smem(K k, int optin) {
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
 }
 
+// The launch's tile kernel: the AB2 code is only in the kernels of batches
+// that carry a history (it costs the others registers).
+template <int NPE>
+static decltype(&supg_tile_kernel<NPE, 128, false, false>) supg_tile(bool mixed, int threads, bool history) {
+  if (threads == 256) {
+    if (mixed) return history ? supg_tile_kernel<NPE, 256, true, true> : supg_tile_kernel<NPE, 256, true, false>;
+    return history ? supg_tile_kernel<NPE, 256, false, true> : supg_tile_kernel<NPE, 256, false, false>;
+  }
+  if (mixed) return history ? supg_tile_kernel<NPE, 128, true, true> : supg_tile_kernel<NPE, 128, true, false>;
+  return history ? supg_tile_kernel<NPE, 128, false, true> : supg_tile_kernel<NPE, 128, false, false>;
+}
+
+template <int NPE>
+static cudaError_t raise_tile_smem(int optin) {
+  cudaError_t e = cudaSuccess;
+  for (int v = 0; v < 8 && e == cudaSuccess; ++v)
+    e = raise_dyn_smem(supg_tile<NPE>((v & 1) != 0, (v & 2) ? 256 : 128, (v & 4) != 0), optin);
+  return e;
+}
+
 // Raises the kernels' dynamic shared-memory limit to the device's opt-in
 // maximum (the attribute is per kernel and process-wide, so a batch with
 // small tiles must not lower it below what another batch launches with; the
@@ -462,43 +535,24 @@ cudaError_t supg_configure(size_t smem, int npe) {
   if (e != cudaSuccess) return e;
   (void)smem;  // checked against the limit by the caller
   if (npe == 4) {
-    e = raise_dyn_smem(supg_tile_kernel<4, 128, false>, optin);
-    if (e == cudaSuccess) e = raise_dyn_smem(supg_tile_kernel<4, 256, false>, optin);
-    if (e == cudaSuccess) e = raise_dyn_smem(supg_tile_kernel<4, 128, true>, optin);
-    if (e == cudaSuccess) e = raise_dyn_smem(supg_tile_kernel<4, 256, true>, optin);
+    e = raise_tile_smem<4>(optin);
     if (e == cudaSuccess) e = raise_dyn_smem(supg_pressure_kernel<4>, optin);
     if (e == cudaSuccess) e = raise_dyn_smem(supg_stats_kernel<4>, optin);
   } else {
-    e = raise_dyn_smem(supg_geo_kernel, optin);
-    if (e == cudaSuccess) e = raise_dyn_smem(supg_tile_kernel<8, 128, false>, optin);
-    if (e == cudaSuccess) e = raise_dyn_smem(supg_tile_kernel<8, 256, false>, optin);
-    if (e == cudaSuccess) e = raise_dyn_smem(supg_tile_kernel<8, 128, true>, optin);
-    if (e == cudaSuccess) e = raise_dyn_smem(supg_tile_kernel<8, 256, true>, optin);
+    e = raise_tile_smem<8>(optin);
+    if (e == cudaSuccess) e = raise_dyn_smem(supg_geo_kernel, optin);
     if (e == cudaSuccess) e = raise_dyn_smem(supg_pressure_kernel<8>, optin);
     if (e == cudaSuccess) e = raise_dyn_smem(supg_stats_kernel<8>, optin);
   }
   return e;
 }
 
-template <int NPE, bool MIXED>
-static void launch_supg_tile(const DevBatch& B, int tn_max, int inc_max, int threads, size_t smem, cudaStream_t s) {
-  if (threads == 256)
-    supg_tile_kernel<NPE, 256, MIXED><<<B.n_tiles, 256, smem, s>>>(B, tn_max, inc_max);
-  else
-    supg_tile_kernel<NPE, 128, MIXED><<<B.n_tiles, 128, smem, s>>>(B, tn_max, inc_max);
-}
-
 cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int inc_max, int threads, int iface_blocks, int npe,
                              bool mixed, bool xpack, cudaStream_t s, cudaEvent_t* ev) {
-  const size_t smem = supg_smem_bytes(tn_max, inc_max, npe, threads);
+  const size_t smem = supg_smem_bytes(tn_max, inc_max, npe, threads, mixed);
   if (ev) cudaEventRecord(ev[0], s);
-  if (npe == 4) {
-    if (mixed) launch_supg_tile<4, true>(B, tn_max, inc_max, threads, smem, s);
-    else launch_supg_tile<4, false>(B, tn_max, inc_max, threads, smem, s);
-  } else {
-    if (mixed) launch_supg_tile<8, true>(B, tn_max, inc_max, threads, smem, s);
-    else launch_supg_tile<8, false>(B, tn_max, inc_max, threads, smem, s);
-  }
+  auto k = npe == 4 ? supg_tile<4>(mixed, threads, B.sdus != nullptr) : supg_tile<8>(mixed, threads, B.sdus != nullptr);
+  k<<<B.n_tiles, threads == 256 ? 256 : 128, smem, s>>>(B, tn_max, inc_max);
   if (ev) cudaEventRecord(ev[1], s);
   if (xpack)
     supg_xpack_kernel<<<iface_blocks, 256, 0, s>>>(B);

@@ -39,7 +39,7 @@ cudaError_t launch_vms_xupdate(const DevBatch& B, int blocks, cudaStream_t s);
 cudaError_t launch_vms_diagnostics(const DevBatch& B, const double* cres_buf, const int32_t* off, const int32_t* ent,
                                    int32_t n_nodes, const int32_t* eo, int64_t eb, int64_t ec, int64_t nb,
                                    double* el, double* out, int blocks, cudaStream_t s);
-size_t supg_smem_bytes(int tn_max, int inc_max, int npe, int threads);
+size_t supg_smem_bytes(int tn_max, int inc_max, int npe, int threads, bool mixed);
 cudaError_t supg_configure(size_t smem, int npe);
 cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int inc_max, int threads, int iface_blocks, int npe, bool mixed,
                              bool xpack, cudaStream_t s, cudaEvent_t* ev);
@@ -464,7 +464,7 @@ static int configure(fm_batch* b) {
   if (b->tn_max <= b->configured_tn && b->inc_max <= b->configured_inc) return FM_OK;
   const int tn = std::max(b->tn_max, b->configured_tn), inc = std::max(b->inc_max, b->configured_inc);
   size_t smem = b->solver == FM_SOLVER_VMS ? vms_smem_bytes(tn, inc, b->threads, b->precision == FM_MIXED)
-                                           : supg_smem_bytes(tn, inc, b->npe, b->threads);
+                                           : supg_smem_bytes(tn, inc, b->npe, b->threads, b->precision == FM_MIXED);
   // 227 KB opt-in limit per block, less room for the kernels' static shared memory
   if (smem + 1024 > 227 * 1024) return fail(FM_ERR_INVALID, "tile too large for shared memory; lower tile_nodes");
   cudaError_t ce = b->solver == FM_SOLVER_VMS ? vms_configure(tn, inc) : supg_configure(smem, b->npe);

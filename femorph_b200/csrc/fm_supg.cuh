@@ -142,360 +142,513 @@ __device__ __forceinline__ double jacobian(const double dN[NPE][3], const double
   return jacobian_at<NPE>([&](int n, int a) { return dN[n][a]; }, sx, sy, sz, ln, inv);
 }
 
-// Per Gauss point (per element for tet4): G = J^-T J^-1
-// (femElement.cpp:192-232), the G:G term of tau, (mu/rho)^2 cI G:G
-// (eval_stabilization, src lines 336-377), and G's cofactor inverse
-// (eval_bulk_modulus, src lines 382-441).
-__device__ __forceinline__ void tet_metric(const double inv[3][3], double nu, double cI, double G[3][3], double& t3,
-                                           double iG[3][3]) {
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) G[a][b] = inv[0][a] * inv[0][b] + inv[1][a] * inv[1][b] + inv[2][a] * inv[2][b];
-  t3 = 0.0;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) t3 += G[a][0] * G[a][0] + G[a][1] * G[a][1] + G[a][2] * G[a][2];
-  t3 = t3 * nu * nu * cI;
-  const double m00 = G[0][0], m01 = G[0][1], m02 = G[0][2], m10 = G[1][0], m11 = G[1][1], m12 = G[1][2],
-               m20 = G[2][0], m21 = G[2][1], m22 = G[2][2];
-  const double dG = m00 * (m11 * m22 - m21 * m12) - m01 * (m10 * m22 - m12 * m20) + m02 * (m10 * m21 - m11 * m20);
-  const double idg = 1.0 / dG;
-  iG[0][0] = (m11 * m22 - m21 * m12) * idg;
-  iG[0][1] = (m02 * m21 - m01 * m22) * idg;
-  iG[0][2] = (m01 * m12 - m02 * m11) * idg;
-  iG[1][0] = (m12 * m20 - m10 * m22) * idg;
-  iG[1][1] = (m00 * m22 - m02 * m20) * idg;
-  iG[1][2] = (m10 * m02 - m00 * m12) * idg;
-  iG[2][0] = (m10 * m21 - m20 * m11) * idg;
-  iG[2][1] = (m20 * m01 - m00 * m21) * idg;
-  iG[2][2] = (m00 * m11 - m10 * m01) * idg;
-}
-
 // Gauss-point geometry of one hexa8 element, formed once per placement and
 // kept in HBM: per point g the inverse Jacobian (9 entries) and det J, entry
 // q of point g at geo[(g * FM_GEO_PER_GP + q) * E + e] (coalesced over the
 // tile's consecutive element slots).  The mesh does not move, so these are
 // the values the element loop would form at every step from the same
 // coordinates with the same expressions.
-__device__ __forceinline__ double geo_at(const double* geo, int64_t E, int g, double inv[3][3]) {
-  const double* q = geo + (int64_t)g * FM_GEO_PER_GP * E;
+//
+// The element loop streams it through shared memory: thread tid's rows of ten
+// values sit in a column of NB rows (stride THREADS) that the thread fills
+// for itself with asynchronous copies, NB - 1 points ahead, so neither a
+// register nor a barrier is spent on the look-ahead.  (Asking L1 for the rows
+// two points ahead and reading them there lost most of them again before
+// their use: 12 warps x 3 points x 2.5 KB do not fit beside the tiles' shared
+// memory; FP64 channel of 1 M hexa 0.438 -> 0.377 ms a step.)  PAIRED: the
+// points once in hexa_point's order, else 0..7, `passes` times round (B-bar:
+// n = 8..15 are points 0..7 again).
+__device__ __forceinline__ int hexa_point(int n) { return (n & ~1) + ((n & 1) ^ ((n >> 1) & 1) ^ 1); }
+__device__ __forceinline__ void copy_async(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+template <typename T, int THREADS, int NB, bool PAIRED>
+struct GeoStream {
+  T* column;
+  const T* geo;  // the element's first value
+  int64_t E;
+  int passes;    // times round the points (PAIRED: once)
+  // starts the copy of the n-th point; one group a call, also an empty one
+  __device__ __forceinline__ void copy(int n) const {
+    if (n < (PAIRED ? 8 : 8 * passes)) {
+      const T* q = geo + (int64_t)(PAIRED ? hexa_point(n) : (n & 7)) * FM_GEO_PER_GP * E;
+      T* d = column + (n & (NB - 1)) * FM_GEO_PER_GP * THREADS;
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+      for (int k = 0; k < FM_GEO_PER_GP; ++k) copy_async(d + k * THREADS, q + k * E);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // the copies an element's first row() expects to be on their way
+  __device__ __forceinline__ void start() const {
 #pragma unroll
-    for (int b = 0; b < 3; ++b) inv[a][b] = __ldg(q + (a * 3 + b) * E);
-  return __ldg(q + 9 * E);
+    for (int n = 0; n < NB - 1; ++n) copy(n);
+  }
+  // the n-th point's inverse Jacobian; returns its determinant.  n = 0, 1, ...
+  // in turn after start()
+  __device__ __forceinline__ T row(int n, T inv[3][3]) const {
+    copy(n + NB - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(NB - 1) : "memory");
+    const T* d = column + (n & (NB - 1)) * FM_GEO_PER_GP * THREADS;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) inv[i / 3][i % 3] = d[i * THREADS];
+    return d[9 * THREADS];
+  }
+  // the same straight from memory (the FP64 form's B-bar passes: keeping the
+  // stream going through them too cost the main loop 100 bytes of spill)
+  __device__ __forceinline__ T load(int n, T inv[3][3]) const {
+    const T* q = geo + (int64_t)(PAIRED ? hexa_point(n) : n) * FM_GEO_PER_GP * E;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) inv[i / 3][i % 3] = __ldg(q + i * E);
+    return __ldg(q + 9 * E);
+  }
+};
+// Rows of the column: FP64 two (a third costs the third CTA an SM: 0.565
+// instead of 0.377 ms), FP32 four (two 0.0729, four 0.0724 ms a step on the
+// 93x37x29 AB2 + B-bar channel; read from L1 0.0767).
+constexpr int FM_GEO_ROWS64 = 2, FM_GEO_ROWS32 = 4;
+template <int THREADS>
+using GeoStream64 = GeoStream<double, THREADS, FM_GEO_ROWS64, true>;
+template <int THREADS>
+using GeoStream32 = GeoStream<float, THREADS, FM_GEO_ROWS32, false>;
+
+// Doubles a thread of the tile kernels' per-thread region: tet4 the 12
+// staged entries; hexa8 FP64 the 24 velocity coefficients and the geometry
+// rows; hexa8 mixed its geometry rows.
+__host__ __device__ constexpr size_t supg_stage_doubles(int npe, bool mixed, int threads) {
+  return (size_t)threads * (npe == 4 ? 12 : mixed ? FM_GEO_ROWS32 * FM_GEO_PER_GP / 2 : 24 + FM_GEO_ROWS64 * FM_GEO_PER_GP);
 }
 
-// Requests point g's ten entries into L1 ahead of their use (the loads of a
-// warp cover consecutive element slots: one or two 128-byte lines an entry).
-template <typename T>
-__device__ __forceinline__ void geo_prefetch(const T* geo, int64_t E, int g) {
-  const T* q = geo + (int64_t)g * FM_GEO_PER_GP * E;
-#pragma unroll
-  for (int k = 0; k < FM_GEO_PER_GP; ++k) asm volatile("prefetch.global.L1 [%0];" ::"l"(q + k * E));
+// Inverse (cofactors, femUtils.cpp:716-770) and determinant of a 3x3 matrix.
+__device__ __forceinline__ double inverse3(const double J[3][3], double inv[3][3]) {
+  const double c0 = J[1][1] * J[2][2] - J[2][1] * J[1][2], c1 = J[1][2] * J[2][0] - J[1][0] * J[2][2],
+               c2 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+  const double det = J[0][0] * c0 + J[0][1] * c1 + J[0][2] * c2;
+  const double id = 1.0 / det;
+  inv[0][0] = c0 * id;
+  inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
+  inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
+  inv[1][0] = c1 * id;
+  inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
+  inv[1][2] = (J[1][0] * J[0][2] - J[0][0] * J[1][2]) * id;
+  inv[2][0] = c2 * id;
+  inv[2][1] = (J[2][0] * J[0][1] - J[0][0] * J[2][1]) * id;
+  inv[2][2] = (J[0][0] * J[1][1] - J[1][0] * J[0][1]) * id;
+  return det;
 }
 
-// The mixed form's copy: the same FP64 values rounded to FP32.
-__device__ __forceinline__ float geo_at_f(const float* geo, int64_t E, int g, float inv[3][3]) {
-  const float* q = geo + (int64_t)g * FM_GEO_PER_GP * E;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) inv[a][b] = __ldg(q + (a * 3 + b) * E);
-  return __ldg(q + 9 * E);
+// Signed sums of eight corner values (femHexa8.cpp:13-42 corner order) that
+// give 8 x the coefficients of {1, x, y, z, xy, yz, xz, xyz}, and the
+// transposed sums, node a taking sum_m sign_m(a) q[m]: 24 additions each.
+__device__ __forceinline__ void hexa_to_modes(const double n[8], double m[8]) {
+  const double a0 = n[1] + n[0], a1 = n[1] - n[0], b0 = n[2] + n[3], b1 = n[2] - n[3];
+  const double e0 = n[5] + n[4], e1 = n[5] - n[4], f0 = n[6] + n[7], f1 = n[6] - n[7];
+  const double p0 = b0 + a0, p2 = b0 - a0, p1 = b1 + a1, p4 = b1 - a1;
+  const double q0 = f0 + e0, q2 = f0 - e0, q1 = f1 + e1, q4 = f1 - e1;
+  m[0] = q0 + p0; m[3] = q0 - p0;
+  m[2] = q2 + p2; m[5] = q2 - p2;
+  m[1] = q1 + p1; m[6] = q1 - p1;
+  m[4] = q4 + p4; m[7] = q4 - p4;
+}
+__device__ __forceinline__ void hexa_to_nodes(const double q[8], double n[8]) {
+  const double zp0 = q[0] + q[3], zm0 = q[0] - q[3], zp2 = q[2] + q[5], zm2 = q[2] - q[5];
+  const double zp1 = q[1] + q[6], zm1 = q[1] - q[6], zp4 = q[4] + q[7], zm4 = q[4] - q[7];
+  const double a = zm0 - zm2, b = zm0 + zm2, c = zp0 - zp2, d = zp0 + zp2;      // even in x: y-z-, y+z-, y-z+, y+z+
+  const double A = zm1 - zm4, Bx = zm1 + zm4, Cx = zp1 - zp4, D = zp1 + zp4;    // odd in x
+  n[0] = a - A; n[1] = a + A;
+  n[3] = b - Bx; n[2] = b + Bx;
+  n[4] = c - Cx; n[5] = c + Cx;
+  n[7] = d - D; n[6] = d + D;
 }
 
-// One element: k[a][c] = -dt (sum of the enabled K_i u_e)[a][c].  Coordinates
-// and velocities are read from the tile's shared-memory node arrays through
-// the local ids ln[]; with GEO the Gauss-point inverse Jacobians and
-// determinants are read from the stored geometry instead (geo = the
-// element's first entry, E = the row stride).  Also returns the element's
-// lambda (volume average) and regime (average of the Gauss-point regimes)
-// for output.
-template <int NPE, bool GEO = false>
-__device__ __forceinline__ void supg_element(const DevProb& P, const ShapeTable<NPE, double>& tab, const double* sx,
-                                             const double* sy, const double* sz, const double* su, const double* sv,
-                                             const double* sw, const int ln[NPE], double k[NPE][3], double& lam_el,
-                                             double& reg_el, const double* geo = nullptr, int64_t E = 0) {
-  const double rho = P.rho, mu = P.mu, alpha = P.alpha, cI = P.c_i;
+// One tet4 element: k[a][c] = -dt (sum of the enabled K_i u_e)[a][c], its
+// lambda (volume average) and regime (average of the Gauss-point regimes).
+// The Jacobian, the velocity gradient, the metric G = J^-T J^-1, the shear
+// part of the stress and the weight w are element constants, and with
+// lN_a(g) = ALPHA (a = g) or BETA the velocity at the points is
+// BETA sum_a u_a + (ALPHA - BETA) u_g; so only u_g, tau, nu_C, lambda and the
+// convection (u_g . grad) u are formed per point, and the points enter the
+// forces through sums,
+//   k_a[c] = -dt w ( sum_d gd_a[d] T[c][d] + rho (BETA sum_g conv_g + (ALPHA - BETA) conv_a)[c] ),
+//   T[c][d] = stress_cd (with sum_g lambda) + rho div sum_g nu_C delta_cd + rho sum_g tau_g u_g[d] conv_g[c],
+// with gd_3 = -(gd_0 + gd_1 + gd_2).  u^T G^-1 u = |J^T u|^2 needs no inverse
+// of G.  FP64 instructions are what bounds the tile kernel here (fixed
+// latency chains at 12 warps an SM), so their number is what counts.
+__device__ __forceinline__ void supg_element_tet(const DevProb& P, const double* sx, const double* sy, const double* sz,
+                                                 const double* su, const double* sv, const double* sw, const int ln[4],
+                                                 double k[4][3], double& lam_el, double& reg_el) {
+  const double rho = P.rho, mu = P.mu, alpha = P.alpha;
   const double nu = mu / rho;
-  const bool bbar = (P.ex_mask & 2) != 0;
   const bool iK1 = (P.ex_mask & 4) != 0, iK2 = (P.ex_mask & 8) != 0, iK3 = (P.ex_mask & 16) != 0,
              iK4 = (P.ex_mask & 32) != 0;
-  const double wq = GaussRule<NPE>::weight();
+  constexpr double A = 0.58541020, Bt = 0.13819660, AB = A - Bt;
+  double J[3][3];  // J[a][c] = x_a[c] - x_3[c]
+  {
+    const double x3 = sx[ln[3]], y3 = sy[ln[3]], z3 = sz[ln[3]];
 #pragma unroll
-  for (int a = 0; a < NPE; ++a) k[a][0] = k[a][1] = k[a][2] = 0.0;
-  // B-bar (eval_avg_shapeDeriv, src lines 660-707, and the B matrix rows
-  // 0-2, src lines 234-256).  With sd0[a][c] = sum_g w_g gd_g[a][c] / V the
-  // volume-averaged derivatives, B1 = (sd0[a][0] - gd[a][0]) / 3, B2 =
-  // gd[a][0] - B1 and likewise B3/B4, B5/B6 for y and z, the sums over the
-  // nodes are
-  //   strain:  eps_c = gr_cc - 2 d_c + (d_0 + d_1 + d_2),
-  //            d_c = (Dbar_c - gr_cc) / 3,  Dbar_c = sum_a sd0[a][c] u_c(a)
-  //   force:   r_c(a) w = gd[a][c] (w sig_c - q_c) + sd0[a][c] q_c,
-  //            q_c = w (sig_0 + sig_1 + sig_2 - 2 sig_c) / 3,
-  // so sd0 enters only through the element constants Dbar_c = sum_g w_g
-  // gr_g[c][c] / V (before the Gauss loop) and sd0[a][c] Q_c, Q_c = sum_g q_c
-  // (after it): the 24 averaged derivatives are never held in registers.
-  auto jac_inv = [&](int g, double inv[3][3]) -> double {
-    if constexpr (GEO) return geo_at(geo, E, g, inv);
-    return jacobian_at<NPE>([&](int n, int c) { return tab.dN[g][n][c]; }, sx, sy, sz, ln, inv);
-  };
-  double Dbar[3] = {0.0, 0.0, 0.0}, Qb[3] = {0.0, 0.0, 0.0}, bden = 0.0;
-  if (NPE == 8 && bbar) {
-    double dsum[3] = {0.0, 0.0, 0.0};
-#pragma unroll 1
-    for (int g = 0; g < GaussRule<NPE>::n; ++g) {
-      double inv[3][3];
-      const double w = jac_inv(g, inv) * wq;
-      bden += w;
-      double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-#pragma unroll
-      for (int a = 0; a < NPE; ++a) {
-        const double d0 = tab.dN[g][a][0], d1 = tab.dN[g][a][1], d2 = tab.dN[g][a][2];
-        g0 += (inv[0][0] * d0 + inv[0][1] * d1 + inv[0][2] * d2) * su[ln[a]];
-        g1 += (inv[1][0] * d0 + inv[1][1] * d1 + inv[1][2] * d2) * sv[ln[a]];
-        g2 += (inv[2][0] * d0 + inv[2][1] * d1 + inv[2][2] * d2) * sw[ln[a]];
-      }
-      dsum[0] += w * g0; dsum[1] += w * g1; dsum[2] += w * g2;
+    for (int a = 0; a < 3; ++a) {
+      J[a][0] = sx[ln[a]] - x3;
+      J[a][1] = sy[ln[a]] - y3;
+      J[a][2] = sz[ln[a]] - z3;
     }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) Dbar[c] = dsum[c] / bden;
   }
-  // tet4: the local derivatives are constant, so the Jacobian, its inverse,
-  // G = J^-T J^-1, the G:G term of tau and G's inverse are element constants;
-  // they are formed once here (the same expressions as at every Gauss point,
-  // hence the same values) instead of at each of the 4 points
-  auto dN4 = [](int a, int c) -> double { return a == 3 ? -1.0 : (a == c ? 1.0 : 0.0); };
-  double inv4[3][3], det4 = 0.0, G4[3][3], t3_4 = 0.0, iG4[3][3];
-  if constexpr (NPE == 4) {
-    det4 = jacobian_at<NPE>(dN4, sx, sy, sz, ln, inv4);
-    tet_metric(inv4, nu, cI, G4, t3_4, iG4);
+  double inv[3][3];
+  const double det = inverse3(J, inv);
+  // G's entries (symmetric), its trace and the G:G term of tau
+  const double g00 = inv[0][0] * inv[0][0] + inv[1][0] * inv[1][0] + inv[2][0] * inv[2][0];
+  const double g11 = inv[0][1] * inv[0][1] + inv[1][1] * inv[1][1] + inv[2][1] * inv[2][1];
+  const double g22 = inv[0][2] * inv[0][2] + inv[1][2] * inv[1][2] + inv[2][2] * inv[2][2];
+  const double h01 = 2.0 * (inv[0][0] * inv[0][1] + inv[1][0] * inv[1][1] + inv[2][0] * inv[2][1]);
+  const double h02 = 2.0 * (inv[0][0] * inv[0][2] + inv[1][0] * inv[1][2] + inv[2][0] * inv[2][2]);
+  const double h12 = 2.0 * (inv[0][1] * inv[0][2] + inv[1][1] * inv[1][2] + inv[2][1] * inv[2][2]);
+  const double irG = 1.0 / (g00 + g11 + g22);
+  const double t3 = (g00 * g00 + g11 * g11 + g22 * g22 + 0.5 * (h01 * h01 + h02 * h02 + h12 * h12)) * nu * nu * P.c_i;
+  double U[4][3], gr[3][3], Us[3];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    U[a][0] = su[ln[a]];
+    U[a][1] = sv[ln[a]];
+    U[a][2] = sw[ln[a]];
   }
-  double vol = 0.0, lam_int = 0.0, reg = 0.0;
-  if constexpr (GEO) {
-    geo_prefetch(geo, E, 0);
-    geo_prefetch(geo, E, 1);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double d0 = U[0][c] - U[3][c], d1 = U[1][c] - U[3][c], d2 = U[2][c] - U[3][c];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) gr[c][d] = inv[d][0] * d0 + inv[d][1] * d1 + inv[d][2] * d2;
+    Us[c] = Bt * ((U[0][c] + U[1][c]) + (U[2][c] + U[3][c]));
   }
-#pragma unroll 1
-  for (int g = 0; g < GaussRule<NPE>::n; ++g) {
-    // shape values and local derivatives: tet4 in closed form (constant
-    // derivatives), hexa8 read from the shared-memory table where used; the
-    // global derivatives are formed where used too (no register arrays)
-    double Nq[NPE];
-    if (NPE == 4) {
-      double q[3];
-      GaussRule<NPE>::point(g, q);
-      Nq[0] = q[0]; Nq[1] = q[1]; Nq[2] = q[2]; Nq[3 % NPE] = 1.0 - q[0] - q[1] - q[2];
-    }
-    auto Nv = [&](int a) -> double { return NPE == 4 ? Nq[a] : tab.N[g][a]; };
-    auto dNv = [&](int a, int c) -> double {
-      if (NPE == 4) return dN4(a, c);
-      return tab.dN[g][a][c];
-    };
-    double inv[3][3], G[3][3], t3 = 0.0, iG[3][3];
-    double det;
-    if constexpr (NPE == 4) {
-      det = det4;
+  const double div = gr[0][0] + gr[1][1] + gr[2][2];
+  double M[3][3], cs[3] = {0.0, 0.0, 0.0}, Ls = 0.0, Ns = 0.0, reg = 0.0;
 #pragma unroll
-      for (int a = 0; a < 3; ++a)
+  for (int d = 0; d < 3; ++d) M[d][0] = M[d][1] = M[d][2] = 0.0;
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-          inv[a][b] = inv4[a][b];
-          G[a][b] = G4[a][b];
-          iG[a][b] = iG4[a][b];
-        }
-      t3 = t3_4;
-    } else {
-      if constexpr (GEO) {
-        if (g + 2 < GaussRule<NPE>::n) geo_prefetch(geo, E, g + 2);
-      }
-      det = jac_inv(g, inv);
-      tet_metric(inv, nu, cI, G, t3, iG);
-    }
-    auto gdv = [&](int a, int b) -> double {
-      return inv[b][0] * dNv(a, 0) + inv[b][1] * dNv(a, 1) + inv[b][2] * dNv(a, 2);
-    };
-    // velocity, gradient, divergence at the point.  hexa8: the gradient in
-    // local coordinates first, Lg[c][k] = sum_a dN[a][k] u_a[c], then
-    // gr[c][d] = sum_k inv[d][k] Lg[c][k] (the same sum over the nodes as
-    // sum_a gd[a][d] u_a[c], 99 instead of 144 FLOP a point); tet4's
-    // derivatives are constants, so its global ones cost nothing to form
-    double u[3] = {0.0, 0.0, 0.0}, gr[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-    if constexpr (NPE == 8) {
-      double Lg[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+  for (int g = 0; g < 4; ++g) {
+    double u[3];
 #pragma unroll
-      for (int a = 0; a < NPE; ++a) {
-        const double ua[3] = {su[ln[a]], sv[ln[a]], sw[ln[a]]};
-        const double Na = Nv(a);
-        const double da[3] = {dNv(a, 0), dNv(a, 1), dNv(a, 2)};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          u[c] += Na * ua[c];
-#pragma unroll
-          for (int kk = 0; kk < 3; ++kk) Lg[c][kk] += da[kk] * ua[c];
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) gr[c][d] = inv[d][0] * Lg[c][0] + inv[d][1] * Lg[c][1] + inv[d][2] * Lg[c][2];
-    } else {
-#pragma unroll
-      for (int a = 0; a < NPE; ++a) {
-        const double ua[3] = {su[ln[a]], sv[ln[a]], sw[ln[a]]};
-        const double ga[3] = {gdv(a, 0), gdv(a, 1), gdv(a, 2)};
-        const double Na = Nv(a);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          u[c] += Na * ua[c];
-#pragma unroll
-          for (int d = 0; d < 3; ++d) gr[c][d] += ga[d] * ua[c];
-        }
-      }
-    }
-    const double div = gr[0][0] + gr[1][1] + gr[2][2];
-    // eval_stabilization (dt term removed in the reference)
-    const double trG = G[0][0] + G[1][1] + G[2][2];
-    double t2 = 0.0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) t2 += u[a] * (G[a][0] * u[0] + G[a][1] * u[1] + G[a][2] * u[2]);
-    const double tau = 1.0 / sqrt(t2 + t3);
-    const double nuC = 1.0 / (trG * tau);
+    for (int c = 0; c < 3; ++c) u[c] = Us[c] + AB * U[g][c];
+    // eval_stabilization (dt term removed in the reference): tau = q^-1/2,
+    // nu_C = 1 / (tr G tau) = q^1/2 / tr G
+    const double q = t3 + u[0] * (g00 * u[0] + h01 * u[1] + h02 * u[2]) + u[1] * (g11 * u[1] + h12 * u[2]) +
+                     u[2] * (g22 * u[2]);
+    const double tau = rsqrt_nr(q);
+    Ns += (q == 0.0) ? 0.0 : q * tau;
     // eval_bulk_modulus: lambda = alpha * max(mu/rho, sqrt(u^T G^-1 u))
-    double lam, regime;
-    {
-      const double l2 = sqrt((iG[0][0] * u[0] + iG[0][1] * u[1] + iG[0][2] * u[2]) * u[0] +
-                             (iG[1][0] * u[0] + iG[1][1] * u[1] + iG[1][2] * u[2]) * u[1] +
-                             (iG[2][0] * u[0] + iG[2][1] * u[1] + iG[2][2] * u[2]) * u[2]);
-      const double l1 = nu;
-      lam = alpha * ((l1 < l2) ? l2 : l1);  // std::max(limit_1, limit_2)
-      regime = (l1 > l2) ? 1.0 : 2.0;
-    }
-    const double w = det * wq;
-    vol += w;
-    lam_int += lam * w;
-    reg += regime;
-    double conv[3];
+    const double v0 = J[0][0] * u[0] + J[1][0] * u[1] + J[2][0] * u[2];
+    const double v1 = J[0][1] * u[0] + J[1][1] * u[1] + J[2][1] * u[2];
+    const double v2 = J[0][2] * u[0] + J[1][2] * u[1] + J[2][2] * u[2];
+    const double l2 = sqrt_nr(v0 * v0 + v1 * v1 + v2 * v2);
+    Ls += (nu < l2) ? l2 : nu;  // std::max(limit_1, limit_2)
+    reg += (nu > l2) ? 1.0 : 2.0;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) conv[c] = u[0] * gr[c][0] + u[1] * gr[c][1] + u[2] * gr[c][2];
-    // strain (B u) and stress (D B u)
-    double eps[6];
-    if (NPE == 8 && bbar) {
-      const double d0 = (1.0 / 3.0) * (Dbar[0] - gr[0][0]), d1 = (1.0 / 3.0) * (Dbar[1] - gr[1][1]),
-                   d2 = (1.0 / 3.0) * (Dbar[2] - gr[2][2]);
-      eps[0] = gr[0][0] - d0 + d1 + d2;
-      eps[1] = d0 + gr[1][1] - d1 + d2;
-      eps[2] = d0 + d1 + gr[2][2] - d2;
-    } else {
-      eps[0] = gr[0][0]; eps[1] = gr[1][1]; eps[2] = gr[2][2];
+    for (int c = 0; c < 3; ++c) {
+      const double cv = u[0] * gr[c][0] + u[1] * gr[c][1] + u[2] * gr[c][2];
+      k[g][c] = cv;
+      cs[c] += cv;
+      const double tc = tau * cv;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) M[d][c] += u[d] * tc;
     }
-    eps[3] = gr[0][1] + gr[1][0];
-    eps[4] = gr[1][2] + gr[2][1];
-    eps[5] = gr[0][2] + gr[2][0];
-    const double l2m = lam + 2 * mu;
-    const double sig[6] = {l2m * eps[0] + lam * eps[1] + lam * eps[2], lam * eps[0] + l2m * eps[1] + lam * eps[2],
-                           lam * eps[0] + lam * eps[1] + l2m * eps[2], mu * eps[3], mu * eps[4], mu * eps[5]};
-    const double c1w = rho * w, c3w = rho * tau * w, c4w = rho * nuC * div * w;
-    // normal-stress parts of K2: w sig_c multiplies gd[a][c]; with B-bar less
-    // q_c, whose sd0 part is added after the loop
-    double sd[3] = {sig[0] * w, sig[1] * w, sig[2] * w};
-    if (NPE == 8 && bbar && iK2) {
-      const double st = sig[0] + sig[1] + sig[2];
+  }
+  Ls *= alpha;
+  lam_el = 0.25 * Ls;
+  reg_el = 0.25 * reg;
+  const double w = -P.dt * (det * GaussRule<4>::weight());
+  const double rw = rho * w;
+  double T[3][3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) T[c][d] = iK3 ? rw * M[d][c] : 0.0;
+  if (iK2) {
+    const double n = w * (div * Ls), m4 = 4.0 * (w * mu), m8 = 2.0 * m4;
+    const double s01 = m4 * (gr[0][1] + gr[1][0]), s12 = m4 * (gr[1][2] + gr[2][1]), s02 = m4 * (gr[0][2] + gr[2][0]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) T[c][c] += n + m8 * gr[c][c];
+    T[0][1] += s01; T[1][0] += s01;
+    T[1][2] += s12; T[2][1] += s12;
+    T[0][2] += s02; T[2][0] += s02;
+  }
+  if (iK4) {
+    const double n = rw * div * (Ns * irG);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) T[c][c] += n;
+  }
+  const double c1 = iK1 ? rw * AB : 0.0, c0 = iK1 ? rw * Bt : 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double b = c0 * cs[c];
+    double f3 = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double f = T[c][0] * inv[0][a] + T[c][1] * inv[1][a] + T[c][2] * inv[2][a];
+      k[a][c] = f + (b + c1 * k[a][c]);
+      f3 += f;
+    }
+    k[3][c] = (b + c1 * k[3][c]) - f3;
+  }
+}
+
+// One hexa8 element, same outputs.  The trilinear field is held by its eight
+// coefficients in {1, x, y, z, xy, yz, xz, xyz} (local coordinates; C below,
+// scaled by the powers of s = 1/sqrt(3) that the points +-s bring), a few
+// additions of the nodal values, so a point's velocity and local gradient
+// are sums of coefficients with signs instead of sums over eight nodes of
+// tabulated shape values (16 additions a component for the two points of a
+// pair with the same y and z, against 64 products), and the forces are
+// gathered into the same eight coefficients (K; 25 additions a component
+// and pair against 64 products) and taken back to the nodes once at the end.
+// Nothing is read from shared memory inside the loop.  Per point every force
+// is one matrix and one vector on the test function:
+//   k_a[c] += sum_j W[c][j] dN_a/dxi_j + b[c] N_a,
+//   W = (S + c4w I) J^-1 + c3w conv (J^-T u)^T,  b = c1w conv,
+// S the stress terms of K2, c4w I those of K4.  u^T G^-1 u = |J^T u|^2 with
+// J^T = det J x cof(J^-1) applied through two cross products.  The point
+// geometry comes from the stored one (GeoStream).
+//
+// B-bar (eval_avg_shapeDeriv, src lines 660-707, and the B matrix rows 0-2,
+// src lines 234-256).  With sd0[a][c] = sum_g w_g gd_g[a][c] / V the
+// volume-averaged derivatives, B1 = (sd0[a][0] - gd[a][0]) / 3, B2 =
+// gd[a][0] - B1 and likewise B3/B4, B5/B6 for y and z, the sums over the
+// nodes are
+//   strain:  eps_c = gr_cc - 2 d_c + (d_0 + d_1 + d_2),
+//            d_c = (Dbar_c - gr_cc) / 3,  Dbar_c = sum_a sd0[a][c] u_c(a)
+//   force:   r_c(a) w = gd[a][c] (w sig_c - q_c) + sd0[a][c] q_c,
+//            q_c = w (sig_0 + sig_1 + sig_2 - 2 sig_c) / 3,
+// so sd0 enters only through the element constants Dbar_c = sum_g w_g
+// gr_g[c][c] / V (a pass before the Gauss loop) and sd0[a][c] Q_c,
+// Q_c = sum_g q_c (a pass after it).
+// BBAR is a template parameter so that the other elements do not hold its six
+// element constants.
+template <int THREADS, bool BBAR>
+__device__ __forceinline__ void supg_element_hexa(const DevProb& P, const double* su, const double* sv, const double* sw,
+                                                  const int ln[8], double* coef, double k[8][3], double& lam_el,
+                                                  double& reg_el, const GeoStream64<THREADS>& geo) {
+  const double rho = P.rho, mu = P.mu, alpha = P.alpha;
+  const double nu = mu / rho;
+  const bool iK1 = (P.ex_mask & 4) != 0, iK2 = (P.ex_mask & 8) != 0, iK3 = (P.ex_mask & 16) != 0,
+             iK4 = (P.ex_mask & 32) != 0;
+  constexpr double s = 0.57735026918962573;  // 1/sqrt(3), correctly rounded
+  double K[8][3];
+  // C in the thread's own shared-memory column (stride THREADS): 48 registers
+  // less, which is what lets three CTAs an SM run without spilling (0.496 ->
+  // 0.438 ms a step for 1 M hexa)
+  auto Cv = [&](int m, int c) -> double& { return coef[(m * 3 + c) * THREADS]; };
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double* q = c == 0 ? su : (c == 1 ? sv : sw);
+    double n[8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) n[a] = q[ln[a]];
+    double m[8];
+    hexa_to_modes(n, m);
+    Cv(0, c) = 0.125 * m[0]; Cv(1, c) = 0.125 * m[1]; Cv(2, c) = 0.125 * m[2]; Cv(3, c) = 0.125 * m[3];
+    Cv(4, c) = (0.125 * s) * m[4]; Cv(5, c) = (0.125 * s) * m[5]; Cv(6, c) = (0.125 * s) * m[6];
+    Cv(7, c) = (0.125 * s * s) * m[7];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) K[a][c] = 0.0;
+  }
+  // pair p: the points x = +s and x = -s at y = sy s, z = sz s
+  auto sign_y = [](int p) -> double { return (p & 1) ? 1.0 : -1.0; };
+  auto sign_z = [](int p) -> double { return (p & 2) ? -1.0 : 1.0; };
+  double vol = 0.0, lam_int = 0.0, reg = 0.0;
+  double Dbar[3] = {0.0, 0.0, 0.0}, Qb[3] = {0.0, 0.0, 0.0};
+  if constexpr (BBAR) {
+    double bden = 0.0;
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {
+      const double sy = sign_y(p), sz = sign_z(p), yz = sy * sz;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const double sx = h ? -1.0 : 1.0;
+        double inv[3][3];
+        const double w = geo.load(2 * p + h, inv);
+        bden += w;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double l0 = Cv(1, c) + sy * Cv(4, c) + sz * Cv(6, c) + yz * Cv(7, c);
+          const double l1 = Cv(2, c) + sx * Cv(4, c) + sz * Cv(5, c) + (sx * sz) * Cv(7, c);
+          const double l2 = Cv(3, c) + sx * Cv(6, c) + sy * Cv(5, c) + (sx * sy) * Cv(7, c);
+          Dbar[c] += w * (inv[c][0] * l0 + inv[c][1] * l1 + inv[c][2] * l2);
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) Dbar[c] /= bden;
+  }
+  // one point: velocity u, local gradient L[c][j] -> W, b (see above)
+  auto point = [&](int n, const double u[3], const double L[3][3], double W[3][3], double b[3]) {
+    double inv[3][3];
+    const double det = geo.row(n, inv);
+    double gr[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) gr[c][d] = inv[d][0] * L[c][0] + inv[d][1] * L[c][1] + inv[d][2] * L[c][2];
+    const double div = gr[0][0] + gr[1][1] + gr[2][2];
+    // eval_stabilization (dt term removed in the reference): tau = q^-1/2,
+    // nu_C = 1 / (tr G tau) = q^1/2 / tr G, u^T G u = |J^-1 u|^2
+    double trG, q;
+    {
+      const double g00 = inv[0][0] * inv[0][0] + inv[1][0] * inv[1][0] + inv[2][0] * inv[2][0];
+      const double g11 = inv[0][1] * inv[0][1] + inv[1][1] * inv[1][1] + inv[2][1] * inv[2][1];
+      const double g22 = inv[0][2] * inv[0][2] + inv[1][2] * inv[1][2] + inv[2][2] * inv[2][2];
+      const double g01 = inv[0][0] * inv[0][1] + inv[1][0] * inv[1][1] + inv[2][0] * inv[2][1];
+      const double g02 = inv[0][0] * inv[0][2] + inv[1][0] * inv[1][2] + inv[2][0] * inv[2][2];
+      const double g12 = inv[0][1] * inv[0][2] + inv[1][1] * inv[1][2] + inv[2][1] * inv[2][2];
+      trG = g00 + g11 + g22;
+      q = (g00 * g00 + g11 * g11 + g22 * g22 + 2.0 * (g01 * g01 + g02 * g02 + g12 * g12)) * nu * nu * P.c_i;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const double q = (1.0 / 3.0) * w * (st - 2.0 * sig[c]);
-        Qb[c] += q;
-        sd[c] -= q;
+        const double t = inv[c][0] * u[0] + inv[c][1] * u[1] + inv[c][2] * u[2];
+        q += t * t;
       }
     }
-    if constexpr (NPE == 8) {
-      // hexa8: every term is linear in gd[a] = inv dN[a] (K2: S gd[a] with S
-      // the symmetric matrix of the stress terms above; K4: c4w gd[a]; K3:
-      // u.gd[a]), so inv is folded into one 3x3 matrix and one vector a
-      // point, T = (S + c4w I) inv and ut = inv^T u, and each node takes
-      // T dN[a] and ut.dN[a] (17 instead of ~36 FLOP a node)
-      double S[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-      if (iK2) {
-        S[0][0] = sd[0]; S[1][1] = sd[1]; S[2][2] = sd[2];
-        S[0][1] = S[1][0] = sig[3] * w;
-        S[1][2] = S[2][1] = sig[4] * w;
-        S[0][2] = S[2][0] = sig[5] * w;
-      }
-      if (iK4) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) S[c][c] += c4w;
-      }
-      double T[3][3], ut[3];
-#pragma unroll
-      for (int kk = 0; kk < 3; ++kk) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) T[c][kk] = S[c][0] * inv[0][kk] + S[c][1] * inv[1][kk] + S[c][2] * inv[2][kk];
-        ut[kk] = u[0] * inv[0][kk] + u[1] * inv[1][kk] + u[2] * inv[2][kk];
-      }
-#pragma unroll
-      for (int a = 0; a < NPE; ++a) {
-        const double da[3] = {dNv(a, 0), dNv(a, 1), dNv(a, 2)};
-        double sa = 0.0;
-        if (iK1) sa = c1w * Nv(a);
-        if (iK3) sa += c3w * (ut[0] * da[0] + ut[1] * da[1] + ut[2] * da[2]);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) k[a][c] += T[c][0] * da[0] + T[c][1] * da[1] + T[c][2] * da[2] + sa * conv[c];
-      }
-    } else {
-#pragma unroll
-    for (int a = 0; a < NPE; ++a) {
-      const double ga[3] = {gdv(a, 0), gdv(a, 1), gdv(a, 2)};
-      const double Aa = u[0] * ga[0] + u[1] * ga[1] + u[2] * ga[2];
-      double f[3] = {0.0, 0.0, 0.0};
-      if (iK1) {
-        const double Na = Nv(a);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[c] += c1w * Na * conv[c];
-      }
-      if (iK3) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[c] += c3w * Aa * conv[c];
-      }
-      if (iK4) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[c] += c4w * ga[c];
-      }
-      if (iK2) {
-        f[0] += ga[0] * sd[0] + (ga[1] * sig[3] + ga[2] * sig[5]) * w;
-        f[1] += ga[1] * sd[1] + (ga[0] * sig[3] + ga[2] * sig[4]) * w;
-        f[2] += ga[2] * sd[2] + (ga[1] * sig[4] + ga[0] * sig[5]) * w;
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) k[a][c] += f[c];
+    const double tau = rsqrt_nr(q);
+    const double nuC = ((q == 0.0) ? 0.0 : q * tau) * rcp_nr(trG);
+    // eval_bulk_modulus: lambda = alpha * max(mu/rho, sqrt(u^T G^-1 u));
+    // J^T u / det J = (u . (r1 x r2), u . (r2 x r0), u . (r0 x r1)), r_i the
+    // rows of J^-1
+    double lam;
+    {
+      const double a0 = u[1] * inv[0][2] - u[2] * inv[0][1], a1 = u[2] * inv[0][0] - u[0] * inv[0][2],
+                   a2 = u[0] * inv[0][1] - u[1] * inv[0][0];  // u x r0
+      const double b0 = u[1] * inv[1][2] - u[2] * inv[1][1], b1 = u[2] * inv[1][0] - u[0] * inv[1][2],
+                   b2 = u[0] * inv[1][1] - u[1] * inv[1][0];  // u x r1
+      const double v0 = inv[2][0] * b0 + inv[2][1] * b1 + inv[2][2] * b2;
+      const double v1 = inv[2][0] * a0 + inv[2][1] * a1 + inv[2][2] * a2;  // sign dropped (squared)
+      const double v2 = inv[1][0] * a0 + inv[1][1] * a1 + inv[1][2] * a2;
+      const double l2 = fabs(det) * sqrt_nr(v0 * v0 + v1 * v1 + v2 * v2);
+      lam = alpha * ((nu < l2) ? l2 : nu);  // std::max(limit_1, limit_2)
+      reg += (nu > l2) ? 1.0 : 2.0;
     }
-    }
-  }
-  if (NPE == 8 && bbar && iK2) {
-    // k[a][c] += sd0[a][c] Q_c, sd0 formed again Gauss point by Gauss point
+    const double w = det;  // quadrature weight 1
+    vol += w;
+    lam_int += lam * w;
+    double S[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+    if (iK2) {
+      const double mw = mu * w, m2 = 2.0 * mw;
+      double e[3] = {gr[0][0], gr[1][1], gr[2][2]}, tr = div;
+      if constexpr (BBAR) {
+        const double d0 = (1.0 / 3.0) * (Dbar[0] - e[0]), d1 = (1.0 / 3.0) * (Dbar[1] - e[1]),
+                     d2 = (1.0 / 3.0) * (Dbar[2] - e[2]);
+        const double t = d0 + d1 + d2;
+        e[0] += t - 2.0 * d0;
+        e[1] += t - 2.0 * d1;
+        e[2] += t - 2.0 * d2;
+        tr = e[0] + e[1] + e[2];
+      }
+      const double lt = lam * w * tr;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) Qb[c] /= bden;
+      for (int c = 0; c < 3; ++c) S[c][c] = lt + m2 * e[c];
+      if constexpr (BBAR) {
+        const double st = S[0][0] + S[1][1] + S[2][2];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double qc = (1.0 / 3.0) * (st - 2.0 * S[c][c]);
+          Qb[c] += qc;
+          S[c][c] -= qc;
+        }
+      }
+      S[0][1] = S[1][0] = mw * (gr[0][1] + gr[1][0]);
+      S[1][2] = S[2][1] = mw * (gr[1][2] + gr[2][1]);
+      S[0][2] = S[2][0] = mw * (gr[0][2] + gr[2][0]);
+    }
+    if (iK4) {
+      const double c4w = rho * nuC * div * w;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) S[c][c] += c4w;
+    }
+    const double c1w = iK1 ? rho * w : 0.0, c3w = iK3 ? rho * tau * w : 0.0;
+    double ut[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) ut[j] = u[0] * inv[0][j] + u[1] * inv[1][j] + u[2] * inv[2][j];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double cv = u[0] * gr[c][0] + u[1] * gr[c][1] + u[2] * gr[c][2];
+      b[c] = c1w * cv;
+      const double c3 = c3w * cv;
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        W[c][j] = c3 * ut[j] + (S[c][0] * inv[0][j] + S[c][1] * inv[1][j] + S[c][2] * inv[2][j]);
+    }
+  };
 #pragma unroll 1
-    for (int g = 0; g < GaussRule<NPE>::n; ++g) {
-      double inv[3][3];
-      const double w = jac_inv(g, inv) * wq;
-      const double s0 = w * Qb[0], s1 = w * Qb[1], s2 = w * Qb[2];
+  for (int p = 0; p < 4; ++p) {
+    const double sy = sign_y(p), sz = sign_z(p), yz = sy * sz;
+    double Wp[3][3], Wm[3][3], bp[3], bm[3];
+    {
+      double up[3], um[3], Lp[3][3], Lm[3][3];
 #pragma unroll
-      for (int a = 0; a < NPE; ++a) {
-        const double d0 = tab.dN[g][a][0], d1 = tab.dN[g][a][1], d2 = tab.dN[g][a][2];
-        k[a][0] += (inv[0][0] * d0 + inv[0][1] * d1 + inv[0][2] * d2) * s0;
-        k[a][1] += (inv[1][0] * d0 + inv[1][1] * d1 + inv[1][2] * d2) * s1;
-        k[a][2] += (inv[2][0] * d0 + inv[2][1] * d1 + inv[2][2] * d2) * s2;
+      for (int c = 0; c < 3; ++c) {
+        const double B0 = Cv(2, c) + sz * Cv(5, c), B1 = Cv(4, c) + sz * Cv(7, c);
+        const double D0 = Cv(3, c) + sy * Cv(5, c), D1 = Cv(6, c) + sy * Cv(7, c);
+        const double A1 = Cv(1, c) + sz * Cv(6, c) + sy * B1;
+        const double Ev = sy * B0 + sz * Cv(3, c);
+        up[c] = Cv(0, c) + s * (Ev + A1);
+        um[c] = Cv(0, c) + s * (Ev - A1);
+        Lp[c][0] = A1; Lp[c][1] = B0 + B1; Lp[c][2] = D0 + D1;
+        Lm[c][0] = A1; Lm[c][1] = B0 - B1; Lm[c][2] = D0 - D1;
+      }
+      point(2 * p, up, Lp, Wp, bp);
+      point(2 * p + 1, um, Lm, Wm, bm);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double bs = s * (bp[c] + bm[c]);
+      const double Q = (Wp[c][0] + Wm[c][0]) + s * (bp[c] - bm[c]);
+      const double es = Wp[c][1] + Wm[c][1], ed = Wp[c][1] - Wm[c][1];
+      const double zs = Wp[c][2] + Wm[c][2], zd = Wp[c][2] - Wm[c][2];
+      K[0][c] += bs;  // x 1/s at the end
+      K[1][c] += Q;
+      K[2][c] += es + sy * bs;
+      K[3][c] += zs + sz * bs;
+      K[4][c] += sy * Q + ed;                       // x s
+      K[5][c] += sz * es + (sy * zs + yz * bs);     // x s
+      K[6][c] += sz * Q + zd;                       // x s
+      K[7][c] += yz * Q + (sz * ed + sy * zd);      // x s^2
+    }
+  }
+  if (BBAR && iK2) {
+    // k_a[c] += sd0[a][c] Q_c, sd0 formed again point by point
+#pragma unroll
+    for (int c = 0; c < 3; ++c) Qb[c] /= vol;
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {
+      const double sy = sign_y(p), sz = sign_z(p), yz = sy * sz;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const double sx = h ? -1.0 : 1.0;
+        double inv[3][3];
+        const double w = geo.load(2 * p + h, inv);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double f = w * Qb[c];
+          const double w0 = f * inv[c][0], w1 = f * inv[c][1], w2 = f * inv[c][2];
+          K[1][c] += w0;
+          K[2][c] += w1;
+          K[3][c] += w2;
+          K[4][c] += sy * w0 + sx * w1;
+          K[5][c] += sz * w1 + sy * w2;
+          K[6][c] += sz * w0 + sx * w2;
+          K[7][c] += yz * w0 + ((sx * sz) * w1 + (sx * sy) * w2);
+        }
       }
     }
   }
-  const double mdt = -P.dt;
+  const double m = -0.125 * P.dt;
 #pragma unroll
-  for (int a = 0; a < NPE; ++a)
+  for (int c = 0; c < 3; ++c) {
+    const double q[8] = {(m / s) * K[0][c], m * K[1][c], m * K[2][c], m * K[3][c],
+                         (m * s) * K[4][c], (m * s) * K[5][c], (m * s) * K[6][c], (m * s * s) * K[7][c]};
+    double n[8];
+    hexa_to_nodes(q, n);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) k[a][c] *= mdt;
+    for (int a = 0; a < 8; ++a) k[a][c] = n[a];
+  }
   lam_el = lam_int / vol;
-  reg_el = reg / (double)GaussRule<NPE>::n;
+  reg_el = reg / 8.0;
 }
 
 }  // namespace fm
@@ -524,7 +677,9 @@ __device__ __forceinline__ float rsqrt_f(float x) {
   return y * fmaf(-0.5f * x, y * y, 1.5f);
 }
 
-// FP32 form of tet_metric.
+// G = J^-T J^-1 (femElement.cpp:192-232), the G:G term of tau, (mu/rho)^2 cI G:G
+// (eval_stabilization, src lines 336-377), and G's cofactor inverse
+// (eval_bulk_modulus, src lines 382-441).
 __device__ __forceinline__ void metric_f(const float inv[3][3], float nu, float cI, float G[3][3], float& t3,
                                          float iG[3][3]) {
 #pragma unroll
@@ -550,13 +705,14 @@ __device__ __forceinline__ void metric_f(const float inv[3][3], float nu, float 
   iG[2][2] = (m00 * m11 - m10 * m01) * idg;
 }
 
-template <int NPE, bool GEO = false>
+template <int NPE, class GEOS>
 __device__ __forceinline__ void supg_element_mixed(const DevProb& P, const ShapeTable<NPE, float>& tab,
                                                    const ShapeTable<NPE, double>& tabd, const float Xr[NPE][3],
                                                    const float U0[3], const float Ud[NPE][3], bool precise,
                                                    const double* sx, const double* sy, const double* sz,
                                                    const int ln[NPE], double k[NPE][3], double& lam_el,
-                                                   double& reg_el, const float* geo = nullptr, int64_t E = 0) {
+                                                   double& reg_el, const GEOS& geo) {
+  constexpr bool GEO = NPE == 8;
   const float rho = (float)P.rho, mu = (float)P.mu, alpha = (float)P.alpha, cI = (float)P.c_i;
   const float nu = (float)(P.mu / P.rho);
   const bool bbar = (P.ex_mask & 2) != 0;
@@ -583,7 +739,7 @@ __device__ __forceinline__ void supg_element_mixed(const DevProb& P, const Shape
   // per Gauss point: inverse Jacobian and det, FP32 or (precise) FP64; with
   // GEO read from the stored geometry (formed in FP64 for every element)
   auto geometry = [&](int g, float inv[3][3]) -> float {
-    if constexpr (GEO) return geo_at_f(geo, E, g, inv);
+    if constexpr (GEO) return geo.row(g, inv);
     if (precise) {
       double dN[NPE][3], invd[3][3];
 #pragma unroll
@@ -657,10 +813,6 @@ __device__ __forceinline__ void supg_element_mixed(const DevProb& P, const Shape
     metric_f(inv4, nu, cI, G4, t3_4, iG4);
   }
   float vol = 0.0f, lam_int = 0.0f, reg = 0.0f;
-  if constexpr (GEO) {
-    geo_prefetch(geo, E, 0);
-    geo_prefetch(geo, E, 1);
-  }
 #pragma unroll 1
   for (int g = 0; g < GaussRule<NPE>::n; ++g) {
     float inv[3][3], G[3][3], t3, iG[3][3];
@@ -677,10 +829,7 @@ __device__ __forceinline__ void supg_element_mixed(const DevProb& P, const Shape
         }
       t3 = t3_4;
     } else {
-      if constexpr (GEO) {
-        if (g + 2 < GaussRule<NPE>::n) geo_prefetch(geo, E, g + 2);
-      }
-      det = geometry(g, inv);
+      det = geometry((NPE == 8 && bbar ? 8 : 0) + g, inv);
       metric_f(inv, nu, cI, G, t3, iG);
     }
     float gd[NPE][3];
