@@ -222,6 +222,19 @@ void compute_mass(fm_problem* p) {
 // so it is first touched by the distributing threads, not zeroed first.
 static void sort_by_key(const hvec<uint64_t>& key, hvec<int64_t>& order) {
   const int64_t E = (int64_t)key.size();
+  struct KV {
+    uint64_t k;
+    int64_t i;
+    bool operator<(const KV& o) const { return k < o.k || (k == o.k && i < o.i); }
+  };
+  if (E < 65536) {  // the buckets alone would cost more
+    hvec<KV> kv(E);
+    for (int64_t i = 0; i < E; ++i) kv[i] = KV{key[i], i};
+    std::sort(kv.begin(), kv.end());
+    order.resize(E);
+    for (int64_t i = 0; i < E; ++i) order[i] = kv[i].i;
+    return;
+  }
   constexpr int NB = 1 << 16, SHIFT = 63 - 16;
   const int64_t hw = std::max<int64_t>(1, std::min<int64_t>(32, std::thread::hardware_concurrency()));
   const int64_t nw = std::min<int64_t>(hw, std::max<int64_t>(1, E / 65536));
@@ -249,11 +262,6 @@ static void sort_by_key(const hvec<uint64_t>& key, hvec<int64_t>& order) {
     }
     start[NB] = acc;
   }
-  struct KV {
-    uint64_t k;
-    int64_t i;
-    bool operator<(const KV& o) const { return k < o.k || (k == o.k && i < o.i); }
-  };
   hvec<KV> kv(E);
   run([&](int64_t w, int64_t b, int64_t e) {
     int64_t* h = &hist[(size_t)w * NB];
@@ -389,29 +397,73 @@ static inline uint64_t spread3(uint64_t v) {
   return v;
 }
 
+// Bounding box of n points (per-thread extremes combined: min / max are exact).
+static void bounding_box(const double* x, int64_t n, double lo[3], double hi[3]) {
+  std::vector<std::array<double, 6>> part(64, {1e300, 1e300, 1e300, -1e300, -1e300, -1e300});
+  parallel_blocks(n, [&](int64_t ib, int64_t ie, int w) {
+    std::array<double, 6>& b = part[w];
+    for (int64_t i = ib; i < ie; ++i)
+      for (int k = 0; k < 3; ++k) {
+        b[k] = std::min(b[k], x[i * 3 + k]);
+        b[3 + k] = std::max(b[3 + k], x[i * 3 + k]);
+      }
+  }, 1 << 14);
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = 1e300;
+    hi[k] = -1e300;
+  }
+  for (const auto& b : part)
+    for (int k = 0; k < 3; ++k) {
+      lo[k] = std::min(lo[k], b[k]);
+      hi[k] = std::max(hi[k], b[3 + k]);
+    }
+}
+
+// Node indices sorted by the Morton code of their coordinates (21 bits per
+// axis over the bounding cube, 10 below 65,536 nodes, which three counting
+// passes sort), ties in node order; a coordinate that is not finite counts as
+// the box's lower end.
+void morton_order_nodes(const double* x, int64_t n, hvec<int64_t>& order) {
+  double lo[3], hi[3];
+  bounding_box(x, n, lo, hi);
+  double span = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
+  if (!(span > 0 && span < 1e300)) span = 1.0;
+  const bool small = n < 65536;
+  const double cells = small ? 1023.0 : 2097151.0;
+  hvec<uint64_t> code(n);
+  parallel_blocks(n, [&](int64_t ib, int64_t ie, int) {
+    for (int64_t i = ib; i < ie; ++i) {
+      uint64_t q[3];
+      for (int k = 0; k < 3; ++k) {
+        const double t = (x[i * 3 + k] - lo[k]) / span;
+        q[k] = t > 0.0 ? (uint64_t)(std::min(t, 1.0) * cells) : 0u;
+      }
+      code[i] = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
+    }
+  }, 1 << 16);
+  if (small) {
+    hvec<int64_t> from(n);
+    order.resize(n);
+    for (int64_t i = 0; i < n; ++i) order[i] = i;
+    for (int shift = 0; shift < 30; shift += 10) {
+      int64_t at[1025] = {0};
+      for (int64_t i = 0; i < n; ++i) at[((code[i] >> shift) & 1023) + 1]++;
+      for (int k = 0; k < 1024; ++k) at[k + 1] += at[k];
+      from.swap(order);
+      for (int64_t i = 0; i < n; ++i) order[at[(code[from[i]] >> shift) & 1023]++] = from[i];
+    }
+    return;
+  }
+  sort_by_key(code, order);
+}
+
 // Element indices sorted by the Morton code of the element centroid (21
 // bits per axis over the mesh's bounding cube), ties in element order.
 void morton_order(const fm_problem* p, hvec<int64_t>& order) {
   const int npe = p->etype;
   const int64_t E = p->E, N = p->N;
-  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  {
-    // bounding box: per-thread extremes combined (min / max are exact)
-    std::vector<std::array<double, 6>> part(64, {1e300, 1e300, 1e300, -1e300, -1e300, -1e300});
-    parallel_blocks(N, [&](int64_t ib, int64_t ie, int w) {
-      std::array<double, 6>& b = part[w];
-      for (int64_t i = ib; i < ie; ++i)
-        for (int k = 0; k < 3; ++k) {
-          b[k] = std::min(b[k], p->coords[i * 3 + k]);
-          b[3 + k] = std::max(b[3 + k], p->coords[i * 3 + k]);
-        }
-    }, 1 << 14);
-    for (const auto& b : part)
-      for (int k = 0; k < 3; ++k) {
-        lo[k] = std::min(lo[k], b[k]);
-        hi[k] = std::max(hi[k], b[3 + k]);
-      }
-  }
+  double lo[3], hi[3];
+  bounding_box(p->coords.data(), N, lo, hi);
   double span = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
   if (!(span > 0)) span = 1.0;
   hvec<uint64_t> code(E);

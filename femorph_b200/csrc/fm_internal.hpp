@@ -225,4 +225,5 @@ constexpr int FM_GEO_PER_GP = 10;
 int build_layout(fm_problem* const* probs, int n, int tile_elems, int tile_nodes, Layout& L);
 int check_layout(const fm_problem* p, const Layout& L);
 void morton_order(const fm_problem* p, hvec<int64_t>& order);
+void morton_order_nodes(const double* x, int64_t n, hvec<int64_t>& order);
 }  // namespace fm

@@ -8,8 +8,11 @@
 // (the order of the reference's assembly loop, femSolver.cpp:446-459), the
 // right-hand side (sources in ELSOURCE row order, then the face Neumann
 // values, femSolver.cpp:478-558) and the Dirichlet rows.
-// Device: conjugate gradients with a Jacobi preconditioner.  Per iteration
-// three kernels: q = K p with the partial sums of p.q, the updates of x, r, z
+// Device: conjugate gradients with a Jacobi preconditioner, the whole solve in
+// one resident kernel (fm_poisson_resident.cuh) where every CTA's direction
+// fits its shared memory.  Larger systems (above about 20,000 rows an SM, or a
+// row with tens of thousands of columns) take three kernels an iteration:
+// q = K p with the partial sums of p.q, the updates of x, r, z
 // with the partial sums of r.z and r.r, and p = z + beta p; the last block of
 // the first two (ticket counter, no waiting) sums the block partials in block
 // order and forms alpha / beta, so every reduction has a fixed order and the
@@ -385,12 +388,13 @@ __global__ void __launch_bounds__(kThreads) avg_kernel(Cg c) {
   double s0, s1;
   if (last_block_sums(c, s, 0.0, &s0, &s1) && threadIdx.x == 0) c.scal[7] = s0 / (double)c.n;
 }
-// out = x - shift (shift = the average for FM_POISSON_PPE, else 0).
-__global__ void __launch_bounds__(kThreads) shift_kernel(const double* x, const double* scal, int ppe, int64_t n,
-                                                         double* out) {
+// out = x - shift (shift = the average for FM_POISSON_PPE, else 0) in node
+// order; row_of: the row of each node (null: the node's own number).
+__global__ void __launch_bounds__(kThreads) shift_kernel(const double* x, const int32_t* row_of, const double* scal,
+                                                         int ppe, int64_t n, double* out) {
   const double a = ppe ? scal[7] : 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = x[i] - a;
+    out[i] = x[row_of ? row_of[i] : i] - a;
 }
 
 // Element wall distance of evalDistanceFromPoissonSolution
@@ -424,6 +428,12 @@ __global__ void __launch_bounds__(kThreads) distance_kernel(const double* coords
   }
 }
 
+}  // namespace
+
+#include "fm_poisson_resident.cuh"
+
+namespace {
+
 struct DeviceRestore {
   int prev = -1;
   DeviceRestore() {
@@ -445,6 +455,9 @@ struct fm_poisson {
   // device arrays (one allocation)
   void* block = nullptr;
   Cg c{};
+  bool resident = false;  // solved by cg_resident_kernel over R (rows reordered)
+  CgResident R{};
+  int32_t* row_of = nullptr;
   double* coords = nullptr;
   int32_t* conn = nullptr;
   double* out = nullptr;   // x with the PPE average removed
@@ -729,20 +742,6 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
     if (nnz >= INT32_MAX) return fail(FM_ERR_INVALID, "matrix too large for 32-bit row offsets");
     rowp[v + 1] = (int32_t)nnz;
   }
-  fm::hvec<int32_t> col(nnz);
-  fm::hvec<double> val(nnz);
-  {
-    std::vector<std::thread> th;
-    for (int64_t kb = 0; kb < nblk; ++kb)
-      th.emplace_back([&, kb] {
-        const int64_t r0 = rowp[N * kb / nblk];
-        std::copy(bcol[kb].begin(), bcol[kb].end(), col.begin() + r0);
-        std::copy(bval[kb].begin(), bval[kb].end(), val.begin() + r0);
-        std::vector<int32_t>().swap(bcol[kb]);
-        std::vector<double>().swap(bval[kb]);
-      });
-    for (auto& x : th) x.join();
-  }
   // no Dirichlet row: K is singular (constants), so the right-hand side is
   // projected onto its range (zero sum) to make the system consistent
   if (d->n_dirichlet == 0) {
@@ -768,8 +767,58 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   if (device < 0 || device >= ndev) return fail(FM_ERR_INVALID, "bad device ordinal");
   DeviceRestore restore;
   PCK(cudaSetDevice(device));
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  // the resident kernel's blocks, when the device can hold one an SM
+  ResidentHost H;
+  {
+    int coop = 0, optin = 0, nb = 0;
+    cudaFuncAttributes fa;
+    PCK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+    PCK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    PCK(cudaFuncGetAttributes(&fa, resident_kernel(1024, 4)));  // the larger static part
+    const size_t limit = (size_t)optin - fa.sharedSizeBytes;
+    // node v's row, in the block of the row pass that formed it
+    auto row = [&](int64_t v) {
+      int64_t kb = v * nblk / N;
+      while (N * (kb + 1) / nblk <= v) ++kb;
+      const int32_t at = rowp[v] - rowp[N * kb / nblk];
+      return std::pair<const int32_t*, const double*>(bcol[kb].data() + at, bval[kb].data() + at);
+    };
+    if (coop) build_resident(d->coords, N, rowp, row, sms, limit, H);
+    if (H.fits) {
+      // the attribute is process-wide: always the maximum, whatever this solver needs
+      const ResidentKernel k = resident_kernel(H.R.threads, H.R.vectors);
+      PCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+      PCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, H.R.threads, H.R.smem));
+      H.fits = nb > 0 && (int64_t)nb * sms >= H.R.ctas;
+    }
+    if (H.fits) {
+      auto reorder = [&](std::vector<double>& v) {
+        std::vector<double> t(N);
+        for (int64_t i = 0; i < N; ++i) t[i] = v[H.node_of[i]];
+        v.swap(t);
+      };
+      reorder(dinv);
+      reorder(bvec);
+      reorder(xinit);
+    }
+  }
+  fm::hvec<int32_t> col(H.fits ? 0 : nnz);
+  fm::hvec<double> val(H.fits ? 0 : nnz);
+  if (!H.fits) {
+    std::vector<std::thread> th;
+    for (int64_t kb = 0; kb < nblk; ++kb)
+      th.emplace_back([&, kb] {
+        const int64_t r0 = rowp[N * kb / nblk];
+        std::copy(bcol[kb].begin(), bcol[kb].end(), col.begin() + r0);
+        std::copy(bval[kb].begin(), bval[kb].end(), val.begin() + r0);
+      });
+    for (auto& x : th) x.join();
+  }
   fm_poisson* s = new fm_poisson();
   s->device = device;
+  s->resident = H.fits;
   s->npe = npe;
   s->problem = d->problem;
   s->N = N;
@@ -791,8 +840,6 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   for (int64_t k = 0; k < d->n_dirichlet; ++k) s->h_dir[d->dir_node[k]] = 1.0;
   s->view = fm::PoissonHostView{N, E, npe, d->problem, s->h_coords.data(), s->h_conn.data(), s->h_diff.data(),
                                 s->h_src.data(), s->h_neu.data(), s->h_dir.data()};
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   s->blocks = (int)std::max<int64_t>(1, std::min<int64_t>((N + kThreads - 1) / kThreads, (int64_t)sms * 8));
   s->eblocks = (int)std::max<int64_t>(1, std::min<int64_t>((E + kThreads - 1) / kThreads, (int64_t)sms * 8));
   // one device allocation carved into the arrays (256-byte aligned)
@@ -802,11 +849,15 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
     total = off + std::max<size_t>(bytes, 16);
     return off;
   };
-  const size_t o_rowp = take((N + 1) * 4), o_col = take(nnz * 4), o_val = take(nnz * 8), o_dinv = take(N * 8),
-               o_b = take(N * 8), o_xi = take(N * 8), o_x = take(N * 8), o_r = take(N * 8), o_z = take(N * 8), o_p = take(N * 8),
+  const size_t o_rowp = take(H.fits ? 0 : (N + 1) * 4), o_col = take(H.fits ? 0 : nnz * 4), o_val = take(H.fits ? 0 : nnz * 8), o_dinv = take(N * 8),
+               o_b = take(N * 8), o_xi = take(N * 8), o_x = take(N * 8), o_r = take(N * 8), o_z = take(N * 8), o_p = take(H.fits ? 0 : N * 8),
                o_q = take(N * 8), o_part = take((size_t)2 * s->blocks * 8), o_scal = take(8 * 8), o_ctl = take(8 * 4),
                o_out = take(N * 8), o_coords = take(N * 3 * 8), o_conn = take(E * npe * 4),
                o_dist = take(d->problem == FM_POISSON_DISTANCE ? E * 8 : 16);
+  const size_t o_row_of = take(H.fits ? N * 4 : 0), o_row0 = take(H.row0.size() * 4), o_halo0 = take(H.halo0.size() * 4),
+               o_halo = take(H.halo.size() * 4), o_slice0 = take(H.slice0.size() * 4),
+               o_slice_at = take(H.slice_at.size() * 4), o_rval = take(H.val.size() * 8),
+               o_rcol = take(H.col.size() * 2), o_parts = take(H.fits ? (size_t)H.R.ctas * 32 : 0), o_arrived = take(8);
   if (cudaMalloc(&s->block, total) != cudaSuccess) {
     cudaGetLastError();
     fm_poisson_destroy(s);
@@ -833,6 +884,19 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   s->coords = reinterpret_cast<double*>(base + o_coords);
   s->conn = reinterpret_cast<int32_t*>(base + o_conn);
   s->dist = reinterpret_cast<double*>(base + o_dist);
+  if (H.fits) {
+    s->R = H.R;
+    s->row_of = reinterpret_cast<int32_t*>(base + o_row_of);
+    s->R.row0 = reinterpret_cast<int32_t*>(base + o_row0);
+    s->R.halo0 = reinterpret_cast<int32_t*>(base + o_halo0);
+    s->R.halo = reinterpret_cast<int32_t*>(base + o_halo);
+    s->R.slice0 = reinterpret_cast<int32_t*>(base + o_slice0);
+    s->R.slice_at = reinterpret_cast<int32_t*>(base + o_slice_at);
+    s->R.val = reinterpret_cast<double*>(base + o_rval);
+    s->R.col = reinterpret_cast<uint16_t*>(base + o_rcol);
+    s->R.partials = reinterpret_cast<double2*>(base + o_parts);
+    s->R.arrived = reinterpret_cast<unsigned long long*>(base + o_arrived);
+  }
   auto fail_free = [&](const char* what, cudaError_t e) {
     std::string m = std::string(what) + ": " + cudaGetErrorString(e);
     fm_poisson_destroy(s);
@@ -848,9 +912,20 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   auto up = [&](void* dst, const void* src, size_t bytes) {
     return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
   };
-  if (e == cudaSuccess) e = up((void*)c.rowp, rowp.data(), (N + 1) * 4);
-  if (e == cudaSuccess) e = up((void*)c.col, col.data(), nnz * 4);
-  if (e == cudaSuccess) e = up((void*)c.val, val.data(), nnz * 8);
+  if (H.fits) {
+    e = up((void*)s->row_of, H.row_of.data(), N * 4);
+    if (e == cudaSuccess) e = up((void*)s->R.row0, H.row0.data(), H.row0.size() * 4);
+    if (e == cudaSuccess) e = up((void*)s->R.halo0, H.halo0.data(), H.halo0.size() * 4);
+    if (e == cudaSuccess) e = up((void*)s->R.halo, H.halo.data(), H.halo.size() * 4);
+    if (e == cudaSuccess) e = up((void*)s->R.slice0, H.slice0.data(), H.slice0.size() * 4);
+    if (e == cudaSuccess) e = up((void*)s->R.slice_at, H.slice_at.data(), H.slice_at.size() * 4);
+    if (e == cudaSuccess) e = up((void*)s->R.val, H.val.data(), H.val.size() * 8);
+    if (e == cudaSuccess) e = up((void*)s->R.col, H.col.data(), H.col.size() * 2);
+  } else {
+    e = up((void*)c.rowp, rowp.data(), (N + 1) * 4);
+    if (e == cudaSuccess) e = up((void*)c.col, col.data(), nnz * 4);
+    if (e == cudaSuccess) e = up((void*)c.val, val.data(), nnz * 8);
+  }
   if (e == cudaSuccess) e = up((void*)c.dinv, dinv.data(), N * 8);
   if (e == cudaSuccess) e = up((void*)c.b, bvec.data(), N * 8);
   if (e == cudaSuccess) e = up((void*)c.xinit, xinit.data(), N * 8);
@@ -905,35 +980,43 @@ FM_API int fm_poisson_solve(fm_poisson* s, double rel_tol, int32_t max_iter, int
   PCK(cudaMemcpyAsync(c.ctl, ctl_init, sizeof(ctl_init), cudaMemcpyHostToDevice, st));
   PCK(cudaMemcpyAsync(c.scal + 5, sc, sizeof(sc), cudaMemcpyHostToDevice, st));
   PCK(cudaEventRecord(s->ev0, st));
-  cg_init_kernel<<<G, kThreads, 0, st>>>(c);
-  PCK(cudaGetLastError());
-  if (!s->graph) {
-    cudaGraph_t g = nullptr;
-    PCK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    for (int i = 0; i < FM_CG_GRAPH; ++i) {
-      cg_spmv_kernel<<<G, kThreads, 0, st>>>(c);
-      cg_update_kernel<<<G, kThreads, 0, st>>>(c);
-      cg_direction_kernel<<<G, kThreads, 0, st>>>(c);
+  if (s->resident) {
+    PCK(cudaMemsetAsync(s->R.arrived, 0, sizeof(*s->R.arrived), st));
+    Cg cc = c;
+    void* args[] = {&cc, &s->R};
+    PCK(cudaLaunchCooperativeKernel((const void*)resident_kernel(s->R.threads, s->R.vectors), dim3(s->R.ctas), dim3(s->R.threads), args,
+                                    s->R.smem, st));
+  } else {
+    cg_init_kernel<<<G, kThreads, 0, st>>>(c);
+    PCK(cudaGetLastError());
+    if (!s->graph) {
+      cudaGraph_t g = nullptr;
+      PCK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+      for (int i = 0; i < FM_CG_GRAPH; ++i) {
+        cg_spmv_kernel<<<G, kThreads, 0, st>>>(c);
+        cg_update_kernel<<<G, kThreads, 0, st>>>(c);
+        cg_direction_kernel<<<G, kThreads, 0, st>>>(c);
+      }
+      const cudaError_t ce = cudaStreamEndCapture(st, &g);
+      if (ce != cudaSuccess) return fail(FM_ERR_CUDA, std::string("CG graph capture: ") + cudaGetErrorString(ce));
+      const cudaError_t ie = cudaGraphInstantiate(&s->graph, g, 0);
+      cudaGraphDestroy(g);
+      if (ie != cudaSuccess) {
+        s->graph = nullptr;
+        return fail(FM_ERR_CUDA, std::string("CG graph instantiate: ") + cudaGetErrorString(ie));
+      }
     }
-    const cudaError_t ce = cudaStreamEndCapture(st, &g);
-    if (ce != cudaSuccess) return fail(FM_ERR_CUDA, std::string("CG graph capture: ") + cudaGetErrorString(ce));
-    const cudaError_t ie = cudaGraphInstantiate(&s->graph, g, 0);
-    cudaGraphDestroy(g);
-    if (ie != cudaSuccess) {
-      s->graph = nullptr;
-      return fail(FM_ERR_CUDA, std::string("CG graph instantiate: ") + cudaGetErrorString(ie));
+    // replay blocks of iterations until the device raises its done flag
+    for (int64_t launched = 0;; launched += FM_CG_GRAPH) {
+      PCK(cudaMemcpyAsync(s->h_ctl, c.ctl, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+      PCK(cudaStreamSynchronize(st));
+      if (s->h_ctl[0] || launched > (int64_t)max_iter + FM_CG_GRAPH) break;
+      PCK(cudaGraphLaunch(s->graph, st));
     }
-  }
-  // replay blocks of iterations until the device raises its done flag
-  for (int64_t launched = 0;; launched += FM_CG_GRAPH) {
-    PCK(cudaMemcpyAsync(s->h_ctl, c.ctl, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    PCK(cudaStreamSynchronize(st));
-    if (s->h_ctl[0] || launched > (int64_t)max_iter + FM_CG_GRAPH) break;
-    PCK(cudaGraphLaunch(s->graph, st));
   }
   PCK(cudaEventRecord(s->ev1, st));
   avg_kernel<<<G, kThreads, 0, st>>>(c);
-  shift_kernel<<<G, kThreads, 0, st>>>(c.x, c.scal, s->problem == FM_POISSON_PPE, s->N, s->out);
+  shift_kernel<<<G, kThreads, 0, st>>>(c.x, s->row_of, c.scal, s->problem == FM_POISSON_PPE, s->N, s->out);
   if (s->problem == FM_POISSON_DISTANCE)
     distance_kernel<<<s->eblocks, kThreads, 0, st>>>(s->coords, s->conn, s->npe, s->E, s->out, s->dist);
   PCK(cudaGetLastError());
@@ -946,6 +1029,7 @@ FM_API int fm_poisson_solve(fm_poisson* s, double rel_tol, int32_t max_iter, int
   if (iterations) *iterations = s->h_ctl[1];
   const double bb = s->bb;
   if (rel_residual) *rel_residual = bb > 0.0 ? std::sqrt(s->h_scal[4] / bb) : 0.0;
+  if (s->h_ctl[2] == 2) return fail(FM_ERR_TIMEOUT, "CG: an exchange between the resident blocks did not complete");
   s->has_result = true;
   if (s->h_ctl[2]) return fail(FM_ERR_DIVERGED, "CG breakdown (matrix not positive definite on the search direction, or NaN)");
   return FM_OK;
