@@ -48,6 +48,12 @@ cudaError_t launch_supg_geo(const DevBatch& B, int tile0, int ntiles, int tn_max
 cudaError_t launch_supg_pressure(const DevBatch& B, int tn_max, int npe, double* pres, cudaStream_t s);
 cudaError_t launch_supg_stats(const DevBatch& B, int tile0, int ntiles, int tn_max, int npe, double* out,
                               cudaStream_t s);
+cudaError_t launch_read_nodes(const DevBatch& B, int64_t nb, const int32_t* slot, int64_t n, int fixed, double* u,
+                              double* p, cudaStream_t s);
+cudaError_t launch_read_subscales(const DevBatch& B, int64_t eb, const int32_t* slot, int64_t n, bool centroid,
+                                  double* out, cudaStream_t s);
+cudaError_t launch_read_pair(const double* a, const double* c, const int32_t* slot, int64_t n, double* out,
+                             cudaStream_t s);
 cudaError_t launch_velocity_extrema(const DevBatch& B, int64_t node_begin, int64_t n_nodes, int glob_fixed, int blocks,
                                     double* out, cudaStream_t s);
 
@@ -163,6 +169,7 @@ enum PoolId { P_NODE, P_ELEM, P_TILE, P_TNODE, P_TCOL, P_TINC, P_TOFF, P_SLOT, P
               P_COUNT };
 
 struct Placement {
+  bool elem_slots = false;  // d_elem_slot of this problem is filled
   fm_problem* p = nullptr;
   int64_t off[P_COUNT] = {0};
   int64_t len[P_COUNT] = {0};
@@ -203,6 +210,11 @@ struct fm_batch {
   cudaGraphExec_t graph = nullptr;
   int graph_iters = 0;
   double* d_scratch = nullptr;
+  // read-back (fm_problem_get_state): batch node / element slot of each
+  // problem node / element, relative to the problem's range, and a piece of
+  // the output in the caller's layout
+  int32_t *d_node_slot = nullptr, *d_elem_slot = nullptr;
+  double* d_out = nullptr;
   double* d_stats = nullptr;   // per-CTA partial results of the log reductions
   // partition parts (fm_problem_partition): the batch holds x_slices parts
   // of one partition; external when the others live in other processes,
@@ -329,6 +341,10 @@ static void pool_sizes(const fm_problem* p, const Layout& L, int64_t len[P_COUNT
 }
 static const int64_t kAlign[P_COUNT] = {1, ELEM_ALIGN, 1, 1, 1, 8, 1, 1, 1, 1, 1, 1, 1, 1};
 
+// Doubles of the read-back piece: all of a small batch's nodal output, at most
+// 32 MB.
+static int64_t out_doubles(int64_t nodes) { return std::max<int64_t>(4096, std::min<int64_t>(4 * nodes, 1 << 22)); }
+
 // Allocates the device arrays for the given pool capacities.
 static int allocate(fm_batch* b, const int64_t cap[P_COUNT]) {
   for (int k = 0; k < P_COUNT; ++k) b->pools[k].init(cap[k]);
@@ -370,6 +386,9 @@ static int allocate(fm_batch* b, const int64_t cap[P_COUNT]) {
     total = 0;
     for (double** q : {&x, &y, &z, &su, &sv, &sw, &sp, &pu, &pv, &pw, &pp, &ms}) A((void**)q, NN * sizeof(double));
     A((void**)&nbc, NN * sizeof(int32_t));
+    A((void**)&b->d_node_slot, NN * sizeof(int32_t));
+    A((void**)&b->d_elem_slot, NE * sizeof(int32_t));
+    A((void**)&b->d_out, (size_t)out_doubles(NN) * sizeof(double));
     A((void**)&conn, (size_t)NE * b->npe * sizeof(uint16_t));
     if (b->solver == FM_SOLVER_VMS && b->precision == FM_MIXED) {
       A((void**)&D.sdus32, (size_t)NE * 12 * sizeof(float));
@@ -668,6 +687,7 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
     }
   r = r ? r : put(const_cast<double*>(D.mass), noff, hm.data(), N, s);
   r = r ? r : put(const_cast<int32_t*>(D.node_bc), noff, hbc.data(), N, s);
+  r = r ? r : put(b->d_node_slot, noff, nn.data(), N, s);
   {
     std::vector<BCRec> recs(p->recs);
     for (BCRec& q : recs)
@@ -849,7 +869,7 @@ static int64_t pool_bytes(const int64_t cap[P_COUNT], int solver, int npe, int p
   const int64_t NN = std::max<int64_t>(cap[P_NODE], 1);
   const int64_t NE = (std::max<int64_t>(cap[P_ELEM], 1) + ELEM_ALIGN - 1) / ELEM_ALIGN * ELEM_ALIGN;
   auto at_least = [](int64_t v, int64_t m) { return std::max<int64_t>(v, m); };
-  int64_t b = NN * (12 * 8 + 4) + NE * npe * 2;
+  int64_t b = NN * (12 * 8 + 8) + NE * (npe * 2 + 4) + out_doubles(NN) * 8;
   if (solver == FM_SOLVER_VMS && prec == FM_MIXED) b += NE * 12 * 4;
   else if (solver == FM_SOLVER_VMS || history) b += NE * (solver == FM_SOLVER_VMS ? 12 : 3 * npe) * 8;
   if (solver == FM_SOLVER_SUPG) b += NE * 3 * 8;
@@ -861,6 +881,22 @@ static int64_t pool_bytes(const int64_t cap[P_COUNT], int solver, int npe, int p
   const int64_t NP = at_least(cap[P_PROB], 1);
   b += NP * ((int64_t)sizeof(DevProb) + (int64_t)sizeof(DevProbState) + 4 + 64);
   return b;
+}
+
+// Touches the pages of a large output on a few host threads (a fresh
+// allocation is populated page by page on first use: 2.7 of the 4.2 ms that
+// copying 29 MB into one takes on a single thread).  The contents stay.
+static void touch_pages(void* p, size_t bytes) {
+  constexpr size_t page = 4096, each = 1 << 21;
+  const size_t nt = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), bytes / each});
+  if (nt < 2) return;
+  std::vector<std::thread> th;
+  for (size_t t = 0; t < nt; ++t)
+    th.emplace_back([=] {
+      volatile char* q = static_cast<char*>(p);
+      for (size_t i = bytes * t / nt; i < bytes * (t + 1) / nt; i += page) q[i] = q[i];
+    });
+  for (auto& x : th) x.join();
 }
 
 extern "C" {
@@ -1015,7 +1051,7 @@ int fm_batch_estimate_bytes(fm_problem* const* probs, int32_t n, const fm_tuning
   // tiles, incidence lists and interface partials: ~40 B per element
   const int64_t per_e = (int64_t)npe * 2 + (vms ? (mixed ? 48 : 96) : (3 * npe * 8 + 24)) + 40 +
                         (!vms && npe == 8 ? 8 * FM_GEO_PER_GP * (mixed ? 4 : 8) : 0);
-  *bytes = N * 100 + E * per_e + (16 << 20);
+  *bytes = N * 104 + E * (per_e + 4) + out_doubles(N) * 8 + (16 << 20);
   return FM_OK;
 }
 
@@ -1684,76 +1720,73 @@ int fm_problem_get_state(fm_problem* p, double* u, double* pres, double* elem3, 
   if (!b) return fail(FM_ERR_INVALID, "problem is not in a batch");
   CK(cudaSetDevice(b->device));
   CK(cudaStreamSynchronize(b->stream));
-  const Placement& pl = b->slots[p->index];
+  Placement& pl = b->slots[p->index];
   const int64_t nb = pl.off[P_NODE], eb = pl.off[P_ELEM];
   const int64_t N = p->N, E = p->E;
-  const std::vector<int32_t>& nn = pl.L->node_new[0];
-  const auto& eo = pl.L->elem_old[0];
-  const int64_t EC = (int64_t)eo.size();
-  std::vector<double> tmp(N);
-  double* cols[4] = {b->D.su, b->D.sv, b->D.sw, b->D.sp};
-  if (u) {
-    for (int c = 0; c < 3; ++c) {
-      CK(cudaMemcpy(tmp.data(), cols[c] + nb, sizeof(double) * N, cudaMemcpyDeviceToHost));
-      for (int64_t i = 0; i < N; ++i) u[i * 3 + c] = tmp[nn[i]];
-    }
-    if (b->solver == FM_SOLVER_SUPG && p->params.glob_fixed)
-      for (int64_t i = 0; i < N; ++i)
-        for (int c = 0; c < 3; ++c)
-          if (p->params.glob_fixed & (1 << c)) u[i * 3 + c] = 0.0;
+  const DevBatch& D = b->D;
+  const bool vms = b->solver == FM_SOLVER_VMS;
+  const int64_t out_len = out_doubles(std::max<int64_t>(b->pools[P_NODE].cap, 1));
+  if (((vms && sdus) || elem3 || (!vms && pres)) && !pl.elem_slots) {
+    const auto& eo = pl.L->elem_old[0];
+    hvec<int32_t> slot(E);
+    parallel_blocks((int64_t)eo.size(), [&](int64_t kb, int64_t ke, int) {
+      for (int64_t k = kb; k < ke; ++k)
+        if (eo[k] >= 0) slot[eo[k]] = (int32_t)k;
+    }, 1 << 16);
+    CK(cudaMemcpy(b->d_elem_slot + eb, slot.data(), sizeof(int32_t) * E, cudaMemcpyHostToDevice));
+    pl.elem_slots = true;
   }
-  if (b->solver == FM_SOLVER_VMS) {
-    if (pres) {
-      CK(cudaMemcpy(tmp.data(), cols[3] + nb, sizeof(double) * N, cudaMemcpyDeviceToHost));
-      for (int64_t i = 0; i < N; ++i) pres[i] = tmp[nn[i]];
-    }
-    if (elem3 || sdus) {
-      std::vector<double> h((size_t)E * 12), col(EC);
-      std::vector<float> colf(b->D.sdus32 ? EC : 0);
-      for (int q = 0; q < 12; ++q) {
-        if (b->D.sdus32) {
-          CK(cudaMemcpy(colf.data(), b->D.sdus32 + (int64_t)q * b->D.E + eb, sizeof(float) * EC,
-                        cudaMemcpyDeviceToHost));
-          for (int64_t k = 0; k < EC; ++k) col[k] = colf[k];
-        } else {
-          CK(cudaMemcpy(col.data(), b->D.sdus + (int64_t)q * b->D.E + eb, sizeof(double) * EC,
-                        cudaMemcpyDeviceToHost));
-        }
-        for (int64_t k = 0; k < EC; ++k)
-          if (eo[k] >= 0) h[(size_t)eo[k] * 12 + q] = col[k];
+  // pieces of the output formed on the device in the caller's layout (on the
+  // legacy stream, as the copies) and copied out in one go each; the
+  // caller's pages are touched meanwhile
+  const int32_t* ns = b->d_node_slot + nb;
+  const int32_t* es = b->d_elem_slot + eb;
+  if (u || (vms && pres)) {
+    const int gf = vms ? 0 : p->params.glob_fixed;
+    const int64_t step = out_len / 4;
+    for (int64_t i = 0; i < N; i += step) {
+      const int64_t n = std::min(step, N - i);
+      double* dp = b->d_out + 3 * n;
+      CK(launch_read_nodes(D, nb, ns + i, n, gf, u ? b->d_out : nullptr, vms && pres ? dp : nullptr, 0));
+      if (i == 0) {
+        if (u) touch_pages(u, sizeof(double) * N * 3);
+        if (vms && pres) touch_pages(pres, sizeof(double) * N);
       }
-      if (sdus) memcpy(sdus, h.data(), sizeof(double) * E * 12);
-      if (elem3)
-        for (int64_t e = 0; e < E; ++e)
-          for (int c = 0; c < 3; ++c) {
-            // eval_centroid_subgrid (src lines 713-724): sum_a sdu[a][c]*0.25
-            double s = 0.0;
-            for (int g = 0; g < 4; ++g) s += h[(size_t)e * 12 + g * 3 + c] * 0.25;
-            elem3[e * 3 + c] = s;
-          }
+      if (u) CK(cudaMemcpy(u + 3 * i, b->d_out, sizeof(double) * n * 3, cudaMemcpyDeviceToHost));
+      if (vms && pres) CK(cudaMemcpy(pres + i, dp, sizeof(double) * n, cudaMemcpyDeviceToHost));
     }
+  }
+  // width values an element, formed by launch(first element, count)
+  auto elements = [&](double* to, int width, auto&& launch) -> int {
+    const int64_t step = out_len / width;
+    for (int64_t e = 0; e < E; e += step) {
+      const int64_t n = std::min(step, E - e);
+      CK(launch(e, n));
+      if (e == 0) touch_pages(to, sizeof(double) * E * width);
+      CK(cudaMemcpy(to + e * width, b->d_out, sizeof(double) * n * width, cudaMemcpyDeviceToHost));
+    }
+    return FM_OK;
+  };
+  int r = FM_OK;
+  if (vms) {
+    if (sdus)
+      r = elements(sdus, 12, [&](int64_t e, int64_t n) { return launch_read_subscales(D, eb, es + e, n, false, b->d_out, 0); });
+    if (!r && elem3)
+      r = elements(elem3, 3, [&](int64_t e, int64_t n) { return launch_read_subscales(D, eb, es + e, n, true, b->d_out, 0); });
   } else {
     if (pres) {
-      cudaError_t e = launch_supg_pressure(b->D, b->tn_max, b->npe, b->d_scratch, b->stream);
+      cudaError_t e = launch_supg_pressure(D, b->tn_max, b->npe, b->d_scratch, 0);
       if (e != cudaSuccess) return fail(FM_ERR_CUDA, cudaGetErrorString(e));
-      CK(cudaStreamSynchronize(b->stream));
-      std::vector<double> col(EC);
-      CK(cudaMemcpy(col.data(), b->d_scratch + eb, sizeof(double) * EC, cudaMemcpyDeviceToHost));
-      for (int64_t k = 0; k < EC; ++k)
-        if (eo[k] >= 0) pres[eo[k]] = col[k];
+      r = elements(pres, 1, [&](int64_t e0, int64_t n) {
+        return launch_read_pair(b->d_scratch + eb, nullptr, es + e0, n, b->d_out, 0);
+      });
     }
-    if (elem3) {
-      std::vector<double> c1(EC), c2(EC);
-      CK(cudaMemcpy(c1.data(), b->D.el_lam + eb, sizeof(double) * EC, cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(c2.data(), b->D.el_reg + eb, sizeof(double) * EC, cudaMemcpyDeviceToHost));
-      for (int64_t k = 0; k < EC; ++k) {
-        if (eo[k] < 0) continue;
-        elem3[(int64_t)eo[k] * 2 + 0] = c1[k];
-        elem3[(int64_t)eo[k] * 2 + 1] = c2[k];
-      }
-    }
+    if (!r && elem3)
+      r = elements(elem3, 2, [&](int64_t e0, int64_t n) {
+        return launch_read_pair(D.el_lam + eb, D.el_reg + eb, es + e0, n, b->d_out, 0);
+      });
   }
-  return FM_OK;
+  return r;
 }
 
 }  // extern "C"
