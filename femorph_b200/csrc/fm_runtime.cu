@@ -269,14 +269,48 @@ static int put(T* dev_base, int64_t off, const T* src, int64_t n, cudaStream_t s
   return FM_OK;
 }
 
-// Default launch shape (measured on the 96^3 cavity and the hexa channel):
-// VMS FP64 1024-tet tiles (3 CTAs/SM, register bound), VMS mixed 512-tet
-// tiles (4 CTAs/SM fit the shared memory), SUPG hexa8 384 elements.
+// Elements a tile when the caller gives none.  A problem of many tiles takes
+// full ones (1024 tets, VMS mixed 512, 384 hexa: the larger a tile, the fewer
+// nodes are staged and summed twice).  A problem of at most four waves of
+// CTAs takes tiles that fill its waves, so that no SM idles while others walk
+// a long tile: tiles of whole 128-element chunks below 512, of 32-element
+// steps above, at most 640 tets.  16^3 cavity (24,576 tets): 256 against 1024
+// a tile 20.6 against 43.0 us an iteration; 24^3: 256, 24.6 against 41.4;
+// 30^3: 384, 30.8 against 47.3; 36^3: 640, 44.1 against 47.3; 44^3: 576, 69.3
+// against 83.0; mixed 24^3: 256 against 512 22.6 against 28.7; hexa 93x37x29:
+// 256 against 384 68 against 78.  Not below 256, where a batch of many small
+// problems would pay for the extra interface nodes: 32 cavities of 8..24
+// cells a side take 148.7 us FP64 and 119.6 us mixed (full tiles 157.7 and
+// 118.6; with 128 as the least 170.3 and 140.3).  It depends on the problem
+// alone (its size, and the SM count of a B200 as a constant): a problem's
+// results do not depend on what else is in its batch.
+static int auto_tile_elems(int solver, int npe, int precision, int threads, int64_t E) {
+  const bool vms_mixed = solver == FM_SOLVER_VMS && precision == FM_MIXED;
+  const int full = npe == 8 ? 384 : vms_mixed ? 512 : 1024;
+  if (threads != 128) return full;
+  const int64_t slots = 148 * (vms_mixed ? 4 : 3);  // resident CTAs
+  const int64_t waves = std::max<int64_t>(1, (E + slots * std::min(full, 640) - 1) / (slots * std::min(full, 640)));
+  if (waves > 4) return full;
+  const int64_t te = (E + slots * waves - 1) / (slots * waves);
+  const int64_t up = te < 512 ? std::max<int64_t>(256, (te + 127) / 128 * 128) : (te + 31) / 32 * 32;
+  return (int)std::min<int64_t>(up, full);
+}
+
+// Default launch shape.  tile_nodes: what still lets the CTAs that the kernels'
+// registers allow (VMS FP64 three, mixed four) fit an SM's shared memory; the
+// tiles of a mesh whose cells do not halve evenly have up to 500 nodes at
+// 1024 tets, and one such tile used to cost every CTA of the launch its third
+// neighbour (32 cavities of 8..48 cells a side, full tiles: 580 -> 491 us a
+// step).
 static void default_tuning(int solver, int npe, int precision, fm_tuning& t) {
   if (t.threads != 128 && t.threads != 256) t.threads = 128;
   const bool vms_mixed = solver == FM_SOLVER_VMS && precision == FM_MIXED;
-  if (t.tile_elems <= 0) t.tile_elems = (npe == 8) ? 384 : (vms_mixed ? 512 : 1024);
-  if (t.tile_nodes <= 0) t.tile_nodes = (npe == 8) ? 640 : (vms_mixed ? 256 : 512);
+  if (t.tile_elems < 0) t.tile_elems = 0;  // by the problem (auto_tile_elems)
+  if (t.tile_nodes <= 0) {
+    if (npe == 8) t.tile_nodes = 640;
+    else if (solver == FM_SOLVER_VMS && t.threads == 128) t.tile_nodes = vms_mixed ? 228 : 352;
+    else t.tile_nodes = vms_mixed ? 256 : 512;
+  }
   if (t.tile_nodes > 4096) t.tile_nodes = 4096;
   if (solver == FM_SOLVER_VMS && t.tile_nodes > FM_MAX_TILE_NODES) t.tile_nodes = FM_MAX_TILE_NODES;
   if (t.graph_steps < 0) t.graph_steps = 0;
@@ -285,7 +319,10 @@ static void default_tuning(int solver, int npe, int precision, fm_tuning& t) {
 // Builds (or reuses) the problem's own tile layout for the given tile sizes.
 // Touches only this problem, so different problems may be prepared on
 // different host threads while a batch runs.
-static int prepare(fm_problem* p, int te, int tn, std::shared_ptr<Layout>* out) {
+static int prepare(fm_problem* p, const fm_tuning& t, std::shared_ptr<Layout>* out) {
+  const int te = t.tile_elems > 0 ? t.tile_elems
+                                  : auto_tile_elems(p->params.solver, p->etype, p->params.precision, t.threads, p->E);
+  const int tn = t.tile_nodes;
   if (p->layout && p->layout_te == te && p->layout_tn == tn) {
     *out = p->layout;
     return FM_OK;
@@ -841,7 +878,9 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
 
 // Pool capacities of fm_batch_create_empty for the given maxima.  Tiles hold
 // about tile_elems elements (at least half that unless tile_nodes binds
-// first); each tile start is padded to a multiple of 32 element slots;
+// first).  Without tile_elems (te 0) small problems take small tiles
+// (auto_tile_elems): at most one per 256 elements, and at most four waves of
+// CTAs a problem beside full tiles.  Each tile start is padded to a multiple of 32 element slots;
 // tile-boundary nodes appear once per tile that touches them (about 1.4 N
 // for tet tiles of 1024 elements) and own one interface partial slot each;
 // BC records exist for boundary nodes only.  A problem that needs more than
@@ -849,9 +888,12 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
 static void capacity_pools(const fm_capacity* cap, int te, int64_t c[P_COUNT]) {
   const int64_t E = cap->max_elems, N = cap->max_nodes, P = cap->max_problems, npe = cap->elem_type;
   c[P_NODE] = N;
+  const bool by_problem = te <= 0;
+  if (by_problem) te = auto_tile_elems(cap->solver, (int)npe, cap->precision, 128, (int64_t)1 << 40);  // full tiles
   c[P_TILE] = E / std::max<int64_t>(1, te / 2) + 2 * P;
+  if (by_problem) c[P_TILE] = std::min<int64_t>(E / 128 + 2 * P, c[P_TILE] + 4096 * P);
   c[P_ELEM] = E + 2 * P * ELEM_ALIGN + c[P_TILE] * ELEM_ALIGN;
-  c[P_TNODE] = 2 * N + 16 * c[P_TILE];
+  c[P_TNODE] = 2 * N + (by_problem ? 48 : 16) * c[P_TILE];
   c[P_TCOL] = c[P_TILE] * 130;
   c[P_TINC] = npe * E + 16 * c[P_TILE] + 16 * P;
   c[P_TOFF] = c[P_TNODE] + c[P_TILE];
@@ -1020,7 +1062,7 @@ int fm_problem_prepare(fm_problem* p, const fm_tuning* tuning) {
   if (tuning) t = *tuning;
   default_tuning(p->params.solver, p->etype, p->params.precision, t);
   std::shared_ptr<Layout> L;
-  return prepare(p, t.tile_elems, t.tile_nodes, &L);
+  return prepare(p, t, &L);
 }
 
 int fm_problem_check_layout(fm_problem* p, const fm_tuning* tuning) {
@@ -1031,7 +1073,7 @@ int fm_problem_check_layout(fm_problem* p, const fm_tuning* tuning) {
   if (tuning) t = *tuning;
   default_tuning(p->params.solver, p->etype, p->params.precision, t);
   std::shared_ptr<Layout> L;
-  int r = prepare(p, t.tile_elems, t.tile_nodes, &L);
+  int r = prepare(p, t, &L);
   if (r) return r;
   return check_layout(p, *L);
 }
@@ -1127,7 +1169,7 @@ int fm_batch_create(fm_problem* const* probs, int32_t n, const fm_tuning* tuning
   int64_t cap[P_COUNT] = {0};
   std::vector<std::shared_ptr<Layout>> preps(n);
   for (int i = 0; i < n; ++i) {
-    r = prepare(probs[i], b->tune.tile_elems, b->tune.tile_nodes, &preps[i]);
+    r = prepare(probs[i], b->tune, &preps[i]);
     if (r) {
       delete b;
       return r;
@@ -1216,7 +1258,7 @@ int fm_batch_add(fm_batch* b, fm_problem* p) {
   CK(cudaSetDevice(b->device));
   CK(cudaStreamSynchronize(b->stream));
   std::shared_ptr<Layout> L;
-  int r = prepare(p, b->tune.tile_elems, b->tune.tile_nodes, &L);
+  int r = prepare(p, b->tune, &L);
   if (r) return r;
   return place(b, p, L);
 }

@@ -205,7 +205,18 @@ extern "C" int fm_vms_solve_static(fm_problem* p, int32_t nsteps, int32_t device
   if (p->params.precision != FM_FP64) return fail(FM_ERR_INVALID, "fm_vms_solve_static runs the FP64 form only");
   if (!p->layout) return fail(FM_ERR_INVALID, "call fm_problem_prepare before fm_vms_solve_static");
   if (p->part >= 0) return fail(FM_ERR_INVALID, "fm_vms_solve_static does not run partition parts");
-  const Layout& L = *p->layout;
+  // the prepared layout, or full tiles where its small ones (more interface
+  // partials) would not fit
+  std::shared_ptr<Layout> full;
+  const Layout* pl = p->layout.get();
+  if (plan(p, *pl).total > (size_t)FM_STATIC_SCRATCH_BYTES) {
+    fm_problem* arr[1] = {p};
+    full = std::make_shared<Layout>();
+    const int lr = build_layout(arr, 1, 1024, FM_MAX_TILE_NODES, *full);
+    if (lr) return lr;
+    if (plan(p, *full).total < plan(p, *pl).total) pl = full.get();
+  }
+  const Layout& L = *pl;
   const Offsets o = plan(p, L);
   if (o.total > (size_t)FM_STATIC_SCRATCH_BYTES)
     return fail(FM_ERR_INVALID, "problem needs " + std::to_string(o.total) + " bytes of static scratch; the limit is " +

@@ -106,7 +106,7 @@ typedef struct fm_params {
 /* Launch shape; zero fields take the built-in defaults (or the autotuned
  * values when fm_batch_autotune has run). */
 typedef struct fm_tuning {
-  int32_t tile_elems;      /* elements per tile (one CTA owns one tile)  */
+  int32_t tile_elems;      /* elements per tile (one CTA owns one tile); 0: by each problem's size */
   int32_t tile_nodes;      /* max distinct nodes per tile (shared memory) */
   int32_t threads;         /* threads per CTA */
   int32_t graph_steps;     /* time steps captured per CUDA graph (0: no graph) */
