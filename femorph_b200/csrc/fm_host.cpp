@@ -573,6 +573,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
   for (int pi = 0; pi < n; ++pi) {
     fm_problem* p = probs[pi];
     const int npe = p->etype;
+    const bool vms = p->params.solver == FM_SOLVER_VMS;
     const int64_t E = p->E, N = p->N;
     L.node_begin.push_back(node_base);
     L.elem_begin.push_back(elem_base);
@@ -712,7 +713,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             for (int32_t v : W.inter) local[v] = li++;
             for (int32_t v : W.ifc) local[v] = li++;
             const int32_t n_node = li;
-            {
+            if (!vms) {  // owner threads (SUPG tet4; hexa and VMS have none)
               cnt.assign(n_node, 0);
               for (int64_t oi = tile_start[t]; oi < tile_start[t + 1]; ++oi)
                 for (int a = 0; a < npe; ++a) cnt[local[cs[(size_t)oi * npe + a]]]++;
@@ -728,30 +729,69 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             used.assign(2 * (size_t)n_node, 0);
             col.resize(ne);
             int ncol = 0;
+            // VMS: a warp of the tile kernel adds up its 32 elements one colour
+            // after another, so colours hold at most 32 elements, and a tile
+            // of enough warps (a node has up to 24 elements, hence 24 colours)
+            // spreads its elements over as many colours as it has warps,
+            // always to the emptiest one that fits: 36 colour runs in the 32
+            // warps of a 1024-tet tile, against 60 of the smallest colour
+            // that fits
+            const int nwarp = (int)((ne + 31) / 32);
+            const int even = vms && nwarp >= 26 && nwarp <= 64 ? nwarp : 0;
+            uint64_t level[33] = {0};  // colours below `even` by their size
+            level[0] = even == 64 ? ~0ULL : (1ULL << even) - 1;
+            int csize[128] = {0};
+            uint64_t full0 = 0, full1 = 0;  // VMS: colours with 32 elements
             for (int64_t i = 0; i < ne; ++i) {
               const int32_t* c = &cs[(size_t)(tile_start[t] + i) * npe];
-              uint64_t m0 = 0, m1 = 0;
+              uint64_t m0 = full0, m1 = full1;
               for (int a = 0; a < npe; ++a) {
                 m0 |= used[2 * local[c[a]]];
                 m1 |= used[2 * local[c[a]] + 1];
               }
-              int k;
-              if (~m0) k = __builtin_ctzll(~m0);
+              int k = -1;
+              for (int q = 0; even && q < 32; ++q)
+                if (level[q] & ~m0) {
+                  k = __builtin_ctzll(level[q] & ~m0);
+                  level[q] &= ~(1ULL << k);
+                  level[q + 1] |= 1ULL << k;
+                  break;
+                }
+              if (k >= 0) {
+              } else if (~m0) k = __builtin_ctzll(~m0);
               else if (~m1) k = 64 + __builtin_ctzll(~m1);
               else {
-                W.err = 1;
-                break;
+                // every colour full or taken: past the limit of 32 instead
+                m0 = m1 = 0;
+                for (int a = 0; a < npe; ++a) {
+                  m0 |= used[2 * local[c[a]]];
+                  m1 |= used[2 * local[c[a]] + 1];
+                }
+                if (~m0) k = __builtin_ctzll(~m0);
+                else if (~m1) k = 64 + __builtin_ctzll(~m1);
+                else {
+                  W.err = 1;
+                  break;
+                }
               }
+              if (vms && ++csize[k] >= 32) (k < 64 ? full0 : full1) |= 1ULL << (k & 63);
               col[i] = k;
               ncol = std::max(ncol, k + 1);
               for (int a = 0; a < npe; ++a) used[2 * local[c[a]] + (k >> 6)] |= (1ULL << (k & 63));
             }
             if (W.err) continue;
+            if (vms) {
+              // the largest colours first: they fill whole warps
+              int by[128], at[128], n = 0;
+              for (int k = 0; k < ncol; ++k)
+                if (csize[k]) by[n++] = k;
+              std::stable_sort(by, by + n, [&](int x, int y) { return csize[x] > csize[y]; });
+              for (int k = 0; k < n; ++k) at[by[k]] = k;
+              for (int64_t i = 0; i < ne; ++i) col[i] = at[col[i]];
+              ncol = n;
+            }
             // elements sorted by colour: SUPG processes a tile one colour at a
-            // time; for VMS it spreads each chunk's contributions over all of
-            // the tile's nodes (one or two per node and chunk, which balances
-            // the node-owner accumulation; the space-filling order measured
-            // slower)
+            // time
             // (counting sort by colour: stable, as the element order within a
             // colour must stay the sorted order)
             W.ncol = ncol;
@@ -783,6 +823,12 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             pos.assign(cnt.begin(), cnt.end() - 1);
             for (int64_t i = 0; i < ne; ++i)
               for (int a = 0; a < npe; ++a) W.inc[pos[W.conn[i * npe + a]]++] = (uint16_t)(i * npe + a);
+            // VMS: bit 15 of an element's second node id marks the first
+            // element of a colour (the tile kernel's warps add up one colour
+            // after another)
+            if (vms)
+              for (int k = 0; k < ncol; ++k)
+                if (W.colcnt[k] < ne) W.conn[(size_t)W.colcnt[k] * npe + 1] |= 0x8000;
           }
         });
       for (auto& x : th) x.join();
@@ -1014,14 +1060,14 @@ int check_layout(const fm_problem* p, const Layout& L) {
       }
     }
     // local connectivity (bit 15 of the first id flags an FP64-Jacobian
-    // element in the mixed form)
+    // element in the mixed form, of the second one a colour's first element)
     const uint16_t* cl = &L.conn_local[(size_t)tm.elem_begin * npe];
     for (int32_t i = 0; i < ne; ++i) {
       const int64_t oe = L.elem_old[0][tm.elem_begin + i];
       if (oe < 0 || oe >= E || elem_seen[oe]) return bad("tile " + std::to_string(t) + ": element map");
       elem_seen[oe] = 1;
       for (int a = 0; a < npe; ++a) {
-        const int32_t ln = a == 0 ? (cl[i * npe] & 0x7fff) : cl[i * npe + a];
+        const int32_t ln = a <= 1 ? (cl[i * npe + a] & 0x7fff) : cl[i * npe + a];
         if (ln >= nl) return bad("tile " + std::to_string(t) + ": local node id out of range");
         if (old_of[tn[ln]] != p->conn[oe * npe + a]) return bad("tile " + std::to_string(t) + ": connectivity");
       }
@@ -1033,10 +1079,18 @@ int check_layout(const fm_problem* p, const Layout& L) {
     for (int32_t c = 0; c < tm.n_col; ++c)
       for (int32_t i = co[c]; i < co[c + 1]; ++i)
         for (int a = 0; a < npe; ++a) {
-          const int32_t ln = a == 0 ? (cl[i * npe] & 0x7fff) : cl[i * npe + a];
+          const int32_t ln = a <= 1 ? (cl[i * npe + a] & 0x7fff) : cl[i * npe + a];
           if (colour_stamp[ln] == c) return bad("tile " + std::to_string(t) + ": two elements of a colour share a node");
           colour_stamp[ln] = c;
         }
+    if (p->params.solver == FM_SOLVER_VMS) {
+      // the marks of the colours' first elements (not needed on the tile's first)
+      std::vector<char> first(ne, 0);
+      for (int32_t c = 1; c < tm.n_col; ++c)
+        if (co[c] < ne) first[co[c]] = 1;
+      for (int32_t i = 1; i < ne; ++i)
+        if (((cl[i * npe + 1] & 0x8000) != 0) != (first[i] != 0)) return bad("tile " + std::to_string(t) + ": colour marks");
+    }
     // incidence lists
     const uint16_t* off = &L.tile_off[tm.off_begin];
     const uint16_t* inc = &L.tile_inc[tm.inc_begin];
@@ -1045,7 +1099,7 @@ int check_layout(const fm_problem* p, const Layout& L) {
       for (int32_t k = off[l]; k < off[l + 1]; ++k) {
         const int32_t el = inc[k] / npe, a = inc[k] % npe;
         if (el >= ne) return bad("tile " + std::to_string(t) + ": incidence element");
-        const int32_t ln = a == 0 ? (cl[el * npe] & 0x7fff) : cl[el * npe + a];
+        const int32_t ln = a <= 1 ? (cl[el * npe + a] & 0x7fff) : cl[el * npe + a];
         if (ln != l) return bad("tile " + std::to_string(t) + ": incidence entry of another node");
         if (k > off[l] && inc[k - 1] / npe >= el) return bad("tile " + std::to_string(t) + ": incidence order");
       }

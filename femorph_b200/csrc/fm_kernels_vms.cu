@@ -7,11 +7,11 @@
 //      geometry from the staged coordinates, the pending subscale update of
 //      the previous iteration (assemble_projRes_explicit +
 //      update_subscales_explicit), the element residual (assemble_RHS);
-//   3. stage the chunk's 16 residual entries an element in shared memory;
-//      after one barrier each thread adds, for the nodes it owns, the
-//      chunk's contributions to its shared-memory accumulators, walking the
-//      node's incidence list in element order, so every node receives its
-//      contributions in a fixed order - no atomics;
+//   3. the warps of a ring add their 32 elements' residuals to the ring's
+//      accumulators one warp after another, and within a warp one colour after
+//      another (elements of a colour share no node), so every node receives
+//      its contributions in a fixed order - no atomics, no barrier over the
+//      CTA;
 //   4. nodes interior to the tile are complete: dual update
 //      (update_dual_solution), BCs (setNodeVelocity, apply_zeroTraction,
 //      setDirichletBC) and store; interface nodes store their tile partial.
@@ -32,19 +32,20 @@ namespace fm {
 // differs at BC nodes).  The dual update starts from sol_n, which is the
 // post-BC state at the first dual iteration of a step (update_solution,
 // src lines 726-752) and the pre-BC state afterwards.
-// The problem constants the element and node passes read, copied into
-// registers once per CTA (read through the DevProb in global memory they
-// would be reloaded for every element: the compiler cannot prove that the
-// kernel's own stores leave them unchanged).
+// The problem constants the node pass reads, copied into registers (through
+// the DevProb in global memory they would be reloaded for every node: the
+// compiler cannot prove that the kernel's own stores leave them unchanged).
 struct VmsConsts {
-  double ds, c2, inv_eps;
+  double ds;
   int32_t q1[4];
+};
+// What the element pass reads of the problem, in shared memory.
+struct ElemConsts {
+  double pq[4], inv_dt, c1nu, nu4, c2, inv_eps;
 };
 __device__ __forceinline__ VmsConsts vms_consts(const DevProb& P) {
   VmsConsts c;
   c.ds = P.ds;
-  c.c2 = P.c2;
-  c.inv_eps = P.inv_eps;
   c.q1[0] = P.q1[0]; c.q1[1] = P.q1[1]; c.q1[2] = P.q1[2]; c.q1[3] = P.q1[3];
   return c;
 }
@@ -93,10 +94,9 @@ constexpr long long FM_TAG_BC = 1ll << 62;
 // back to global memory) and the element residual lres.  S: subscale storage
 // type (double, or float in the mixed form).
 template <bool MIXED, typename S>
-__device__ __forceinline__ void vms_element(const DevBatch& B, const VmsConsts& P, int64_t e, const int ln[4],
-                                            bool precise, const double2* s_rec, const S sd_in[12],
-                                            const double pq[4], bool pending, bool first_dual, double inv_dt,
-                                            double c1nu, double nu4, double lres[4][4]) {
+__device__ __forceinline__ void vms_element(const DevBatch& B, const ElemConsts& P, int64_t e, const int ln[4],
+                                            bool precise, const double2* s_rec, const S sd_in[12], bool pending,
+                                            bool first_dual, double lres[4][4]) {
   const int64_t E = B.E;
   // Pass 1 reads the coordinates and Q, the velocity before the last BC
   // application (it differs from the staged state only at BC nodes, whose
@@ -150,8 +150,8 @@ __device__ __forceinline__ void vms_element(const DevBatch& B, const VmsConsts& 
         for (int a = 0; a < 4; ++a) Qd[a][i] = (float)(Q[a][i] - Q[0][i]);
       }
 #pragma unroll
-      for (int a = 0; a < 4; ++a) pqd[a] = (float)(pq[a] - pq[0]);
-      vms_subscale_update_mixed(geo, Q0, Qd, pqd, sdu, (float)inv_dt, (float)c1nu, (float)P.c2, ih, G, Ds);
+      for (int a = 0; a < 4; ++a) pqd[a] = (float)(P.pq[a] - P.pq[0]);
+      vms_subscale_update_mixed(geo, Q0, Qd, pqd, sdu, (float)P.inv_dt, (float)P.c1nu, (float)P.c2, ih, G, Ds);
 #pragma unroll
       for (int q = 0; q < 12; ++q) __stcs(B.sdus32 + (int64_t)q * E + e, sdu[q / 3][q % 3]);
     }
@@ -163,7 +163,7 @@ __device__ __forceinline__ void vms_element(const DevBatch& B, const VmsConsts& 
       for (int a = 0; a < 4; ++a) Ud[a][i] = (float)(U[a][i] - U[0][i]);
     }
     if (first_dual) {
-      vms_residual_mixed<false>(geo, U0, Ud, Pn, Ud, sdu, (float)nu4, (float)P.inv_eps, (float)inv_dt, G, Ds, false,
+      vms_residual_mixed<false>(geo, U0, Ud, Pn, Ud, sdu, (float)P.nu4, (float)P.inv_eps, (float)P.inv_dt, G, Ds, false,
                                 lres);
     } else {
       float Dacc[4][3];
@@ -171,7 +171,7 @@ __device__ __forceinline__ void vms_element(const DevBatch& B, const VmsConsts& 
       for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int i = 0; i < 3; ++i) Dacc[a][i] = (float)(U[a][i] - Q[a][i]);
-      vms_residual_mixed<true>(geo, U0, Ud, Pn, Dacc, sdu, (float)nu4, (float)P.inv_eps, (float)inv_dt, G, Ds, false,
+      vms_residual_mixed<true>(geo, U0, Ud, Pn, Dacc, sdu, (float)P.nu4, (float)P.inv_eps, (float)P.inv_dt, G, Ds, false,
                                lres);
     }
   } else {
@@ -184,61 +184,90 @@ __device__ __forceinline__ void vms_element(const DevBatch& B, const VmsConsts& 
     for (int q = 0; q < 12; ++q) sdu[q / 3][q % 3] = sd_in[q];
     double G[3][3], Gs[3];
     if (pending) {
-      vms_subscale_update<double>(geo, Q, pq, sdu, inv_dt, c1nu, P.c2, ih, G, Gs);
+      vms_subscale_update<double>(geo, Q, P.pq, sdu, P.inv_dt, P.c1nu, P.c2, ih, G, Gs);
 #pragma unroll
       for (int q = 0; q < 12; ++q) __stcs(B.sdus + (int64_t)q * E + e, sdu[q / 3][q % 3]);
     }
     load_post();
     if (first_dual)
-      vms_residual<double, false>(geo, U, Pn, U, sdu, nu4, P.inv_eps, inv_dt, G, Gs, false, lres);
+      vms_residual<double, false>(geo, U, Pn, U, sdu, P.nu4, P.inv_eps, P.inv_dt, G, Gs, false, lres);
     else
-      vms_residual<double, true>(geo, U, Pn, Q, sdu, nu4, P.inv_eps, inv_dt, G, Gs, false, lres);
+      vms_residual<double, true>(geo, U, Pn, Q, sdu, P.nu4, P.inv_eps, P.inv_dt, G, Gs, false, lres);
   }
 }
 
 // Shared memory of one tile CTA, in this order:
-//  node records: 8 doubles x tn_pad (rec_index layout), then four residual
-//    accumulators of tn_pad doubles; tn_pad = tn_max rounded up to even so
-//    every later region is 16-byte aligned;
+//  node records: 8 doubles x tn_pad (rec_index layout), then the residual
+//    accumulators, 4 doubles x tn_pad a set (acc_index layout); tn_pad =
+//    tn_max rounded up to even;
 //  chunk stage: two buffers, each 12 subscale rows + 1 connectivity row of
-//    THREADS slots (bulk-copy targets).  FP64: each buffer is sized to 16 rows
-//    of THREADS doubles because a thread overwrites its own column with its 16
-//    residual entries once it has read its inputs; mixed: a separate
-//    16 x THREADS double region holds the residual entries;
-//  incidence entries (uint16 x inc_max), incidence offsets (uint16 x tn_pad+2).
-template <int THREADS, bool MIXED>
-__host__ __device__ constexpr size_t vms_stage_bytes() {
-  return MIXED ? 2 * ((size_t)12 * THREADS * sizeof(float) + (size_t)THREADS * 8) + (size_t)16 * THREADS * 8
-               : 2 * (size_t)16 * THREADS * 8;
-}
+//    THREADS slots (bulk-copy targets).
 template <int THREADS, bool MIXED>
 __host__ __device__ constexpr size_t vms_stage_buffer_bytes() {
-  return MIXED ? (size_t)12 * THREADS * sizeof(float) + (size_t)THREADS * 8 : (size_t)16 * THREADS * 8;
+  return (size_t)12 * THREADS * (MIXED ? sizeof(float) : sizeof(double)) + (size_t)THREADS * 8;
+}
+
+// Sets of accumulators, each shared by a ring of warps (vms_tile_kernel).
+constexpr int FM_ACC_SETS = 2;
+
+// 16-byte half h of node ln's accumulators: the halves of every fourth node
+// swap places, so that a warp's 16-byte accesses of distinct nodes use all
+// eight 4-bank groups.
+__device__ __forceinline__ int acc_index(int ln, int h) { return ln * 2 + (h ^ ((ln >> 2) & 1)); }
+
+// Named barrier `id` of two warps: the first waits for the second's arrival
+// and then sees what it wrote to shared memory before.
+// (An id known at compile time: a kernel that computes it reserves all 16.)
+template <int N>
+__device__ __forceinline__ void pair_wait(int id) {
+  if (id == N) asm volatile("barrier.cta.sync %0, 64;" ::"n"(N) : "memory");
+  else if constexpr (N > 1) pair_wait<N - 1>(id);
+}
+template <int N>
+__device__ __forceinline__ void pair_arrive(int id) {
+  if (id == N) asm volatile("barrier.cta.arrive %0, 64;" ::"n"(N) : "memory");
+  else if constexpr (N > 1) pair_arrive<N - 1>(id);
 }
 
 // MINB: resident CTAs an SM the variant is compiled for (its register budget).
+//
+// The warps of a ring take turns with a set of accumulators: warp w's turn of
+// a chunk follows warp w - 1's, the first warp's the last one's of the chunk
+// before, through one named barrier a warp (a pair: the warp whose turn ends
+// arrives, the next one waits).  The warps run a turn apart from each other,
+// so neither a barrier over the CTA nor a staged copy of the residuals is
+// needed; a turn is some 200 cycles a colour run against several thousand of
+// element work.  The FM_ACC_SETS sets of accumulators, each with a ring of its
+// own, are added up at the end: a node's sum is that of the rings in order, of
+// a ring's elements in order.  Two sets of two warps against one of four: 361
+// against 378 us a step mixed at 96^3, FP64 472 either way there and 435 against
+// 455 for 32 cavities of 8..48 cells a side, whose tiles have more colour runs.
+//
+// Before, every thread added up the entries of the nodes it owned, after a
+// barrier, from residuals staged in shared memory: 96^3 cavity 518 -> 472 us a
+// step FP64, 408 -> 361 mixed.  What remains is the latency of the FP64 chains
+// at 12 warps an SM (issue slots used 40%, FP64 pipe 36%), the turns (with one
+// ring the kernel took 8% less without waiting for them) and the tile's start.
+// Shared memory is taken from L1, which the node gathers live on: 7 KB a CTA
+// more cost 4% where they crossed a step of the carve-out.
 template <int THREADS, bool MIXED, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int tn_max, int inc_max) {
+__global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int tn_max) {
   using S = typename std::conditional<MIXED, float, double>::type;
+  constexpr int WARPS = THREADS / 32;
   extern __shared__ __align__(16) double sm[];
   const int tn_pad = (tn_max + 1) & ~1;
   double2* s_rec = reinterpret_cast<double2*>(sm);  // per node: (x,y) (z,u) (v,w) (p,tag)
-  double* s_a0 = sm + 8 * tn_pad;  // residual accumulators (each node owned by one thread)
-  double* s_a1 = s_a0 + tn_pad;
-  double* s_a2 = s_a1 + tn_pad;
-  double* s_a3 = s_a2 + tn_pad;
-  char* stage = reinterpret_cast<char*>(s_a3 + tn_pad);
+  double2* s_acc = s_rec + 4 * tn_pad;
+  char* stage = reinterpret_cast<char*>(s_acc + 2 * FM_ACC_SETS * tn_pad);
   constexpr size_t BUF = vms_stage_buffer_bytes<THREADS, MIXED>();
-  double* s_lres_mixed = reinterpret_cast<double*>(stage + 2 * BUF);  // mixed only
-  uint16_t* s_inc = reinterpret_cast<uint16_t*>(stage + vms_stage_bytes<THREADS, MIXED>());  // inc_max (multiple of 8)
-  uint16_t* s_off = s_inc + inc_max;
-  __shared__ uint64_t bars[2];
+  __shared__ uint64_t full[2], empty[2];
   __shared__ int s_abort;
+  __shared__ ElemConsts s_k;
 
   const TileMeta tm = B.tiles[blockIdx.x];
   const int pidx = tm.problem;
   if (pidx < 0) return;  // free tile slot
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // this thread's staged nodes: their ids are loaded before the problem
   // state is checked, so both round trips overlap
   constexpr int MAXOWN = FM_MAX_TILE_NODES / THREADS;  // the host caps tile_nodes
@@ -251,7 +280,6 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
   const DevProbState st = B.pstate[pidx];
   if (st.iter >= B.target[pidx] || st.status != FM_OK) return;
   const DevProb& P = B.probs[pidx];
-  const VmsConsts PC = vms_consts(P);
   const int per_step = P.ndual + 1;
   const bool first_dual = (st.iter % per_step) == 0;
   const bool pending = st.iter > 0;
@@ -270,20 +298,23 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
     const uint32_t bytes_s = rs * (uint32_t)sizeof(S);
     const uint32_t bytes_c = (uint32_t)((nch + 1) & ~1) * 8u;
     S* bs = reinterpret_cast<S*>(stage + b * BUF);
-    mbar_arrive_expect_tx(&bars[b], 12u * bytes_s + bytes_c);
+    mbar_arrive_expect_tx(&full[b], 12u * bytes_s + bytes_c);
 #pragma unroll 1
-    for (int q = 0; q < 12; ++q) bulk_load(bs + q * THREADS, sdus_g + (int64_t)q * E + e0, bytes_s, &bars[b]);
-    bulk_load(bs + 12 * THREADS, conn_g + e0, bytes_c, &bars[b]);
+    for (int q = 0; q < 12; ++q) bulk_load(bs + q * THREADS, sdus_g + (int64_t)q * E + e0, bytes_s, &full[b]);
+    bulk_load(bs + 12 * THREADS, conn_g + e0, bytes_c, &full[b]);
   };
+  int issued = 0;  // chunks (thread 0)
 
   if (tid == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    mbar_init(&empty[0], WARPS);
+    mbar_init(&empty[1], WARPS);
     fence_mbar_init();
     s_abort = 0;
     // the first chunk's copies overlap the node staging below (they target
     // the stage buffers, which the staging does not touch)
-    if (nchunks > 0) issue(0);
+    if (nchunks > 0) issue(issued++);
   }
   // node staging: the gathers of this thread's (up to FM_MAX_TILE_NODES /
   // THREADS) nodes overlap
@@ -298,25 +329,24 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
         s_rec[rec_index(ln, 1)] = make_double2(B.z[g], B.su[g]);
         s_rec[rec_index(ln, 2)] = make_double2(B.sv[g], B.sw[g]);
         s_rec[rec_index(ln, 3)] = make_double2(B.sp[g], __longlong_as_double(tag));
-        s_a0[ln] = 0.0; s_a1[ln] = 0.0; s_a2[ln] = 0.0; s_a3[ln] = 0.0;
+#pragma unroll
+        for (int q = 0; q < FM_ACC_SETS; ++q) {
+          s_acc[2 * (q * tn_pad + ln)] = make_double2(0.0, 0.0);
+          s_acc[2 * (q * tn_pad + ln) + 1] = make_double2(0.0, 0.0);
+        }
       }
     }
   }
-  for (int i = tid; i <= tm.n_node; i += THREADS) s_off[i] = B.tile_off[tm.off_begin + i];
-  {
-    const int ninc = tm.n_elem * 4;
-    const uint4* src = reinterpret_cast<const uint4*>(B.tile_inc + tm.inc_begin);  // 16-byte aligned
-    uint4* dst = reinterpret_cast<uint4*>(s_inc);
-    for (int i = tid; i < (ninc + 7) / 8; i += THREADS) dst[i] = src[i];
+  // the problem's constants, read where they are used (in registers they
+  // would be spilled through the element work)
+  if (tid < 4) s_k.pq[tid] = B.q1p[pidx * 8 + ((st.iter - 1) & 1) * 4 + tid];
+  if (tid == 32) {
+    s_k.inv_dt = 1.0 / P.dt;
+    s_k.c1nu = P.c1 * P.nu;
+    s_k.nu4 = 4.0 * P.nu;
+    s_k.c2 = P.c2;
+    s_k.inv_eps = P.inv_eps;
   }
-  double pq[4];
-  {
-    const double* q = B.q1p + pidx * 8 + ((st.iter - 1) & 1) * 4;
-    pq[0] = q[0]; pq[1] = q[1]; pq[2] = q[2]; pq[3] = q[3];
-  }
-  const double inv_dt = 1.0 / P.dt;
-  const double c1nu = P.c1 * P.nu;
-  const double nu4 = 4.0 * P.nu;
   __syncthreads();
   // one lane asks L2 for a later tile's element rows and interior-node
   // ranges (contiguous), so that tile's bulk copies and gathers hit L2; the
@@ -330,7 +360,6 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
 #pragma unroll 1
       for (int q = 0; q < 12; ++q) bulk_prefetch_l2(sdus_g + (int64_t)q * E + e0, bs);
       bulk_prefetch_l2(conn_g + e0, ((uint32_t)tn.n_elem * 8u + 15u) & ~15u);
-      bulk_prefetch_l2(B.tile_inc + tn.inc_begin, ((uint32_t)tn.n_elem * 8u + 15u) & ~15u);
       if (tn.n_int > 0 && tn.node0 >= 0) {
         const int64_t g0 = tn.node0 & ~1, g1 = ((int64_t)tn.node0 + tn.n_int + 1) & ~1ll;
         const uint32_t nb = (uint32_t)(g1 - g0) * 8u;
@@ -343,24 +372,21 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
     }
   }
 
-  // nodes owned by this thread for the accumulation: j * THREADS + tid;
-  // cur/end walk each one's incidence list in element order, nxt holds the
-  // entry at cur (loaded one step ahead, so the walk's shared-memory loads
-  // do not wait on each other)
-  auto owned_node = [](int t, int j) { return j * THREADS + t; };
-  int cur[MAXOWN], endi[MAXOWN], nxt[MAXOWN];
-#pragma unroll
-  for (int j = 0; j < MAXOWN; ++j) {
-    const int ln = owned_node(tid, j);
-    cur[j] = ln < tm.n_node ? s_off[ln] : 0;
-    endi[j] = ln < tm.n_node ? s_off[ln + 1] : 0;
-    nxt[j] = cur[j] < endi[j] ? s_inc[cur[j]] : 0;
-  }
-  int k = 0;
-  for (; k < nchunks; ++k) {
-    if (tid == 0 && k + 1 < nchunks) {
-      fence_proxy_async_smem();  // buffer (k+1)&1 was last read before the previous barrier
-      issue(k + 1);
+  volatile int* aborted = &s_abort;
+  // the warps of a ring share a set of accumulators
+  constexpr int RING = WARPS / FM_ACC_SETS;
+  const int ring = warp / RING, place = warp % RING;
+  double2* w_acc = s_acc + 2 * ring * tn_pad;
+  for (int k = 0; k < nchunks; ++k) {
+    const int b = k & 1;
+    if (tid == 0 && k + 1 < nchunks && !*aborted) {
+      // buffer b ^ 1 is free once every warp has read its elements of chunk k - 1
+      if (k == 0 || mbar_wait_bounded(&empty[b ^ 1], (uint32_t)(((k - 1) >> 1) & 1), FM_WAIT_LIMIT)) {
+        fence_proxy_async_smem();
+        issue(issued++);
+      } else {
+        *aborted = 1;
+      }
     }
     if (k + 1 == nchunks) {
       // the node update after the last chunk reads the mass and BC index of
@@ -376,139 +402,99 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
       }
     }
     // each thread waits for the chunk itself (the mbarrier phase makes the
-    // bulk-copied bytes visible to it); a timed-out wait skips the chunk and
-    // is agreed on at the end-of-chunk barrier
-    const bool arrived = mbar_wait_bounded(&bars[k & 1], (uint32_t)((k >> 1) & 1), B.wait_limit);
-    const int base = k * THREADS;
-    const int le = base + tid;
+    // bulk-copied bytes visible to it); after a timed-out wait the CTA goes
+    // through its turns without touching anything more
+    bool arrived = false;
+    for (uint32_t i = 0; i < B.wait_limit && !arrived; ++i) {
+      arrived = mbar_try_wait(&full[b], (uint32_t)((k >> 1) & 1));
+      if (!arrived && *aborted) break;
+    }
+    if (!arrived) *aborted = 1;
+    const int le = k * THREADS + tid;
     const bool active = arrived && le < tm.n_elem;
-    char* buf = stage + (k & 1) * BUF;
-    // residual entries.  FP64: [16][THREADS] in the stage buffer, each thread
-    // overwriting its own column (its inputs, already read).  Mixed (own
-    // region): per element 8 16-byte pieces (corner, component pair), piece p
-    // of element col at col * 8 + (p ^ (col & 7)), so that the owners'
-    // scattered 16-byte reads spread over all bank groups (1.5% faster
-    // there; in the FP64 stage buffer it would need one more barrier a chunk,
-    // which costs more than it gains)
-    double* R = MIXED ? s_lres_mixed : reinterpret_cast<double*>(buf);
-    double2* R2 = reinterpret_cast<double2*>(R);
     double lres[4][4];
-    if (active) {
-      const S* bs = reinterpret_cast<const S*>(buf);
-      const uint2 cw = reinterpret_cast<const uint2*>(bs + 12 * THREADS)[tid];
-      int ln[4];
-      // bit 15 of the first id flags (mixed form) an element whose Jacobian
-      // inverse stays in FP64
-      const bool precise = (cw.x & 0x8000u) != 0;
-      ln[0] = cw.x & 0x7fff; ln[1] = cw.x >> 16; ln[2] = cw.y & 0xffff; ln[3] = cw.y >> 16;
+    // the element's corners: bit 15 of the first id flags (mixed form) an
+    // element whose Jacobian inverse stays in FP64, of the second one the
+    // first of a colour
+    uint2 cw = make_uint2(0u, 0u);
+    auto corners = [](uint2 c, int ln[4]) {
+      ln[0] = c.x & 0x7fff; ln[1] = (c.x >> 16) & 0x7fff; ln[2] = c.y & 0xffff; ln[3] = c.y >> 16;
+    };
+    {
       S sd_in[12];
-#pragma unroll
-      for (int q = 0; q < 12; ++q) sd_in[q] = bs[q * THREADS + tid];
-      vms_element<MIXED, S>(B, PC, tm.elem_begin + le, ln, precise, s_rec, sd_in, pq, pending, first_dual, inv_dt,
-                            c1nu, nu4, lres);
-      if (B.diag_res) {
-#pragma unroll
-        for (int r = 0; r < 16; ++r) B.diag_res[(int64_t)r * E + tm.elem_begin + le] = lres[r >> 2][r & 3];
-      }
-    }
-    if constexpr (MIXED) {
-      // the mixed form's residual region is its own, so the barrier that lets
-      // it be overwritten (owners of the previous chunk done) comes after
-      // this chunk's element work: warps that finish the previous chunk's
-      // accumulation early go on with their elements instead of waiting
-      if (k > 0) __syncthreads();
       if (active) {
-        double2* Rt = R2 + tid * 8;
+        const S* bs = reinterpret_cast<const S*>(stage + b * BUF);
+        cw = reinterpret_cast<const uint2*>(bs + 12 * THREADS)[tid];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          Rt[q ^ (tid & 7)] = make_double2(lres[q >> 1][2 * (q & 1)], lres[q >> 1][2 * (q & 1) + 1]);
+        for (int q = 0; q < 12; ++q) sd_in[q] = bs[q * THREADS + tid];
       }
-      // any timed-out wait aborts here, before the accumulation
-      if (__syncthreads_or(!arrived)) {
-        if (tid == 0) s_abort = 1;
-        break;
-      }
-    } else {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[b]);
       if (active) {
+        int ln[4];
+        corners(cw, ln);
+        vms_element<MIXED, S>(B, s_k, tm.elem_begin + le, ln, (cw.x & 0x8000u) != 0, s_rec, sd_in, pending, first_dual,
+                              lres);
+        if (B.diag_res) {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) R[r * THREADS + tid] = lres[r >> 2][r & 3];
-      }
-      __syncthreads();
-    }
-    // owners add this chunk's contributions to their nodes, in element order
-#pragma unroll
-    for (int j = 0; j < MAXOWN; ++j) {
-      const int ln = owned_node(tid, j);
-      int c = cur[j];
-      const int ce = endi[j];
-      int ent = nxt[j];
-      // nodes without an entry in this chunk leave their accumulators alone
-      if (c < ce && (ent >> 2) - base < THREADS) {
-        double a0 = s_a0[ln], a1 = s_a1[ln], a2 = s_a2[ln], a3 = s_a3[ln];
-        // the residual entries of incidence entry e (of this chunk)
-        auto fetch = [&](int e, double v[4]) {
-          const int col = (e >> 2) - base;
-          if constexpr (MIXED) {
-            const double2* Rc = R2 + col * 8;
-            const int q0i = 2 * (e & 3), sw = col & 7;
-            const double2 q0 = Rc[q0i ^ sw], q1 = Rc[(q0i + 1) ^ sw];
-            v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y;
-          } else {
-            const double* Rp = R + (e & 3) * 4 * THREADS + col;  // rows 4*corner .. 4*corner+3
-            v[0] = Rp[0]; v[1] = Rp[THREADS]; v[2] = Rp[2 * THREADS]; v[3] = Rp[3 * THREADS];
-          }
-        };
-        // two entries a pass (their loads overlap), added in element order;
-        // the entries after them are loaded one pass ahead
-        while (true) {
-          const int ent1 = s_inc[c + 1 < ce ? c + 1 : c];
-          const int ent2 = s_inc[c + 2 < ce ? c + 2 : c];
-          const bool two = c + 1 < ce && (ent1 >> 2) - base < THREADS;
-          double v[4], w[4];
-          fetch(ent, v);
-          fetch(two ? ent1 : ent, w);
-          a0 += v[0]; a1 += v[1]; a2 += v[2]; a3 += v[3];
-          if (!two) {
-            ++c;
-            ent = ent1;
-            break;
-          }
-          a0 += w[0]; a1 += w[1]; a2 += w[2]; a3 += w[3];
-          c += 2;
-          ent = ent2;
-          if (c >= ce || (ent >> 2) - base >= THREADS) break;
+          for (int r = 0; r < 16; ++r) B.diag_res[(int64_t)r * E + tm.elem_begin + le] = lres[r >> 2][r & 3];
         }
-        cur[j] = c;
-        nxt[j] = ent;
-        s_a0[ln] = a0; s_a1[ln] = a1; s_a2[ln] = a2; s_a3[ln] = a3;
       }
     }
-    // FP64 end of chunk: stage buffer k&1 (holding this chunk's residuals) is
-    // free again; any timed-out wait aborts
-    if constexpr (!MIXED) {
-      if (__syncthreads_or(!arrived)) {
-        if (tid == 0) s_abort = 1;
-        break;
+    // unpacked again rather than held through the element work
+    if (!MIXED) asm volatile("" : "+r"(cw.x), "+r"(cw.y));
+    int ln[4];
+    corners(cw, ln);
+    const unsigned firsts = __ballot_sync(0xffffffffu, (cw.x >> 31) != 0) & ~1u;
+    const int mine = __popc(firsts & (0xffffffffu >> (31 - lane)));
+    const int colours = __popc(firsts) + 1;
+    if (RING > 1 && k + place > 0) pair_wait<WARPS>(1 + warp);
+    for (int c = 0; c < colours; ++c) {
+      if (active && mine == c) {
+        double2 v[4][2];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          v[a][0] = w_acc[acc_index(ln[a], 0)];
+          v[a][1] = w_acc[acc_index(ln[a], 1)];
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          v[a][0].x += lres[a][0];
+          v[a][0].y += lres[a][1];
+          v[a][1].x += lres[a][2];
+          v[a][1].y += lres[a][3];
+          w_acc[acc_index(ln[a], 0)] = v[a][0];
+          w_acc[acc_index(ln[a], 1)] = v[a][1];
+        }
       }
+      __syncwarp();
     }
+    if (RING > 1 && (k + 1 < nchunks || place + 1 < RING)) pair_arrive<WARPS>(1 + ring * RING + (place + 1) % RING);
   }
   __syncthreads();
   if (s_abort) {
     // a copy never completed: wait (bounded) for the copies this CTA issued,
     // report, and leave the tile's nodes untouched
     if (tid == 0) {
-      for (int j = k; j < nchunks && j <= k + 1; ++j)
-        mbar_wait_bounded(&bars[j & 1], (uint32_t)((j >> 1) & 1), FM_DRAIN_LIMIT);
+      for (int j = issued > 2 ? issued - 2 : 0; j < issued; ++j)
+        mbar_wait_bounded(&full[j & 1], (uint32_t)((j >> 1) & 1), FM_DRAIN_LIMIT);
       B.pstate[pidx].status = FM_ERR_TIMEOUT;
     }
     return;
   }
   int32_t status = FM_OK;
+  const VmsConsts PC = vms_consts(P);
 #pragma unroll
   for (int j = 0; j < MAXOWN; ++j) {
     const int ln2 = tid + j * THREADS;
     if (ln2 >= tm.n_node) break;
-    const double acc[4] = {s_a0[ln2], s_a1[ln2], s_a2[ln2], s_a3[ln2]};
+    double2 a0 = s_acc[acc_index(ln2, 0)], a1 = s_acc[acc_index(ln2, 1)];
+#pragma unroll
+    for (int q = 1; q < FM_ACC_SETS; ++q) {
+      const double2 b0 = s_acc[2 * q * tn_pad + acc_index(ln2, 0)], b1 = s_acc[2 * q * tn_pad + acc_index(ln2, 1)];
+      a0.x += b0.x; a0.y += b0.y; a1.x += b1.x; a1.y += b1.y;
+    }
+    const double acc[4] = {a0.x, a0.y, a1.x, a1.y};
     if (ln2 < tm.n_int) {
       const double2 r1 = s_rec[rec_index(ln2, 1)], r2 = s_rec[rec_index(ln2, 2)], r3 = s_rec[rec_index(ln2, 3)];
       const int g = (int)(__double_as_longlong(r3.y) & 0x7fffffffll);
@@ -516,8 +502,8 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
       vms_node_update(B, PC, pidx, st.iter, st.time, g, post, acc, first_dual, &status);
     } else {
       const int s = tm.slot_base + (ln2 - tm.n_int);
-      B.part[2 * s] = make_double2(acc[0], acc[1]);
-      B.part[2 * s + 1] = make_double2(acc[2], acc[3]);
+      B.part[2 * s] = a0;
+      B.part[2 * s + 1] = a1;
     }
   }
   if (status != FM_OK) B.pstate[pidx].status = status;
@@ -693,11 +679,11 @@ cudaError_t launch_vms_diagnostics(const DevBatch& B, const double* cres_buf, co
   return cudaGetLastError();
 }
 
-size_t vms_smem_bytes(int tn_max, int inc_max, int threads, bool mixed) {
+size_t vms_smem_bytes(int tn_max, int threads, bool mixed) {
   const size_t tn_pad = (size_t)((tn_max + 1) & ~1);
-  const size_t stage = threads == 256 ? (mixed ? vms_stage_bytes<256, true>() : vms_stage_bytes<256, false>())
-                                      : (mixed ? vms_stage_bytes<128, true>() : vms_stage_bytes<128, false>());
-  return tn_pad * 12 * sizeof(double) + stage + (size_t)inc_max * sizeof(uint16_t) + (tn_pad + 2) * sizeof(uint16_t);
+  const size_t buf = threads == 256 ? (mixed ? vms_stage_buffer_bytes<256, true>() : vms_stage_buffer_bytes<256, false>())
+                                    : (mixed ? vms_stage_buffer_bytes<128, true>() : vms_stage_buffer_bytes<128, false>());
+  return tn_pad * (8 + 4 * FM_ACC_SETS) * sizeof(double) + 2 * buf;
 }
 
 // Register-budget variants of the tile kernel: (threads, mixed, CTAs an SM).
@@ -717,15 +703,15 @@ bool vms_variant_exists(int threads, bool mixed, int ctas) {
 
 // One dual iteration: tile kernel, then the interface pass (xpack: its first
 // half for a batch of partition parts; launch_vms_xupdate completes it).
-cudaError_t launch_vms_iteration(const DevBatch& B, int tn_max, int inc_max, int threads, int ctas, int iface_blocks,
+cudaError_t launch_vms_iteration(const DevBatch& B, int tn_max, int threads, int ctas, int iface_blocks,
                                  bool mixed, bool xpack, cudaStream_t s, cudaEvent_t* ev) {
-  const size_t smem = vms_smem_bytes(tn_max, inc_max, threads, mixed);
+  const size_t smem = vms_smem_bytes(tn_max, threads, mixed);
   if (ctas <= 0) ctas = vms_default_ctas(threads, mixed);
   if (ev) cudaEventRecord(ev[0], s);
   bool launched = false;
 #define FM_VMS_LAUNCH(T, M, C)                                                       \
   if (!launched && threads == T && mixed == M && ctas == C) {                        \
-    vms_tile_kernel<T, M, C><<<B.n_tiles, T, smem, s>>>(B, tn_max, inc_max);         \
+    vms_tile_kernel<T, M, C><<<B.n_tiles, T, smem, s>>>(B, tn_max);         \
     launched = true;                                                                 \
   }
   FM_VMS_VARIANTS(FM_VMS_LAUNCH)
@@ -759,13 +745,11 @@ static cudaError_t raise_dyn_smem(K k, int optin) {
 // opt-in maximum (the attribute is per kernel and process-wide, so a batch
 // with small tiles must not lower it below what another batch launches with;
 // the shared-memory carve-out still follows each launch's actual size).
-cudaError_t vms_configure(int tn_max, int inc_max) {
+cudaError_t vms_configure() {
   int dev = 0, optin = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  (void)tn_max;  // sizes are checked against the limit by the caller
-  (void)inc_max;
 #define FM_VMS_RAISE(T, M, C) \
   if (e == cudaSuccess) e = raise_dyn_smem(vms_tile_kernel<T, M, C>, optin);
   FM_VMS_VARIANTS(FM_VMS_RAISE)

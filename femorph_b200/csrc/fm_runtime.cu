@@ -29,9 +29,9 @@
 
 namespace fm {
 const char* last_error();
-size_t vms_smem_bytes(int tn_max, int inc_max, int threads, bool mixed);
-cudaError_t vms_configure(int tn_max, int inc_max);
-cudaError_t launch_vms_iteration(const DevBatch& B, int tn_max, int inc_max, int threads, int ctas, int iface_blocks,
+size_t vms_smem_bytes(int tn_max, int threads, bool mixed);
+cudaError_t vms_configure();
+cudaError_t launch_vms_iteration(const DevBatch& B, int tn_max, int threads, int ctas, int iface_blocks,
                                  bool mixed, bool xpack, cudaStream_t s, cudaEvent_t* ev);
 int vms_default_ctas(int threads, bool mixed);
 bool vms_variant_exists(int threads, bool mixed, int ctas);
@@ -173,7 +173,7 @@ struct Placement {
   fm_problem* p = nullptr;
   int64_t off[P_COUNT] = {0};
   int64_t len[P_COUNT] = {0};
-  int32_t tn_max = 0, inc_max = 0;
+  int32_t tn_max = 0, inc_max = 0;  // a tile's most nodes; SUPG: incidence entries
   std::shared_ptr<Layout> L;  // the problem's layout (node and element numbering)
   // VMS diagnostics (device, own allocations): per problem node its
   // (element slot * 4 + corner) entries in the problem's element order, the
@@ -270,45 +270,48 @@ static int put(T* dev_base, int64_t off, const T* src, int64_t n, cudaStream_t s
 }
 
 // Elements a tile when the caller gives none.  A problem of many tiles takes
-// full ones (1024 tets, VMS mixed 512, 384 hexa: the larger a tile, the fewer
+// full ones (1024 tets, VMS mixed 768, 384 hexa: the larger a tile, the fewer
 // nodes are staged and summed twice).  A problem of at most four waves of
 // CTAs takes tiles that fill its waves, so that no SM idles while others walk
-// a long tile: tiles of whole 128-element chunks below 512, of 32-element
-// steps above, at most 640 tets.  16^3 cavity (24,576 tets): 256 against 1024
-// a tile 20.6 against 43.0 us an iteration; 24^3: 256, 24.6 against 41.4;
-// 30^3: 384, 30.8 against 47.3; 36^3: 640, 44.1 against 47.3; 44^3: 576, 69.3
-// against 83.0; mixed 24^3: 256 against 512 22.6 against 28.7; hexa 93x37x29:
-// 256 against 384 68 against 78.  Not below 256, where a batch of many small
-// problems would pay for the extra interface nodes: 32 cavities of 8..24
-// cells a side take 148.7 us FP64 and 119.6 us mixed (full tiles 157.7 and
-// 118.6; with 128 as the least 170.3 and 140.3).  It depends on the problem
+// a long tile: whole 128-element chunks below 512, 32-element steps above, at
+// most 640 tets where four waves of those hold it, else up to full ones.
+// 16^3 cavity (24,576 tets): 256 against 1024 a tile 20.6 against 43.0 us an
+// iteration; 24^3: 256, 24.6 against 41.4; 30^3: 384, 29.4 against 47.3;
+// 36^3: 640, 39.3 (512: 47.6); 44^3: 576, 63.7 against 78.9; 64^3: 896, 160.7
+// against 167.6; mixed 24^3: 256 against 512 24.2 against 28.7; hexa
+// 93x37x29: 256 against 384 68 against 78.  Not below 256, where a batch of
+// many small problems would pay for the extra interface nodes (32 cavities of
+// 8..24 cells a side: 256 at least 148.7 us, 128 at least 170.3, full tiles
+// 157.7, measured before the warps took turns).  It depends on the problem
 // alone (its size, and the SM count of a B200 as a constant): a problem's
 // results do not depend on what else is in its batch.
 static int auto_tile_elems(int solver, int npe, int precision, int threads, int64_t E) {
   const bool vms_mixed = solver == FM_SOLVER_VMS && precision == FM_MIXED;
-  const int full = npe == 8 ? 384 : vms_mixed ? 512 : 1024;
+  const int full = npe == 8 ? 384 : vms_mixed ? 768 : 1024;
   if (threads != 128) return full;
   const int64_t slots = 148 * (vms_mixed ? 4 : 3);  // resident CTAs
-  const int64_t waves = std::max<int64_t>(1, (E + slots * std::min(full, 640) - 1) / (slots * std::min(full, 640)));
-  if (waves > 4) return full;
-  const int64_t te = (E + slots * waves - 1) / (slots * waves);
-  const int64_t up = te < 512 ? std::max<int64_t>(256, (te + 127) / 128 * 128) : (te + 31) / 32 * 32;
-  return (int)std::min<int64_t>(up, full);
+  for (const int most : {std::min(full, 640), full}) {
+    const int64_t waves = std::max<int64_t>(1, (E + slots * most - 1) / (slots * most));
+    if (waves > 4) continue;
+    const int64_t te = (E + slots * waves - 1) / (slots * waves);
+    const int64_t up = te < 512 ? std::max<int64_t>(256, (te + 127) / 128 * 128) : (te + 31) / 32 * 32;
+    return (int)std::min<int64_t>(up, full);
+  }
+  return full;
 }
 
 // Default launch shape.  tile_nodes: what still lets the CTAs that the kernels'
 // registers allow (VMS FP64 three, mixed four) fit an SM's shared memory; the
 // tiles of a mesh whose cells do not halve evenly have up to 500 nodes at
-// 1024 tets, and one such tile used to cost every CTA of the launch its third
-// neighbour (32 cavities of 8..48 cells a side, full tiles: 580 -> 491 us a
-// step).
+// 1024 tets, and one such tile would cost every CTA of the launch its third
+// neighbour.
 static void default_tuning(int solver, int npe, int precision, fm_tuning& t) {
   if (t.threads != 128 && t.threads != 256) t.threads = 128;
   const bool vms_mixed = solver == FM_SOLVER_VMS && precision == FM_MIXED;
   if (t.tile_elems < 0) t.tile_elems = 0;  // by the problem (auto_tile_elems)
   if (t.tile_nodes <= 0) {
     if (npe == 8) t.tile_nodes = 640;
-    else if (solver == FM_SOLVER_VMS && t.threads == 128) t.tile_nodes = vms_mixed ? 228 : 352;
+    else if (solver == FM_SOLVER_VMS && t.threads == 128) t.tile_nodes = vms_mixed ? 330 : 388;
     else t.tile_nodes = vms_mixed ? 256 : 512;
   }
   if (t.tile_nodes > 4096) t.tile_nodes = 4096;
@@ -366,8 +369,10 @@ static void pool_sizes(const fm_problem* p, const Layout& L, int64_t len[P_COUNT
   len[P_TILE] = (int64_t)L.tiles.size();
   len[P_TNODE] = (int64_t)L.tile_nodes.size();
   len[P_TCOL] = (int64_t)L.tile_cols.size();
-  len[P_TINC] = (int64_t)L.tile_inc.size();
-  len[P_TOFF] = (int64_t)L.tile_off.size();
+  // only the SUPG kernels read the incidence lists
+  const bool lists = p->params.solver == FM_SOLVER_SUPG;
+  len[P_TINC] = lists ? (int64_t)L.tile_inc.size() : 0;
+  len[P_TOFF] = lists ? (int64_t)L.tile_off.size() : 0;
   len[P_SLOT] = L.n_slots;
   len[P_IFACE] = (int64_t)L.iface_node.size();
   len[P_ISLOT] = (int64_t)L.iface_slots.size();
@@ -519,11 +524,11 @@ static int allocate(fm_batch* b, const int64_t cap[P_COUNT]) {
 static int configure(fm_batch* b) {
   if (b->tn_max <= b->configured_tn && b->inc_max <= b->configured_inc) return FM_OK;
   const int tn = std::max(b->tn_max, b->configured_tn), inc = std::max(b->inc_max, b->configured_inc);
-  size_t smem = b->solver == FM_SOLVER_VMS ? vms_smem_bytes(tn, inc, b->threads, b->precision == FM_MIXED)
+  size_t smem = b->solver == FM_SOLVER_VMS ? vms_smem_bytes(tn, b->threads, b->precision == FM_MIXED)
                                            : supg_smem_bytes(tn, inc, b->npe, b->threads, b->precision == FM_MIXED);
   // 227 KB opt-in limit per block, less room for the kernels' static shared memory
   if (smem + 1024 > 227 * 1024) return fail(FM_ERR_INVALID, "tile too large for shared memory; lower tile_nodes");
-  cudaError_t ce = b->solver == FM_SOLVER_VMS ? vms_configure(tn, inc) : supg_configure(smem, b->npe);
+  cudaError_t ce = b->solver == FM_SOLVER_VMS ? vms_configure() : supg_configure(smem, b->npe);
   if (ce != cudaSuccess) return fail(FM_ERR_CUDA, std::string("kernel attribute: ") + cudaGetErrorString(ce));
   b->configured_tn = tn;
   b->configured_inc = inc;
@@ -774,7 +779,7 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
       tm.problem = ps;
       pl.tn_max = std::max(pl.tn_max, tm.n_node);
     }
-    pl.inc_max = (L.max_tile_elems * npe + 7) / 8 * 8;
+    if (b->solver == FM_SOLVER_SUPG) pl.inc_max = (L.max_tile_elems * npe + 7) / 8 * 8;
     r = r ? r : put(const_cast<TileMeta*>(D.tiles), pl.off[P_TILE], tiles.data(), (int64_t)tiles.size(), s);
     if (noff == 0) {  // node ids need no relocation
       r = r ? r : put(const_cast<int32_t*>(D.tile_nodes), pl.off[P_TNODE], L.tile_nodes.data(),
@@ -786,8 +791,8 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
       CK(cudaStreamSynchronize(s));  // tnodes goes out of scope
     }
     r = r ? r : put(const_cast<int32_t*>(D.tile_cols), pl.off[P_TCOL], L.tile_cols.data(), (int64_t)L.tile_cols.size(), s);
-    r = r ? r : put(const_cast<uint16_t*>(D.tile_inc), pl.off[P_TINC], L.tile_inc.data(), (int64_t)L.tile_inc.size(), s);
-    r = r ? r : put(const_cast<uint16_t*>(D.tile_off), pl.off[P_TOFF], L.tile_off.data(), (int64_t)L.tile_off.size(), s);
+    r = r ? r : put(const_cast<uint16_t*>(D.tile_inc), pl.off[P_TINC], L.tile_inc.data(), pl.len[P_TINC], s);
+    r = r ? r : put(const_cast<uint16_t*>(D.tile_off), pl.off[P_TOFF], L.tile_off.data(), pl.len[P_TOFF], s);
   }
   // interface entries
   {
@@ -895,8 +900,9 @@ static void capacity_pools(const fm_capacity* cap, int te, int64_t c[P_COUNT]) {
   c[P_ELEM] = E + 2 * P * ELEM_ALIGN + c[P_TILE] * ELEM_ALIGN;
   c[P_TNODE] = 2 * N + (by_problem ? 48 : 16) * c[P_TILE];
   c[P_TCOL] = c[P_TILE] * 130;
-  c[P_TINC] = npe * E + 16 * c[P_TILE] + 16 * P;
-  c[P_TOFF] = c[P_TNODE] + c[P_TILE];
+  const bool lists = cap->solver == FM_SOLVER_SUPG;
+  c[P_TINC] = lists ? npe * E + 16 * c[P_TILE] + 16 * P : 0;
+  c[P_TOFF] = lists ? c[P_TNODE] + c[P_TILE] : 0;
   c[P_SLOT] = 2 * N + 32 * c[P_TILE];
   c[P_IFACE] = N;
   c[P_ISLOT] = c[P_SLOT];
@@ -1312,7 +1318,7 @@ int fm_batch_destroy(fm_batch* b) {
 // again after it).
 static cudaError_t launch_first(fm_batch* b, cudaStream_t s, cudaEvent_t* ev) {
   if (b->solver == FM_SOLVER_VMS)
-    return launch_vms_iteration(b->D, b->tn_max, b->inc_max, b->threads, b->tune.ctas_per_sm, b->iface_blocks,
+    return launch_vms_iteration(b->D, b->tn_max, b->threads, b->tune.ctas_per_sm, b->iface_blocks,
                                 b->precision == FM_MIXED, b->exchange, s, ev);
   return launch_supg_step(b->D, b->tn_max, b->inc_max, b->threads, b->iface_blocks, b->npe, b->precision == FM_MIXED,
                           b->exchange,

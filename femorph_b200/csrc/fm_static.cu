@@ -33,9 +33,9 @@
 #include "fm_internal.hpp"
 
 namespace fm {
-cudaError_t vms_configure(int tn_max, int inc_max);
-size_t vms_smem_bytes(int tn_max, int inc_max, int threads, bool mixed);
-cudaError_t launch_vms_iteration(const DevBatch& B, int tn_max, int inc_max, int threads, int ctas, int iface_blocks,
+cudaError_t vms_configure();
+size_t vms_smem_bytes(int tn_max, int threads, bool mixed);
+cudaError_t launch_vms_iteration(const DevBatch& B, int tn_max, int threads, int ctas, int iface_blocks,
                                  bool mixed, bool xpack, cudaStream_t s, cudaEvent_t* ev);
 }  // namespace fm
 
@@ -58,7 +58,7 @@ int scratch_address(int device, unsigned char** out) {
     cudaError_t e = cudaGetSymbolAddress((void**)&ptr, fm_static_scratch);
     if (e != cudaSuccess || !ptr)
       return fail(FM_ERR_CUDA, std::string("cudaGetSymbolAddress(fm_static_scratch): ") + cudaGetErrorString(e));
-    e = vms_configure(0, 0);  // kernels' shared-memory limit (no allocation)
+    e = vms_configure();  // kernels' shared-memory limit (no allocation)
     if (e != cudaSuccess) return fail(FM_ERR_CUDA, std::string("kernel attribute: ") + cudaGetErrorString(e));
     g_scratch_addr[device] = ptr;
   }
@@ -224,9 +224,8 @@ extern "C" int fm_vms_solve_static(fm_problem* p, int32_t nsteps, int32_t device
                                     " (about 200,000 tetrahedra): use fm_batch_create for larger problems");
   int tn_max = 0;
   for (const TileMeta& tm : L.tiles) tn_max = std::max(tn_max, tm.n_node);
-  const int inc_max = (L.max_tile_elems * 4 + 7) / 8 * 8;
   const int threads = 128;
-  if (tn_max > FM_MAX_TILE_NODES || vms_smem_bytes(tn_max, inc_max, threads, false) + 1024 > 227 * 1024)
+  if (tn_max > FM_MAX_TILE_NODES || vms_smem_bytes(tn_max, threads, false) + 1024 > 227 * 1024)
     return fail(FM_ERR_INVALID, "prepared tiles are too large for the VMS kernels");
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(FM_ERR_NODEVICE, "no CUDA device");
@@ -344,7 +343,7 @@ extern "C" int fm_vms_solve_static(fm_problem* p, int32_t nsteps, int32_t device
   CKS(cudaGetLastError());
   const int iface_blocks = (int)std::max<int64_t>(1, std::min<int64_t>((D.n_iface + 255) / 256, 148 * 8));
   for (int32_t it = 0; it < target; ++it)
-    CKS(launch_vms_iteration(D, tn_max, inc_max, threads, 0, iface_blocks, false, false, s, nullptr));
+    CKS(launch_vms_iteration(D, tn_max, threads, 0, iface_blocks, false, false, s, nullptr));
   double* du = reinterpret_cast<double*>(base + o.out_u);
   double* dp = reinterpret_cast<double*>(base + o.out_p);
   static_gather_kernel<<<blocks, 256, 0, s>>>(D, reinterpret_cast<const int32_t*>(base + o.in_node_new), (int32_t)N,
