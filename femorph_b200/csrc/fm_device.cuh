@@ -33,9 +33,6 @@ struct DevBatch {
   const TileMeta* tiles;
   int32_t n_tiles;
   const int32_t* tile_nodes;
-  const int32_t* tile_cols;
-  const uint16_t* tile_inc;       // per tile: node -> (element*npe + corner) entries, element order
-  const uint16_t* tile_off;       // per tile: n_node+1 offsets into tile_inc
   // interface
   double2* part;                  // [slot][2]: (c0, c1) (c2, c3), one 32-byte sector a slot
   const int32_t* iface_node;
@@ -121,6 +118,28 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   for (uint32_t i = 0; i < limit; ++i)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
+}
+
+// Named barrier `id` of two warps: the first waits for the second's arrival
+// and then sees what it wrote to shared memory before.
+// (An id known at compile time: a kernel that computes it reserves all 16.)
+template <int N>
+__device__ __forceinline__ void pair_wait(int id) {
+  if (id == N) asm volatile("barrier.cta.sync %0, 64;" ::"n"(N) : "memory");
+  else if constexpr (N > 1) pair_wait<N - 1>(id);
+}
+template <int N>
+__device__ __forceinline__ void pair_arrive(int id) {
+  if (id == N) asm volatile("barrier.cta.arrive %0, 64;" ::"n"(N) : "memory");
+  else if constexpr (N > 1) pair_arrive<N - 1>(id);
+}
+
+// Colour runs of a warp's 32 elements: `first` marks an element that starts a
+// colour.  Returns how many runs there are and this lane's run.
+__device__ __forceinline__ int colour_runs(bool first, int& mine) {
+  const unsigned firsts = __ballot_sync(0xffffffffu, first) & ~1u;
+  mine = __popc(firsts & (0xffffffffu >> (31 - (threadIdx.x & 31))));
+  return __popc(firsts) + 1;
 }
 
 // ---- reciprocal, inverse cube root and square root ----

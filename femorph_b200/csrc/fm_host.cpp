@@ -485,70 +485,6 @@ void morton_order(const fm_problem* p, hvec<int64_t>& order) {
   sort_by_key(code, order);
 }
 
-// Orders one tile's interface nodes for the node-owner accumulation of the
-// tile kernels, in which the thread p % FM_OWNER_THREADS adds up the
-// contributions of the tile's local node p.  Interior nodes keep positions
-// [0, n_int) (their batch ids are consecutive from local node 0); the
-// interface nodes, heaviest first (incident elements in the tile plus a fixed
-// cost per node), take a free position of the thread with the least work so
-// far (ties: the lowest thread).  Without it the threads that own an
-// interior node (up to 24 incident elements) also own as many interface
-// nodes as the others, and the slowest owner sets the length of every
-// chunk's accumulation.  Each node's sum keeps its element order, so the
-// results do not depend on this order.
-//   w_int / w_ifc: incident elements of the interior / interface nodes (in
-//   their current order); ifc: the interface nodes, reordered in place.
-constexpr int FM_OWNER_THREADS = 128;
-struct BalanceScratch {
-  std::vector<int32_t> by_w, count, out;
-  std::vector<uint64_t> heap;
-};
-static void balance_owners(const std::vector<int32_t>& w_int, const std::vector<int32_t>& w_ifc,
-                           std::vector<int32_t>& ifc, BalanceScratch& sc) {
-  const int n_int = (int)w_int.size(), n_ifc = (int)w_ifc.size(), n_node = n_int + n_ifc;
-  constexpr int64_t kNodeCost = 2;  // accumulator load / store and walk set-up, in entry units
-  int64_t load[FM_OWNER_THREADS] = {};
-  int next[FM_OWNER_THREADS];
-  for (int q = 0; q < n_int; ++q) load[q % FM_OWNER_THREADS] += w_int[q] + kNodeCost;
-  // min-heap of (load, thread) packed as load * 256 + thread (thread < 256,
-  // so the order is that of the pairs) over the threads with a free
-  // interface position
-  std::vector<uint64_t>& heap = sc.heap;
-  heap.clear();
-  for (int t = 0; t < FM_OWNER_THREADS; ++t) {
-    int q = n_int + ((t - n_int % FM_OWNER_THREADS) + FM_OWNER_THREADS) % FM_OWNER_THREADS;
-    next[t] = q;
-    if (q < n_node) heap.push_back((uint64_t)load[t] * 256u + (uint64_t)t);
-  }
-  std::make_heap(heap.begin(), heap.end(), std::greater<uint64_t>());
-  // interface nodes heaviest first, equal weights in their current order (a
-  // stable counting sort on the weight)
-  int32_t wmax = 0;
-  for (int32_t w : w_ifc) wmax = std::max(wmax, w);
-  std::vector<int32_t>& count = sc.count;
-  count.assign((size_t)wmax + 2, 0);
-  for (int32_t w : w_ifc) count[wmax - w + 1]++;
-  for (int32_t k = 0; k <= wmax; ++k) count[k + 1] += count[k];
-  std::vector<int32_t>& by_w = sc.by_w;
-  by_w.resize(n_ifc);
-  for (int32_t i = 0; i < n_ifc; ++i) by_w[count[wmax - w_ifc[i]]++] = i;
-  std::vector<int32_t>& out = sc.out;
-  out.resize(n_ifc);
-  for (int32_t i : by_w) {
-    std::pop_heap(heap.begin(), heap.end(), std::greater<uint64_t>());
-    const uint64_t key = heap.back();
-    heap.pop_back();
-    const int t = (int)(key & 255u);
-    out[next[t] - n_int] = ifc[i];
-    next[t] += FM_OWNER_THREADS;
-    if (next[t] < n_node) {
-      heap.push_back(key + (uint64_t)(w_ifc[i] + kNodeCost) * 256u);
-      std::push_heap(heap.begin(), heap.end(), std::greater<uint64_t>());
-    }
-  }
-  ifc.swap(out);
-}
-
 // Builds the batch layout:
 //  1. elements of each problem sorted by the Morton code of their centroid;
 //  2. cut greedily into tiles of <= tile_elems elements and <= tile_nodes
@@ -573,7 +509,6 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
   for (int pi = 0; pi < n; ++pi) {
     fm_problem* p = probs[pi];
     const int npe = p->etype;
-    const bool vms = p->params.solver == FM_SOLVER_VMS;
     const int64_t E = p->E, N = p->N;
     L.node_begin.push_back(node_base);
     L.elem_begin.push_back(elem_base);
@@ -664,17 +599,15 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
     int64_t next = iface_begin + ifc_at[ntile];
     for (int64_t i = 0; i < N; ++i)
       if (nn[i] < 0) nn[i] = (int32_t)(node_base + next++);  // isolated nodes
-    // 4./5. tiles: local nodes, colouring, local connectivity, incidence
-    // lists - built for every tile in parallel (per-worker scratch), then
+    // 4./5. tiles: local nodes, colouring, local connectivity - built for every tile in parallel (per-worker scratch), then
     // placed in tile order
     struct TileWork {
       std::vector<int32_t> inter, ifc;  // old node ids in local order
       std::vector<int32_t> eo;          // old element of each tile element (colour order)
       std::vector<uint16_t> conn;       // ne x npe tile-local ids
       std::vector<int32_t> colcnt;      // colour offsets (ncol + 1)
-      std::vector<uint16_t> off, inc;   // incidence offsets (n_node + 1) and entries (ne * npe)
       int ncol = 0;
-      int err = 0;                      // 1: > 128 colours, 2: 16-bit incidence overflow
+      int err = 0;                      // 1: > 128 colours, 2: 16-bit corner count overflow
     };
     std::vector<TileWork> tw(ntile);
     {
@@ -685,8 +618,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
         th.emplace_back([&, w] {
           std::vector<int32_t> local(N, -1);
           std::vector<uint64_t> used;                 // per-worker scratch, reused tile by tile
-          std::vector<int32_t> col, idx, cnt, pos, w_int, w_ifc, own;
-          BalanceScratch bal;
+          std::vector<int32_t> col, idx, pos, own;
           for (int t = (int)(ntile * w / nw); t < (int)(ntile * (w + 1) / nw); ++t) {
             TileWork& W = tw[t];
             own.clear();
@@ -702,8 +634,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
               }
             }
             // interior nodes in their (contiguous) batch order, then interface
-            // nodes by id, reordered to balance the owner threads.  The
-            // interior nodes and the interface nodes this tile touches first
+            // nodes by id.  The interior nodes and those this tile touches first
             // were numbered in this same first-touch walk, so they arrive in
             // id order; only the interface nodes of earlier tiles (all with
             // smaller ids) are sorted
@@ -713,35 +644,24 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             for (int32_t v : W.inter) local[v] = li++;
             for (int32_t v : W.ifc) local[v] = li++;
             const int32_t n_node = li;
-            if (!vms) {  // owner threads (SUPG tet4; hexa and VMS have none)
-              cnt.assign(n_node, 0);
-              for (int64_t oi = tile_start[t]; oi < tile_start[t + 1]; ++oi)
-                for (int a = 0; a < npe; ++a) cnt[local[cs[(size_t)oi * npe + a]]]++;
-              const int n_int = (int)W.inter.size();
-              w_int.assign(cnt.begin(), cnt.begin() + n_int);
-              w_ifc.assign(cnt.begin() + n_int, cnt.end());
-              balance_owners(w_int, w_ifc, W.ifc, bal);
-              li = n_int;
-              for (int32_t v : W.ifc) local[v] = li++;
-            }
             // colouring (greedy, up to 128 colours)
             const int64_t ne = tile_start[t + 1] - tile_start[t];
             used.assign(2 * (size_t)n_node, 0);
             col.resize(ne);
             int ncol = 0;
-            // VMS: a warp of the tile kernel adds up its 32 elements one colour
+            // A warp of the tile kernel adds up its 32 elements one colour
             // after another, so colours hold at most 32 elements, and a tile
-            // of enough warps (a node has up to 24 elements, hence 24 colours)
-            // spreads its elements over as many colours as it has warps,
-            // always to the emptiest one that fits: 36 colour runs in the 32
-            // warps of a 1024-tet tile, against 60 of the smallest colour
-            // that fits
+            // of enough warps (a node has up to 24 tets or 8 hexa, hence as
+            // many colours) spreads its elements over as many colours as it
+            // has warps, always to the emptiest one that fits: 36 colour runs
+            // in the 32 warps of a 1024-tet tile, against 60 of the smallest
+            // colour that fits
             const int nwarp = (int)((ne + 31) / 32);
-            const int even = vms && nwarp >= 26 && nwarp <= 64 ? nwarp : 0;
+            const int even = nwarp >= (npe == 4 ? 26 : 10) && nwarp <= 64 ? nwarp : 0;
             uint64_t level[33] = {0};  // colours below `even` by their size
             level[0] = even == 64 ? ~0ULL : (1ULL << even) - 1;
             int csize[128] = {0};
-            uint64_t full0 = 0, full1 = 0;  // VMS: colours with 32 elements
+            uint64_t full0 = 0, full1 = 0;  // colours with 32 elements
             for (int64_t i = 0; i < ne; ++i) {
               const int32_t* c = &cs[(size_t)(tile_start[t] + i) * npe];
               uint64_t m0 = full0, m1 = full1;
@@ -774,13 +694,13 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
                   break;
                 }
               }
-              if (vms && ++csize[k] >= 32) (k < 64 ? full0 : full1) |= 1ULL << (k & 63);
+              if (++csize[k] >= 32) (k < 64 ? full0 : full1) |= 1ULL << (k & 63);
               col[i] = k;
               ncol = std::max(ncol, k + 1);
               for (int a = 0; a < npe; ++a) used[2 * local[c[a]] + (k >> 6)] |= (1ULL << (k & 63));
             }
             if (W.err) continue;
-            if (vms) {
+            {
               // the largest colours first: they fill whole warps
               int by[128], at[128], n = 0;
               for (int k = 0; k < ncol; ++k)
@@ -790,8 +710,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
               for (int64_t i = 0; i < ne; ++i) col[i] = at[col[i]];
               ncol = n;
             }
-            // elements sorted by colour: SUPG processes a tile one colour at a
-            // time
+            // elements sorted by colour
             // (counting sort by colour: stable, as the element order within a
             // colour must stay the sorted order)
             W.ncol = ncol;
@@ -809,26 +728,26 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
               const int32_t* c = &cs[(size_t)oi * npe];
               for (int a = 0; a < npe; ++a) W.conn[(size_t)i * npe + a] = (uint16_t)local[c[a]];
             }
-            // node -> incident (element, corner) lists in element order
+            // entries of a tile are counted in 16 bits
             if (ne * npe > 65535) {
               W.err = 2;
               continue;
             }
-            cnt.assign(n_node + 1, 0);
-            for (int64_t i = 0; i < ne * npe; ++i) cnt[W.conn[i] + 1]++;
-            for (int k2 = 0; k2 < n_node; ++k2) cnt[k2 + 1] += cnt[k2];
-            W.off.resize(n_node + 1);
-            for (int k2 = 0; k2 <= n_node; ++k2) W.off[k2] = (uint16_t)cnt[k2];
-            W.inc.resize((size_t)ne * npe);
-            pos.assign(cnt.begin(), cnt.end() - 1);
-            for (int64_t i = 0; i < ne; ++i)
-              for (int a = 0; a < npe; ++a) W.inc[pos[W.conn[i * npe + a]]++] = (uint16_t)(i * npe + a);
-            // VMS: bit 15 of an element's second node id marks the first
+            // bit 15 of an element's second node id marks the first
             // element of a colour (the tile kernel's warps add up one colour
             // after another)
-            if (vms)
-              for (int k = 0; k < ncol; ++k)
+            for (int k = 0; k < ncol; ++k)
                 if (W.colcnt[k] < ne) W.conn[(size_t)W.colcnt[k] * npe + 1] |= 0x8000;
+            // and of a hexa's third one that its corners repeat a node (a
+            // collapsed hexa), so that they are added one by one
+            if (npe == 8)
+              for (int64_t i = 0; i < ne; ++i) {
+                const uint16_t* c = &W.conn[(size_t)i * 8];
+                bool same = false;
+                for (int a = 0; a < 8; ++a)
+                  for (int b = 0; b < a; ++b) same |= (c[a] & 0x7fff) == (c[b] & 0x7fff);
+                if (same) W.conn[(size_t)i * 8 + 2] |= 0x8000;
+              }
           }
         });
       for (auto& x : th) x.join();
@@ -839,15 +758,12 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
     }
     // placement: every tile starts at a multiple of ELEM_ALIGN element slots
     // (padding slots in between are never processed, so each chunk of a
-    // tile's element arrays starts on a 16-byte, in fact 128-byte, boundary)
-    // and its incidence entries at a multiple of 8; offsets first, then the
-    // blocks are copied in parallel
+    // tile's element arrays starts on a 16-byte, in fact 128-byte, boundary);
+    // offsets first, then the blocks are copied in parallel
     std::vector<TileMeta> tms(ntile);
-    int64_t e_out = 0, inc_prev = 0;
+    int64_t e_out = 0;
     {
-      int64_t tn_off = (int64_t)L.tile_nodes.size(), col_off = (int64_t)L.tile_cols.size();
-      int64_t inc_off = (int64_t)L.tile_inc.size(), off_off = (int64_t)L.tile_off.size(), sb = slot_base;
-      inc_prev = inc_off;
+      int64_t tn_off = (int64_t)L.tile_nodes.size(), col_off = (int64_t)L.tile_cols.size(), sb = slot_base;
       for (int t = 0; t < ntile; ++t) {
         const TileWork& W = tw[t];
         TileMeta& tm = tms[t];
@@ -862,27 +778,18 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
         tm.slot_base = (int32_t)sb;
         tm.col_begin = (int32_t)col_off;
         tm.n_col = W.ncol;
-        inc_off = (inc_off + 7) / 8 * 8;
-        tm.inc_begin = (int32_t)inc_off;
-        tm.off_begin = (int32_t)off_off;
         e_out += tm.n_elem;
         tn_off += tm.n_node;
         sb += (int64_t)W.ifc.size();
         col_off += (int64_t)W.colcnt.size();
-        inc_off += (int64_t)W.inc.size();
-        off_off += (int64_t)W.off.size();
         L.max_colors = std::max(L.max_colors, W.ncol);
         L.max_tile_elems = std::max<int32_t>(L.max_tile_elems, tm.n_elem);
       }
       // final sizes at once (the last problem includes the trailing
-      // padding: chunk copies round their length up to 16 bytes, and the
-      // incidence lists are copied in 16-byte pieces); the new ranges are
-      // first written by the per-tile copies below
-      const bool last_prob = pi == n - 1;
+      // padding: chunk copies round their length up to 16 bytes); the new
+      // ranges are first written by the per-tile copies below
       L.tile_nodes.resize(tn_off);
       L.tile_cols.resize(col_off);
-      L.tile_inc.resize(last_prob ? (inc_off + 7) / 8 * 8 + 8 : inc_off);
-      L.tile_off.resize(off_off);
       slot_base = sb;
     }
     e_out = (e_out + ELEM_ALIGN - 1) / ELEM_ALIGN * ELEM_ALIGN;
@@ -890,9 +797,6 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
     eo.resize(e_out);
     const int64_t conn_end = elem_base + e_out + (pi == n - 1 ? ELEM_ALIGN : 0);
     L.conn_local.resize((size_t)conn_end * npe);
-    const int64_t inc_end = (int64_t)L.tile_inc.size();
-    if (ntile > 0)  // alignment gap after the previous problem's entries
-      std::fill(L.tile_inc.begin() + inc_prev, L.tile_inc.begin() + tms[0].inc_begin, 0);
     // each tile fills its ranges and the padding up to the next tile (a few
     // tiles a block: the per-tile copies are large)
     parallel_blocks(ntile, [&](int64_t tb, int64_t te2, int) {
@@ -903,10 +807,6 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
         for (int32_t v : W.inter) *tn++ = nn[v];
         for (int32_t v : W.ifc) *tn++ = nn[v];
         std::copy(W.colcnt.begin(), W.colcnt.end(), L.tile_cols.begin() + tm.col_begin);
-        std::copy(W.off.begin(), W.off.end(), L.tile_off.begin() + tm.off_begin);
-        const int64_t inc_next = t + 1 < ntile ? tms[t + 1].inc_begin : inc_end;
-        std::copy(W.inc.begin(), W.inc.end(), L.tile_inc.begin() + tm.inc_begin);
-        std::fill(L.tile_inc.begin() + tm.inc_begin + (int64_t)W.inc.size(), L.tile_inc.begin() + inc_next, 0);
         const int64_t el_next = t + 1 < ntile ? tms[t + 1].elem_begin : conn_end;
         std::copy(W.conn.begin(), W.conn.end(), L.conn_local.begin() + (size_t)tm.elem_begin * npe);
         std::fill(L.conn_local.begin() + (size_t)(tm.elem_begin + tm.n_elem) * npe,
@@ -1016,10 +916,10 @@ namespace fm {
 // Checks the invariants the tile kernels rely on in one problem's layout
 // (one problem, built by build_layout): local connectivity inside the tile's
 // node list; distinct nodes in a tile, interior ones touched by this tile
-// only; elements of one colour sharing no node (the hexa8 colour rounds add
-// without ordering); every (element, corner) once in its node's incidence
-// list, in element order; each interface node's partial slots, one per
-// touching tile, in tile order; every element and node of the problem once.
+// only; elements of one colour sharing no node (a warp adds up a colour
+// without ordering) and the marks of the colours' first elements; each
+// interface node's partial slots, one per touching tile, in tile order; every
+// element and node of the problem once.
 int check_layout(const fm_problem* p, const Layout& L) {
   auto bad = [](const std::string& m) { return fail(FM_ERR_INVALID, "layout check: " + m); };
   const int npe = p->etype;
@@ -1060,14 +960,15 @@ int check_layout(const fm_problem* p, const Layout& L) {
       }
     }
     // local connectivity (bit 15 of the first id flags an FP64-Jacobian
-    // element in the mixed form, of the second one a colour's first element)
+    // element in the mixed form, of the second one a colour's first element,
+    // of the third one a collapsed hexa)
     const uint16_t* cl = &L.conn_local[(size_t)tm.elem_begin * npe];
     for (int32_t i = 0; i < ne; ++i) {
       const int64_t oe = L.elem_old[0][tm.elem_begin + i];
       if (oe < 0 || oe >= E || elem_seen[oe]) return bad("tile " + std::to_string(t) + ": element map");
       elem_seen[oe] = 1;
       for (int a = 0; a < npe; ++a) {
-        const int32_t ln = a <= 1 ? (cl[i * npe + a] & 0x7fff) : cl[i * npe + a];
+        const int32_t ln = cl[i * npe + a] & 0x7fff;
         if (ln >= nl) return bad("tile " + std::to_string(t) + ": local node id out of range");
         if (old_of[tn[ln]] != p->conn[oe * npe + a]) return bad("tile " + std::to_string(t) + ": connectivity");
       }
@@ -1079,11 +980,11 @@ int check_layout(const fm_problem* p, const Layout& L) {
     for (int32_t c = 0; c < tm.n_col; ++c)
       for (int32_t i = co[c]; i < co[c + 1]; ++i)
         for (int a = 0; a < npe; ++a) {
-          const int32_t ln = a <= 1 ? (cl[i * npe + a] & 0x7fff) : cl[i * npe + a];
+          const int32_t ln = cl[i * npe + a] & 0x7fff;
           if (colour_stamp[ln] == c) return bad("tile " + std::to_string(t) + ": two elements of a colour share a node");
           colour_stamp[ln] = c;
         }
-    if (p->params.solver == FM_SOLVER_VMS) {
+    {
       // the marks of the colours' first elements (not needed on the tile's first)
       std::vector<char> first(ne, 0);
       for (int32_t c = 1; c < tm.n_col; ++c)
@@ -1091,18 +992,6 @@ int check_layout(const fm_problem* p, const Layout& L) {
       for (int32_t i = 1; i < ne; ++i)
         if (((cl[i * npe + 1] & 0x8000) != 0) != (first[i] != 0)) return bad("tile " + std::to_string(t) + ": colour marks");
     }
-    // incidence lists
-    const uint16_t* off = &L.tile_off[tm.off_begin];
-    const uint16_t* inc = &L.tile_inc[tm.inc_begin];
-    if (off[0] != 0 || off[nl] != ne * npe) return bad("tile " + std::to_string(t) + ": incidence offsets");
-    for (int32_t l = 0; l < nl; ++l)
-      for (int32_t k = off[l]; k < off[l + 1]; ++k) {
-        const int32_t el = inc[k] / npe, a = inc[k] % npe;
-        if (el >= ne) return bad("tile " + std::to_string(t) + ": incidence element");
-        const int32_t ln = a <= 1 ? (cl[el * npe + a] & 0x7fff) : cl[el * npe + a];
-        if (ln != l) return bad("tile " + std::to_string(t) + ": incidence entry of another node");
-        if (k > off[l] && inc[k - 1] / npe >= el) return bad("tile " + std::to_string(t) + ": incidence order");
-      }
   }
   for (int64_t e = 0; e < E; ++e)
     if (!elem_seen[e]) return bad("element " + std::to_string(e) + " in no tile");

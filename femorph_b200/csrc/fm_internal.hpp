@@ -118,10 +118,8 @@ struct TileMeta {
   int32_t node_begin, n_node;   // range in tile_nodes
   int32_t n_int;                // first n_int local nodes are interior
   int32_t slot_base;            // partial slot of local node n_int
-  int32_t col_begin, n_col;     // colour offsets in tile_cols[col_begin .. +n_col]
+  int32_t col_begin, n_col;     // colour offsets in the layout's tile_cols[col_begin .. +n_col] (host)
   int32_t problem;
-  int32_t inc_begin;            // node->element incidence entries in tile_inc (multiple of 8)
-  int32_t off_begin;            // per-node offsets (n_node+1) into those entries, in tile_off
   int32_t node0;                // batch id of local node 0 when the interior nodes are
                                 // consecutive batch ids from it (-1 otherwise); set at placement
 };
@@ -196,10 +194,6 @@ struct Layout {
   std::vector<TileMeta> tiles;
   hvec<int32_t> tile_nodes;
   std::vector<int32_t> tile_cols;
-  // Per tile, for every local node, the (element-in-tile * npe + corner)
-  // entries of its incident elements in element order: the fixed order in
-  // which the node-owner threads add element contributions.
-  hvec<uint16_t> tile_inc, tile_off;
   int32_t max_tile_elems = 0;
   hvec<uint16_t> conn_local;          // n_elems x npe
   std::vector<int32_t> iface_node, iface_slot_beg, iface_slots, iface_prob;
@@ -218,8 +212,8 @@ constexpr int ELEM_ALIGN = 32;
 // SUPG hexa8 FP64: stored geometry values per Gauss point (inverse Jacobian
 // and det J), 8 points an element.
 constexpr int FM_GEO_PER_GP = 10;
-// VMS tiles: at most this many nodes (each CTA thread owns up to
-// FM_MAX_TILE_NODES / threads of them during accumulation).
+// VMS tiles: at most this many nodes (the shared memory of a CTA's
+// accumulators).
 #define FM_MAX_TILE_NODES 512
 
 int build_layout(fm_problem* const* probs, int n, int tile_elems, int tile_nodes, Layout& L);

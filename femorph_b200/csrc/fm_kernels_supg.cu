@@ -61,16 +61,14 @@ __device__ __forceinline__ void check_exit(const DevBatch& B, const DevProb& P, 
 // at three with its coefficients in shared memory 0.438 ms; tet4 at four
 // CTAs 0.170, at three 0.164 ms).
 //
-// Accumulation of the element contributions into the tile's nodes, in the
-// order of the elements (colour-sorted) in both schemes, so both give the
-// same sums:
-//  - tet4 (GATHER): element threads write their 12 entries to shared memory,
-//    then each node's owner thread adds the entries of this chunk's elements
-//    from the node's incidence list (two barriers a chunk; the one that
-//    frees the staged entries sits after the next chunk's element work);
-//  - hexa8: one round per colour present in the chunk (elements of one
-//    colour share no node), a barrier after each; the 24 entries a hexa
-//    would stage cost more shared memory than the barriers cost time.
+// Accumulation of the element contributions into the tile's nodes: in turn, as
+// in vms_tile_kernel (rings of warps, colour run by colour run), in an order
+// fixed by the tile.  tet4 has two rings; hexa8 one of four warps, for want of
+// shared memory.  Before, every thread staged its contributions and the
+// node's owner thread walked a list of its corners between two barriers a
+// chunk (tet4), or colours followed each other with a barrier each (hexa8):
+// 145 against 117 us a step on 1.57 M tets FP64, 135 against 111 mixed, and
+// 372 against 339 on 1.05 M hexa8 FP64, 330 against 295 mixed.
 //
 // The hexa8 kernels (GEO) read each Gauss point's inverse Jacobian and det J
 // from the geometry stored at placement (supg_geo_kernel; FP64, or rounded
@@ -78,8 +76,8 @@ __device__ __forceinline__ void check_exit(const DevBatch& B, const DevProb& P, 
 // coordinates at every step, and stage no coordinates.
 template <int NPE, int THREADS, bool MIXED, bool HISTORY>
 __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED && !HISTORY ? 4 : 3) : 1)
-    supg_tile_kernel(DevBatch B, int tn_max, int inc_max) {
-  constexpr bool GATHER = NPE == 4;
+    supg_tile_kernel(DevBatch B, int tn_max) {
+  constexpr int WARPS = THREADS / 32, SETS = supg_acc_sets(NPE), RING = WARPS / SETS;
   constexpr bool GEO = NPE == 8;
   extern __shared__ double sm[];
   double* s_x = sm;  // coordinates: tet4 only
@@ -88,16 +86,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
   double* s_u = s_z + (GEO ? 0 : tn_max);
   double* s_v = s_u + tn_max;
   double* s_w = s_v + tn_max;
-  double* s_a0 = s_w + tn_max;
-  double* s_a1 = s_a0 + tn_max;
-  double* s_a2 = s_a1 + tn_max;
-  // GATHER: [NPE * 3][THREADS] staged entries; hexa8: each thread's own
-  // column (supg_stage_doubles)
-  double* R = s_a2 + tn_max;
-  int32_t* s_col = (int32_t*)(R + supg_stage_doubles(NPE, MIXED, THREADS));  // colour offsets (<= 129)
-  uint16_t* s_inc = (uint16_t*)(s_col + 130);                      // GATHER: incidence entries
-  uint16_t* s_off = s_inc + (GATHER ? inc_max : 0);                // GATHER: per-node offsets
-  uint16_t* s_cur = s_off + (GATHER ? tn_max + 1 : 0);             // GATHER: per-node cursors
+  double* s_acc = s_w + tn_max;  // SETS x 3 x tn_max accumulators
+  double* R = s_acc + SETS * 3 * tn_max;  // hexa8: each thread's own column (supg_stage_doubles)
   __shared__ ShapeTable<NPE, double> s_shape;
   __shared__ ShapeTable<NPE, float> s_shape_f;
 
@@ -118,17 +108,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
     double u = B.su[g], v = B.sv[g], w = B.sw[g];
     mask_fixed(P.glob_fixed, u, v, w);
     s_u[ln] = u; s_v[ln] = v; s_w[ln] = w;
-    s_a0[ln] = 0.0; s_a1[ln] = 0.0; s_a2[ln] = 0.0;
-  }
-  for (int c = tid; c <= tm.n_col; c += THREADS) s_col[c] = B.tile_cols[tm.col_begin + c];
-  if (GATHER) {
-    for (int i = tid; i <= tm.n_node; i += THREADS) {
-      const uint16_t o = B.tile_off[tm.off_begin + i];
-      s_off[i] = o;
-      if (i < tm.n_node) s_cur[i] = o;
-    }
-    const int ninc = tm.n_elem * NPE;
-    for (int i = tid; i < ninc; i += THREADS) s_inc[i] = B.tile_inc[tm.inc_begin + i];
+#pragma unroll
+    for (int q = 0; q < 3 * SETS; ++q) s_acc[q * tn_max + ln] = 0.0;
   }
   if constexpr (MIXED) {
     fill_shape_table<NPE, double>(&s_shape);
@@ -136,15 +117,13 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
   }
   __syncthreads();
   const int64_t E = B.E;
-  // one lane asks L2 for a later tile's connectivity, incidence entries, AB2
-  // history rows and interior-node ranges (see vms_tile_kernel)
+  // one lane asks L2 for a later tile's connectivity, AB2 history rows and interior-node ranges (see vms_tile_kernel)
   if (B.l2_ahead > 0 && tid == THREADS - 32 && blockIdx.x + B.l2_ahead < (unsigned)B.n_tiles) {
     const TileMeta tn = B.tiles[blockIdx.x + B.l2_ahead];
     if (tn.problem >= 0 && tn.n_elem > 0) {
       const int64_t e0 = tn.elem_begin;  // multiple of 32 slots: 16-byte aligned rows
       const uint32_t cb = ((uint32_t)tn.n_elem * NPE * 2u + 15u) & ~15u;
       bulk_prefetch_l2(B.conn + e0 * NPE, cb);
-      if (GATHER) bulk_prefetch_l2(B.tile_inc + tn.inc_begin, cb);
       if (B.sdus) {
 #pragma unroll 1
         for (int q = 0; q < 3 * NPE; ++q) bulk_prefetch_l2(B.sdus + (int64_t)q * E + e0, ((uint32_t)tn.n_elem * 8u + 15u) & ~15u);
@@ -162,7 +141,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
       }
     }
   }
-  int c_lo = 0;
+  // the warps of a ring share a set of accumulators (see vms_tile_kernel)
+  const int warp = tid >> 5, ring = warp / RING, place = warp % RING;
+  double* w_acc = s_acc + ring * 3 * tn_max;
   using ConnRow = typename std::conditional<NPE == 4, uint2, uint4>::type;
   const ConnRow* conn_g = reinterpret_cast<const ConnRow*>(B.conn) + tm.elem_begin;
   // hexa8: the stored geometry of element le of this tile
@@ -188,6 +169,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
     double k[NPE][3];
     int ln[NPE];
     ConnRow cw = next;
+    // bit 15 of the second id: the first of a colour; of the third: a collapsed
+    // hexa, whose corners repeat a node
+    bool first = false, repeated = false;
     if constexpr (AHEAD) {
       if (le + THREADS < tm.n_elem) next = __ldg(conn_g + le + THREADS);
     } else {
@@ -195,6 +179,10 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
     }
     if (active) {
       const int64_t e = tm.elem_begin + le;
+      first = (cw.x >> 31) != 0;
+      cw.x &= 0x7fffffffu;
+      repeated = (cw.y & 0x8000u) != 0;
+      cw.y &= 0xffff7fffu;
       if constexpr (NPE == 4) {
         ln[0] = cw.x & 0xffff; ln[1] = cw.x >> 16; ln[2] = cw.y & 0xffff; ln[3] = cw.y >> 16;
       } else {
@@ -261,56 +249,42 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
       // the next chunk's first points on their way while this one is added up
       if (le + THREADS < tm.n_elem) geo_of(le + THREADS).start();
     }
-    if constexpr (GATHER) {
-      // the barrier that frees R (owners of the previous chunk done) comes
-      // after this chunk's element work, not at the end of the accumulation
-      if (base > 0) __syncthreads();
-      if (active) {
+    int mine;
+    const int colours = colour_runs(first, mine);
+    if (RING > 1 && base + place > 0) pair_wait<WARPS>(1 + warp);
+    for (int q = 0; q < colours; ++q) {
+      if (active && mine == q) {
 #pragma unroll
-        for (int a = 0; a < NPE; ++a)
+        for (int c = 0; c < 3; ++c) {
+          double* acc = w_acc + c * tn_max;
+          if (NPE == 8 && repeated) {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) R[(a * 3 + c) * THREADS + tid] = k[a][c];
-      }
-      __syncthreads();
-      // owners add this chunk's entries to their nodes, in element order
-      for (int n = tid; n < tm.n_node; n += THREADS) {
-        int c = s_cur[n];
-        const int ce = s_off[n + 1];
-        if (c >= ce) continue;
-        double a0 = s_a0[n], a1 = s_a1[n], a2 = s_a2[n];
-        while (c < ce) {
-          const int ent = s_inc[c];
-          const int col = ent / NPE - base;
-          if (col >= THREADS) break;
-          const double* Rp = R + (ent % NPE) * 3 * THREADS + col;
-          a0 += Rp[0];
-          a1 += Rp[THREADS];
-          a2 += Rp[2 * THREADS];
-          ++c;
-        }
-        s_cur[n] = (uint16_t)c;
-        s_a0[n] = a0; s_a1[n] = a1; s_a2[n] = a2;
-      }
-    } else {
-      while (c_lo < tm.n_col && s_col[c_lo + 1] <= base) ++c_lo;
-      for (int c = c_lo; c < tm.n_col && s_col[c] < base + THREADS; ++c) {
-        if (active && le >= s_col[c] && le < s_col[c + 1]) {
+            for (int a = 0; a < NPE; ++a) acc[ln[a]] += k[a][c];
+          } else {
+            double v[NPE];
 #pragma unroll
-          for (int a = 0; a < NPE; ++a) {
-            s_a0[ln[a]] += k[a][0];
-            s_a1[ln[a]] += k[a][1];
-            s_a2[ln[a]] += k[a][2];
+            for (int a = 0; a < NPE; ++a) v[a] = acc[ln[a]];
+#pragma unroll
+            for (int a = 0; a < NPE; ++a) acc[ln[a]] = v[a] + k[a][c];
           }
         }
-        __syncthreads();
       }
+      __syncwarp();
     }
+    if (RING > 1 && (base + THREADS < tm.n_elem || place + 1 < RING))
+      pair_arrive<WARPS>(1 + ring * RING + (place + 1) % RING);
   }
   __syncthreads();
   int32_t status = FM_OK;
   double max_u2 = 0.0;
   for (int l2 = tid; l2 < tm.n_node; l2 += THREADS) {
-    const double acc[3] = {s_a0[l2], s_a1[l2], s_a2[l2]};
+    double acc[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      acc[c] = s_acc[c * tn_max + l2];
+#pragma unroll
+      for (int q = 1; q < SETS; ++q) acc[c] += s_acc[(3 * q + c) * tn_max + l2];
+    }
     if (l2 < tm.n_int) {
       const int g = B.tile_nodes[tm.node_begin + l2];
       const double old[3] = {s_u[l2], s_v[l2], s_w[l2]};
@@ -348,8 +322,9 @@ __global__ void supg_geo_kernel(DevBatch B, int tile0) {
   for (int le = threadIdx.x; le < tm.n_elem; le += blockDim.x) {
     const int64_t e = tm.elem_begin + le;
     const uint4 cw = __ldg(reinterpret_cast<const uint4*>(B.conn) + e);
-    // bit 15 of the first id is the mixed form's FP64-Jacobian flag
-    const int ln[8] = {(int)(cw.x & 0x7fff), (int)(cw.x >> 16), (int)(cw.y & 0xffff), (int)(cw.y >> 16),
+    // bit 15 of the first three ids: the mixed form's FP64-Jacobian flag, the
+    // first of a colour, a collapsed hexa
+    const int ln[8] = {(int)(cw.x & 0x7fff), (int)((cw.x >> 16) & 0x7fff), (int)(cw.y & 0x7fff), (int)(cw.y >> 16),
                        (int)(cw.z & 0xffff), (int)(cw.z >> 16), (int)(cw.w & 0xffff), (int)(cw.w >> 16)};
 #pragma unroll 1
     for (int g = 0; g < 8; ++g) {
@@ -488,10 +463,9 @@ __global__ void supg_pressure_kernel(DevBatch B, int tn_max, double* pres) {
   }
 }
 
-size_t supg_smem_bytes(int tn_max, int inc_max, int npe, int threads, bool mixed) {
-  const bool gather = npe == 4;
-  return ((size_t)tn_max * (npe == 4 ? 9 : 6) + supg_stage_doubles(npe, mixed, threads)) * sizeof(double) +
-         130 * sizeof(int32_t) + (gather ? ((size_t)inc_max + 2 * (size_t)tn_max + 1) * sizeof(uint16_t) : 0);
+size_t supg_smem_bytes(int tn_max, int npe, int threads, bool mixed) {
+  return ((size_t)tn_max * ((npe == 4 ? 6 : 3) + 3 * supg_acc_sets(npe)) + supg_stage_doubles(npe, mixed, threads)) *
+         sizeof(double);
 }
 
 // Sets kernel k's dynamic shared-memory limit to the device's opt-in
@@ -547,12 +521,12 @@ cudaError_t supg_configure(size_t smem, int npe) {
   return e;
 }
 
-cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int inc_max, int threads, int iface_blocks, int npe,
+cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int threads, int iface_blocks, int npe,
                              bool mixed, bool xpack, cudaStream_t s, cudaEvent_t* ev) {
-  const size_t smem = supg_smem_bytes(tn_max, inc_max, npe, threads, mixed);
+  const size_t smem = supg_smem_bytes(tn_max, npe, threads, mixed);
   if (ev) cudaEventRecord(ev[0], s);
   auto k = npe == 4 ? supg_tile<4>(mixed, threads, B.sdus != nullptr) : supg_tile<8>(mixed, threads, B.sdus != nullptr);
-  k<<<B.n_tiles, threads == 256 ? 256 : 128, smem, s>>>(B, tn_max, inc_max);
+  k<<<B.n_tiles, threads == 256 ? 256 : 128, smem, s>>>(B, tn_max);
   if (ev) cudaEventRecord(ev[1], s);
   if (xpack)
     supg_xpack_kernel<<<iface_blocks, 256, 0, s>>>(B);

@@ -215,20 +215,6 @@ constexpr int FM_ACC_SETS = 2;
 // eight 4-bank groups.
 __device__ __forceinline__ int acc_index(int ln, int h) { return ln * 2 + (h ^ ((ln >> 2) & 1)); }
 
-// Named barrier `id` of two warps: the first waits for the second's arrival
-// and then sees what it wrote to shared memory before.
-// (An id known at compile time: a kernel that computes it reserves all 16.)
-template <int N>
-__device__ __forceinline__ void pair_wait(int id) {
-  if (id == N) asm volatile("barrier.cta.sync %0, 64;" ::"n"(N) : "memory");
-  else if constexpr (N > 1) pair_wait<N - 1>(id);
-}
-template <int N>
-__device__ __forceinline__ void pair_arrive(int id) {
-  if (id == N) asm volatile("barrier.cta.arrive %0, 64;" ::"n"(N) : "memory");
-  else if constexpr (N > 1) pair_arrive<N - 1>(id);
-}
-
 // MINB: resident CTAs an SM the variant is compiled for (its register budget).
 //
 // The warps of a ring take turns with a set of accumulators: warp w's turn of
@@ -445,9 +431,8 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
     if (!MIXED) asm volatile("" : "+r"(cw.x), "+r"(cw.y));
     int ln[4];
     corners(cw, ln);
-    const unsigned firsts = __ballot_sync(0xffffffffu, (cw.x >> 31) != 0) & ~1u;
-    const int mine = __popc(firsts & (0xffffffffu >> (31 - lane)));
-    const int colours = __popc(firsts) + 1;
+    int mine;
+    const int colours = colour_runs((cw.x >> 31) != 0, mine);
     if (RING > 1 && k + place > 0) pair_wait<WARPS>(1 + warp);
     for (int c = 0; c < colours; ++c) {
       if (active && mine == c) {

@@ -39,9 +39,9 @@ cudaError_t launch_vms_xupdate(const DevBatch& B, int blocks, cudaStream_t s);
 cudaError_t launch_vms_diagnostics(const DevBatch& B, const double* cres_buf, const int32_t* off, const int32_t* ent,
                                    int32_t n_nodes, const int32_t* eo, int64_t eb, int64_t ec, int64_t nb,
                                    double* el, double* out, int blocks, cudaStream_t s);
-size_t supg_smem_bytes(int tn_max, int inc_max, int npe, int threads, bool mixed);
+size_t supg_smem_bytes(int tn_max, int npe, int threads, bool mixed);
 cudaError_t supg_configure(size_t smem, int npe);
-cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int inc_max, int threads, int iface_blocks, int npe, bool mixed,
+cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int threads, int iface_blocks, int npe, bool mixed,
                              bool xpack, cudaStream_t s, cudaEvent_t* ev);
 cudaError_t launch_supg_xupdate(const DevBatch& B, int blocks, cudaStream_t s);
 cudaError_t launch_supg_geo(const DevBatch& B, int tile0, int ntiles, int tn_max, cudaStream_t s);
@@ -165,7 +165,7 @@ struct Pool {
   }
 };
 
-enum PoolId { P_NODE, P_ELEM, P_TILE, P_TNODE, P_TCOL, P_TINC, P_TOFF, P_SLOT, P_IFACE, P_ISLOT, P_REC, P_TAB, P_ROW, P_PROB,
+enum PoolId { P_NODE, P_ELEM, P_TILE, P_TNODE, P_SLOT, P_IFACE, P_ISLOT, P_REC, P_TAB, P_ROW, P_PROB,
               P_COUNT };
 
 struct Placement {
@@ -173,7 +173,7 @@ struct Placement {
   fm_problem* p = nullptr;
   int64_t off[P_COUNT] = {0};
   int64_t len[P_COUNT] = {0};
-  int32_t tn_max = 0, inc_max = 0;  // a tile's most nodes; SUPG: incidence entries
+  int32_t tn_max = 0;  // a tile's most nodes
   std::shared_ptr<Layout> L;  // the problem's layout (node and element numbering)
   // VMS diagnostics (device, own allocations): per problem node its
   // (element slot * 4 + corner) entries in the problem's element order, the
@@ -198,8 +198,8 @@ struct fm_batch {
   std::vector<Placement> slots;     // by problem slot (P_PROB offset)
   DevBatch D{};
   std::vector<void*> allocs;
-  int tn_max = 0, inc_max = 0, threads = 128, iface_blocks = 1, graph_steps = 0;
-  int configured_tn = 0, configured_inc = 0;
+  int tn_max = 0, threads = 128, iface_blocks = 1, graph_steps = 0;
+  int configured_tn = 0;
   bool has_history = false;
   std::vector<int32_t> iters;       // host copy of each slot's completed iterations
   int32_t* h_targets = nullptr;     // pinned staging of the target array
@@ -325,7 +325,7 @@ static void default_tuning(int solver, int npe, int precision, fm_tuning& t) {
 static int prepare(fm_problem* p, const fm_tuning& t, std::shared_ptr<Layout>* out) {
   const int te = t.tile_elems > 0 ? t.tile_elems
                                   : auto_tile_elems(p->params.solver, p->etype, p->params.precision, t.threads, p->E);
-  const int tn = t.tile_nodes;
+  int tn = t.tile_nodes;
   if (p->layout && p->layout_te == te && p->layout_tn == tn) {
     *out = p->layout;
     return FM_OK;
@@ -334,6 +334,23 @@ static int prepare(fm_problem* p, const fm_tuning& t, std::shared_ptr<Layout>* o
   fm_problem* arr[1] = {p};
   int r = build_layout(arr, 1, te, tn, *L);
   if (r) return r;
+  if (p->params.solver == FM_SOLVER_SUPG) {
+    // A caller's node limit may give tiles that the SUPG kernels' shared
+    // memory does not hold (tet4 2400 nodes, FP64 hexa8 with 256 threads
+    // 2943): those of up to 3200 nodes are cut smaller, larger ones are left
+    // to be refused when the batch is formed.
+    const bool mixed = p->params.precision == FM_MIXED;
+    const size_t base = supg_smem_bytes(0, p->etype, t.threads, mixed);
+    const int fit = (int)((227 * 1024 - 1024 - base) / (supg_smem_bytes(1, p->etype, t.threads, mixed) - base));
+    int most = 0;
+    for (const TileMeta& tm : L->tiles) most = std::max<int>(most, tm.n_node);
+    if (most > fit && most <= 3200) {
+      tn = fit;
+      L = std::make_shared<Layout>();
+      r = build_layout(arr, 1, te, tn, *L);
+      if (r) return r;
+    }
+  }
   if (p->params.precision == FM_MIXED) {
     // mixed form: elements whose Jacobian inverse stays in FP64 (aspect ratio
     // above the limit) are flagged in bit 15 of their first tile-local node id
@@ -368,11 +385,6 @@ static void pool_sizes(const fm_problem* p, const Layout& L, int64_t len[P_COUNT
   len[P_ELEM] = L.n_elems;  // includes the trailing over-read padding
   len[P_TILE] = (int64_t)L.tiles.size();
   len[P_TNODE] = (int64_t)L.tile_nodes.size();
-  len[P_TCOL] = (int64_t)L.tile_cols.size();
-  // only the SUPG kernels read the incidence lists
-  const bool lists = p->params.solver == FM_SOLVER_SUPG;
-  len[P_TINC] = lists ? (int64_t)L.tile_inc.size() : 0;
-  len[P_TOFF] = lists ? (int64_t)L.tile_off.size() : 0;
   len[P_SLOT] = L.n_slots;
   len[P_IFACE] = (int64_t)L.iface_node.size();
   len[P_ISLOT] = (int64_t)L.iface_slots.size();
@@ -381,7 +393,7 @@ static void pool_sizes(const fm_problem* p, const Layout& L, int64_t len[P_COUNT
   len[P_ROW] = (int64_t)p->tab_rows.size() / 4;
   len[P_PROB] = 1;
 }
-static const int64_t kAlign[P_COUNT] = {1, ELEM_ALIGN, 1, 1, 1, 8, 1, 1, 1, 1, 1, 1, 1, 1};
+static const int64_t kAlign[P_COUNT] = {1, ELEM_ALIGN, 1, 1, 1, 1, 1, 1, 1, 1, 1};
 
 // Doubles of the read-back piece: all of a small batch's nodal output, at most
 // 32 MB.
@@ -403,8 +415,7 @@ static int allocate(fm_batch* b, const int64_t cap[P_COUNT]) {
   int32_t* nbc;
   uint16_t* conn;
   TileMeta* tiles;
-  int32_t *tnodes, *tcols;
-  uint16_t *tinc, *toff;
+  int32_t* tnodes;
   int32_t *inode, *isb, *isc, *iprob, *islots;
   BCRec* recs;
   int32_t *toffs, *tlens;
@@ -448,9 +459,6 @@ static int allocate(fm_batch* b, const int64_t cap[P_COUNT]) {
     }
     A((void**)&tiles, std::max<int64_t>(cap[P_TILE], 1) * sizeof(TileMeta));
     A((void**)&tnodes, std::max<int64_t>(cap[P_TNODE], 1) * sizeof(int32_t));
-    A((void**)&tcols, std::max<int64_t>(cap[P_TCOL], 1) * sizeof(int32_t));
-    A((void**)&tinc, std::max<int64_t>(cap[P_TINC], 8) * sizeof(uint16_t));
-    A((void**)&toff, std::max<int64_t>(cap[P_TOFF], 1) * sizeof(uint16_t));
     A((void**)&D.part, std::max<int64_t>(cap[P_SLOT], 1) * 4 * sizeof(double));
     for (int32_t** q : {&inode, &isb, &isc, &iprob}) A((void**)q, std::max<int64_t>(cap[P_IFACE], 1) * sizeof(int32_t));
     A((void**)&islots, std::max<int64_t>(cap[P_ISLOT], 1) * sizeof(int32_t));
@@ -486,7 +494,7 @@ static int allocate(fm_batch* b, const int64_t cap[P_COUNT]) {
   D.x = x; D.y = y; D.z = z; D.su = su; D.sv = sv; D.sw = sw; D.sp = sp;
   D.pu = pu; D.pv = pv; D.pw = pw; D.pp = pp; D.mass = ms; D.node_bc = nbc;
   D.conn = conn; D.E = NE;
-  D.tiles = tiles; D.tile_nodes = tnodes; D.tile_cols = tcols; D.tile_inc = tinc; D.tile_off = toff;
+  D.tiles = tiles; D.tile_nodes = tnodes;
   D.iface_node = inode; D.iface_slot_beg = isb; D.iface_slot_cnt = isc; D.iface_prob = iprob; D.iface_slots = islots;
   D.recs = recs; D.tab_off = toffs; D.tab_len = tlens; D.tab_rows = rows;
   D.probs = dp; D.pstate = ds; D.target = tg; D.q1p = q1; D.done = done;
@@ -522,16 +530,15 @@ static int allocate(fm_batch* b, const int64_t cap[P_COUNT]) {
 
 // Makes the kernels' shared-memory limits cover the current tile maxima.
 static int configure(fm_batch* b) {
-  if (b->tn_max <= b->configured_tn && b->inc_max <= b->configured_inc) return FM_OK;
-  const int tn = std::max(b->tn_max, b->configured_tn), inc = std::max(b->inc_max, b->configured_inc);
+  if (b->tn_max <= b->configured_tn) return FM_OK;
+  const int tn = b->tn_max;
   size_t smem = b->solver == FM_SOLVER_VMS ? vms_smem_bytes(tn, b->threads, b->precision == FM_MIXED)
-                                           : supg_smem_bytes(tn, inc, b->npe, b->threads, b->precision == FM_MIXED);
+                                           : supg_smem_bytes(tn, b->npe, b->threads, b->precision == FM_MIXED);
   // 227 KB opt-in limit per block, less room for the kernels' static shared memory
   if (smem + 1024 > 227 * 1024) return fail(FM_ERR_INVALID, "tile too large for shared memory; lower tile_nodes");
   cudaError_t ce = b->solver == FM_SOLVER_VMS ? vms_configure() : supg_configure(smem, b->npe);
   if (ce != cudaSuccess) return fail(FM_ERR_CUDA, std::string("kernel attribute: ") + cudaGetErrorString(ce));
   b->configured_tn = tn;
-  b->configured_inc = inc;
   return FM_OK;
 }
 
@@ -541,14 +548,10 @@ static void refresh_extent(fm_batch* b) {
   D.n_iface = (int32_t)b->pools[P_IFACE].hwm;
   D.n_probs = (int32_t)b->pools[P_PROB].hwm;
   b->iface_blocks = (int)std::max<int64_t>(1, std::min<int64_t>((D.n_iface + 255) / 256, 148 * 8));
-  int tn = 0, inc = 0;
+  int tn = 0;
   for (const Placement& pl : b->slots)
-    if (pl.p) {
-      tn = std::max(tn, pl.tn_max);
-      inc = std::max(inc, pl.inc_max);
-    }
+    if (pl.p) tn = std::max(tn, pl.tn_max);
   b->tn_max = tn;
-  b->inc_max = inc;
   if (b->graph) {
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
@@ -764,9 +767,6 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
       tm.elem_begin += (int32_t)eoff;
       tm.node_begin += (int32_t)pl.off[P_TNODE];
       tm.slot_base += (int32_t)soff;
-      tm.col_begin += (int32_t)pl.off[P_TCOL];
-      tm.inc_begin += (int32_t)pl.off[P_TINC];
-      tm.off_begin += (int32_t)pl.off[P_TOFF];
       // the look-ahead prefetch reads node0 .. node0 + n_int - 1: checked to
       // be the tile's interior nodes (consecutive by construction), else -1
       // (no node prefetch for the tile)
@@ -779,7 +779,6 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
       tm.problem = ps;
       pl.tn_max = std::max(pl.tn_max, tm.n_node);
     }
-    if (b->solver == FM_SOLVER_SUPG) pl.inc_max = (L.max_tile_elems * npe + 7) / 8 * 8;
     r = r ? r : put(const_cast<TileMeta*>(D.tiles), pl.off[P_TILE], tiles.data(), (int64_t)tiles.size(), s);
     if (noff == 0) {  // node ids need no relocation
       r = r ? r : put(const_cast<int32_t*>(D.tile_nodes), pl.off[P_TNODE], L.tile_nodes.data(),
@@ -790,9 +789,6 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
       r = r ? r : put(const_cast<int32_t*>(D.tile_nodes), pl.off[P_TNODE], tnodes.data(), (int64_t)tnodes.size(), s);
       CK(cudaStreamSynchronize(s));  // tnodes goes out of scope
     }
-    r = r ? r : put(const_cast<int32_t*>(D.tile_cols), pl.off[P_TCOL], L.tile_cols.data(), (int64_t)L.tile_cols.size(), s);
-    r = r ? r : put(const_cast<uint16_t*>(D.tile_inc), pl.off[P_TINC], L.tile_inc.data(), pl.len[P_TINC], s);
-    r = r ? r : put(const_cast<uint16_t*>(D.tile_off), pl.off[P_TOFF], L.tile_off.data(), pl.len[P_TOFF], s);
   }
   // interface entries
   {
@@ -899,10 +895,6 @@ static void capacity_pools(const fm_capacity* cap, int te, int64_t c[P_COUNT]) {
   if (by_problem) c[P_TILE] = std::min<int64_t>(E / 128 + 2 * P, c[P_TILE] + 4096 * P);
   c[P_ELEM] = E + 2 * P * ELEM_ALIGN + c[P_TILE] * ELEM_ALIGN;
   c[P_TNODE] = 2 * N + (by_problem ? 48 : 16) * c[P_TILE];
-  c[P_TCOL] = c[P_TILE] * 130;
-  const bool lists = cap->solver == FM_SOLVER_SUPG;
-  c[P_TINC] = lists ? npe * E + 16 * c[P_TILE] + 16 * P : 0;
-  c[P_TOFF] = lists ? c[P_TNODE] + c[P_TILE] : 0;
   c[P_SLOT] = 2 * N + 32 * c[P_TILE];
   c[P_IFACE] = N;
   c[P_ISLOT] = c[P_SLOT];
@@ -922,8 +914,7 @@ static int64_t pool_bytes(const int64_t cap[P_COUNT], int solver, int npe, int p
   else if (solver == FM_SOLVER_VMS || history) b += NE * (solver == FM_SOLVER_VMS ? 12 : 3 * npe) * 8;
   if (solver == FM_SOLVER_SUPG) b += NE * 3 * 8;
   if (solver == FM_SOLVER_SUPG && npe == 8) b += NE * 8 * FM_GEO_PER_GP * (prec == FM_MIXED ? 4 : 8);
-  b += at_least(cap[P_TILE], 1) * (int64_t)sizeof(TileMeta) + at_least(cap[P_TNODE], 1) * 4 +
-       at_least(cap[P_TCOL], 1) * 4 + at_least(cap[P_TINC], 8) * 2 + at_least(cap[P_TOFF], 1) * 2;
+  b += at_least(cap[P_TILE], 1) * (int64_t)sizeof(TileMeta) + at_least(cap[P_TNODE], 1) * 4;
   b += at_least(cap[P_SLOT], 1) * 4 * 8 + at_least(cap[P_IFACE], 1) * 4 * 4 + at_least(cap[P_ISLOT], 1) * 4;
   b += at_least(cap[P_REC], 1) * (int64_t)sizeof(BCRec) + at_least(cap[P_TAB], 1) * 2 * 4 + at_least(cap[P_ROW], 1) * 32;
   const int64_t NP = at_least(cap[P_PROB], 1);
@@ -1096,7 +1087,7 @@ int fm_batch_estimate_bytes(fm_problem* const* probs, int32_t n, const fm_tuning
   const bool vms = probs[0]->params.solver == FM_SOLVER_VMS;
   const bool mixed = probs[0]->params.precision == FM_MIXED;
   // nodes: 12 FP64 arrays + BC index; elements: connectivity + history;
-  // tiles, incidence lists and interface partials: ~40 B per element
+  // tiles and interface partials: within 40 B per element
   const int64_t per_e = (int64_t)npe * 2 + (vms ? (mixed ? 48 : 96) : (3 * npe * 8 + 24)) + 40 +
                         (!vms && npe == 8 ? 8 * FM_GEO_PER_GP * (mixed ? 4 : 8) : 0);
   *bytes = N * 104 + E * (per_e + 4) + out_doubles(N) * 8 + (16 << 20);
@@ -1320,7 +1311,7 @@ static cudaError_t launch_first(fm_batch* b, cudaStream_t s, cudaEvent_t* ev) {
   if (b->solver == FM_SOLVER_VMS)
     return launch_vms_iteration(b->D, b->tn_max, b->threads, b->tune.ctas_per_sm, b->iface_blocks,
                                 b->precision == FM_MIXED, b->exchange, s, ev);
-  return launch_supg_step(b->D, b->tn_max, b->inc_max, b->threads, b->iface_blocks, b->npe, b->precision == FM_MIXED,
+  return launch_supg_step(b->D, b->tn_max, b->threads, b->iface_blocks, b->npe, b->precision == FM_MIXED,
                           b->exchange,
                           s, ev);
 }

@@ -78,8 +78,8 @@ struct Carve {
 };
 
 struct Offsets {
-  size_t node[12], node_bc, recs, tab_off, tab_len, tab_rows, conn, sdus, tiles, tile_nodes, tile_cols, tile_inc,
-      tile_off, part, iface_node, iface_beg, iface_cnt, iface_prob, iface_slots, prob, pstate, target, q1p, done,
+  size_t node[12], node_bc, recs, tab_off, tab_len, tab_rows, conn, sdus, tiles, tile_nodes, part,
+      iface_node, iface_beg, iface_cnt, iface_prob, iface_slots, prob, pstate, target, q1p, done,
       in_coords, in_init, in_rec, in_mass, in_node_new, out_u, out_p, total;
 };
 
@@ -97,9 +97,6 @@ Offsets plan(const fm_problem* p, const Layout& L) {
   o.sdus = c.take<double>(12 * NE);
   o.tiles = c.take<TileMeta>(L.tiles.size());
   o.tile_nodes = c.take<int32_t>(L.tile_nodes.size());
-  o.tile_cols = c.take<int32_t>(L.tile_cols.size());
-  o.tile_inc = c.take<uint16_t>(L.tile_inc.size());
-  o.tile_off = c.take<uint16_t>(L.tile_off.size());
   o.part = c.take<double>((size_t)L.n_slots * 4);
   o.iface_node = c.take<int32_t>(NI);
   o.iface_beg = c.take<int32_t>(NI + 1);
@@ -257,9 +254,6 @@ extern "C" int fm_vms_solve_static(fm_problem* p, int32_t nsteps, int32_t device
   D.tiles = reinterpret_cast<TileMeta*>(base + o.tiles);
   D.n_tiles = (int32_t)L.tiles.size();
   D.tile_nodes = reinterpret_cast<int32_t*>(base + o.tile_nodes);
-  D.tile_cols = reinterpret_cast<int32_t*>(base + o.tile_cols);
-  D.tile_inc = reinterpret_cast<uint16_t*>(base + o.tile_inc);
-  D.tile_off = reinterpret_cast<uint16_t*>(base + o.tile_off);
   D.part = reinterpret_cast<double2*>(base + o.part);
   D.iface_node = reinterpret_cast<int32_t*>(base + o.iface_node);
   D.iface_slot_beg = reinterpret_cast<int32_t*>(base + o.iface_beg);
@@ -315,9 +309,6 @@ extern "C" int fm_vms_solve_static(fm_problem* p, int32_t nsteps, int32_t device
   CKS(up(base, o.conn, L.conn_local.data(), L.conn_local.size(), s));
   CKS(up(base, o.tiles, L.tiles.data(), L.tiles.size(), s));
   CKS(up(base, o.tile_nodes, L.tile_nodes.data(), L.tile_nodes.size(), s));
-  CKS(up(base, o.tile_cols, L.tile_cols.data(), L.tile_cols.size(), s));
-  CKS(up(base, o.tile_inc, L.tile_inc.data(), L.tile_inc.size(), s));
-  CKS(up(base, o.tile_off, L.tile_off.data(), L.tile_off.size(), s));
   CKS(up(base, o.iface_node, L.iface_node.data(), L.iface_node.size(), s));
   CKS(up(base, o.iface_beg, L.iface_slot_beg.data(), L.iface_slot_beg.size(), s));
   CKS(up(base, o.iface_prob, L.iface_prob.data(), L.iface_prob.size(), s));

@@ -214,12 +214,14 @@ using GeoStream64 = GeoStream<double, THREADS, FM_GEO_ROWS64, true>;
 template <int THREADS>
 using GeoStream32 = GeoStream<float, THREADS, FM_GEO_ROWS32, false>;
 
-// Doubles a thread of the tile kernels' per-thread region: tet4 the 12
-// staged entries; hexa8 FP64 the 24 velocity coefficients and the geometry
-// rows; hexa8 mixed its geometry rows.
+// Doubles of the tile kernels' per-thread region (hexa8): FP64 the 24 velocity
+// coefficients and the geometry rows, mixed its geometry rows.
 __host__ __device__ constexpr size_t supg_stage_doubles(int npe, bool mixed, int threads) {
-  return (size_t)threads * (npe == 4 ? 12 : mixed ? FM_GEO_ROWS32 * FM_GEO_PER_GP / 2 : 24 + FM_GEO_ROWS64 * FM_GEO_PER_GP);
+  return npe == 4 ? 0
+                  : (size_t)threads * (mixed ? FM_GEO_ROWS32 * FM_GEO_PER_GP / 2 : 24 + FM_GEO_ROWS64 * FM_GEO_PER_GP);
 }
+// Sets of accumulators (rings of warps).
+__host__ __device__ constexpr int supg_acc_sets(int npe) { return npe == 4 ? 2 : 1; }
 
 // Inverse (cofactors, femUtils.cpp:716-770) and determinant of a 3x3 matrix.
 __device__ __forceinline__ double inverse3(const double J[3][3], double inv[3][3]) {

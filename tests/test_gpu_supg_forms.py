@@ -89,3 +89,29 @@ def test_both_integrators_in_one_batch(npe, precision):
             assert np.array_equal(x, y)
         c.close()
         h.close()
+
+
+@pytest.mark.parametrize("precision", [api.FM_FP64, api.FM_MIXED])
+@pytest.mark.parametrize("ab2,bbar", [(0, 0), (1, 1)])
+@pytest.mark.parametrize("threads", [128, 256])
+def test_collapsed_hexa(threads, ab2, bbar, precision):
+    """Every third cell split into two wedges, written as hexas whose corners
+    repeat a node: those are added into their nodes corner by corner."""
+    p = mesh.channel(9, 5, 3, seed=6, noise=1e-2, ex_opts=(1 - ab2, bbar, 1, 1, 1, 1))
+    conn = []
+    for i, c in enumerate(np.asarray(p.conn).reshape(-1, 8)):
+        if i % 3:
+            conn.append(c)
+        else:
+            conn += [c[[0, 1, 2, 2, 4, 5, 6, 6]], c[[0, 2, 3, 3, 4, 6, 7, 7]]]
+    p.conn = np.ascontiguousarray(conn, dtype=p.conn.dtype)
+    compare(p, precision, threads=threads)
+
+
+@pytest.mark.parametrize("npe,tile_elems,tile_nodes", [(4, 14000, 2700), (8, 2600, 3100)])
+def test_node_limit_above_shared_memory(npe, tile_elems, tile_nodes):
+    """A node limit whose tiles the kernel's shared memory does not hold
+    gives smaller tiles, not an error."""
+    p = mesh.channel(25, 13, 8, seed=3, noise=1e-2) if npe == 8 else mesh.cavity(14, seed=3, solver=mesh.SUPG,
+                                                                                 cfl=0.05, noise=1e-2)
+    compare(p, api.FM_FP64, tile_elems=tile_elems, tile_nodes=tile_nodes, threads=256)
