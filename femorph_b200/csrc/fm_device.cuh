@@ -120,6 +120,41 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// The step loop's kernels are launched so that a kernel may start before the one
+// ahead of it is complete (launch_overlapped).  Every thread of such a kernel
+// calls grid_dependency_wait, which returns once the kernel ahead is complete
+// (and so, by that one's own wait, those before it), before it returns or reads
+// anything that a kernel of the loop writes; what placement wrote (tile and
+// interface lists) it reads before.  launch_dependents lets the next kernel
+// start: the tile kernels call it after their elements, so that the interface
+// kernel's launch and list reads run beside the last tiles' node updates.  At
+// the tile kernel's start it cost more than it gave (its CTAs took the places of
+// tiles: 96^3 504 instead of 500 us), and the interface kernels do not call it:
+// the next step's tiles would be spread over the SMs that they leave free
+// (24^3 mixed 21.8 instead of 20.0).  Without any of it the launches' gaps show:
+// 8^3 20.5 -> 15.3, 16^3 20.5 -> 16.7, 24^3 mixed 24.6 -> 19.6, 60^3 mixed 126 ->
+// 120.5, 96^3 504.5 -> 496.8 us an iteration.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches k so that it may start before the kernel ahead of it in the stream
+// is complete (after its CTAs have all started and called launch_dependents;
+// after completion for one that does not call it).
+template <typename... A>
+cudaError_t launch_overlapped(void (*k)(A...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 // Named barrier `id` of two warps: the first waits for the second's arrival
 // and then sees what it wrote to shared memory before.
 // (An id known at compile time: a kernel that computes it reserves all 16.)

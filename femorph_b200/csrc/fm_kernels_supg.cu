@@ -93,6 +93,11 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
 
   const TileMeta tm = B.tiles[blockIdx.x];
   const int pidx = tm.problem;
+  if constexpr (MIXED) {
+    fill_shape_table<NPE, double>(&s_shape);
+    fill_shape_table<NPE, float>(&s_shape_f);
+  }
+  grid_dependency_wait();
   if (pidx < 0) return;  // free tile slot
   const DevProbState st = B.pstate[pidx];
   if (st.iter >= B.target[pidx] || st.status != FM_OK) return;
@@ -110,10 +115,6 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
     s_u[ln] = u; s_v[ln] = v; s_w[ln] = w;
 #pragma unroll
     for (int q = 0; q < 3 * SETS; ++q) s_acc[q * tn_max + ln] = 0.0;
-  }
-  if constexpr (MIXED) {
-    fill_shape_table<NPE, double>(&s_shape);
-    fill_shape_table<NPE, float>(&s_shape_f);
   }
   __syncthreads();
   const int64_t E = B.E;
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
       pair_arrive<WARPS>(1 + ring * RING + (place + 1) % RING);
   }
   __syncthreads();
+  launch_dependents();
   int32_t status = FM_OK;
   double max_u2 = 0.0;
   for (int l2 = tid; l2 < tm.n_node; l2 += THREADS) {
@@ -350,11 +352,19 @@ __global__ void supg_geo_kernel(DevBatch B, int tile0) {
 }
 
 __global__ void supg_iface_kernel(DevBatch B) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B.n_iface; i += gridDim.x * blockDim.x) {
-    // entry fields load together with the problem id (see vms_iface_kernel)
-    const int pidx = B.iface_prob[i];
-    const int g = B.iface_node[i];
-    const int k0 = B.iface_slot_beg[i], k1 = k0 + B.iface_slot_cnt[i];
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // entry fields load together with the problem id (see vms_iface_kernel)
+  int pidx = -1, g = 0, k0 = 0, k1 = 0;
+  auto entry = [&]() {
+    pidx = B.iface_prob[i];
+    g = B.iface_node[i];
+    k0 = B.iface_slot_beg[i];
+    k1 = k0 + B.iface_slot_cnt[i];
+  };
+  if (i < B.n_iface) entry();
+  grid_dependency_wait();
+  for (bool first = true; i < B.n_iface; i += gridDim.x * blockDim.x, first = false) {
+    if (!first) entry();
     if (pidx < 0) continue;  // free interface entry
     // partials loaded before the state check (see vms_iface_kernel); the
     // fourth component is not used
@@ -526,14 +536,16 @@ cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int threads, int ifa
   const size_t smem = supg_smem_bytes(tn_max, npe, threads, mixed);
   if (ev) cudaEventRecord(ev[0], s);
   auto k = npe == 4 ? supg_tile<4>(mixed, threads, B.sdus != nullptr) : supg_tile<8>(mixed, threads, B.sdus != nullptr);
-  k<<<B.n_tiles, threads == 256 ? 256 : 128, smem, s>>>(B, tn_max);
+  cudaError_t e = launch_overlapped(k, B.n_tiles, threads == 256 ? 256 : 128, smem, s, B, tn_max);
+  if (e != cudaSuccess) return e;
   if (ev) cudaEventRecord(ev[1], s);
   if (xpack)
     supg_xpack_kernel<<<iface_blocks, 256, 0, s>>>(B);
   else
-    supg_iface_kernel<<<iface_blocks, 256, 0, s>>>(B);
+    e = launch_overlapped(supg_iface_kernel, iface_blocks, 256, (size_t)0, s, B);
   if (ev) cudaEventRecord(ev[2], s);
-  return cudaGetLastError();
+  const cudaError_t le = cudaGetLastError();
+  return e != cudaSuccess ? e : le;
 }
 
 cudaError_t launch_supg_geo(const DevBatch& B, int tile0, int ntiles, int tn_max, cudaStream_t s) {

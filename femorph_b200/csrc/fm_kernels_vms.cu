@@ -252,7 +252,6 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
 
   const TileMeta tm = B.tiles[blockIdx.x];
   const int pidx = tm.problem;
-  if (pidx < 0) return;  // free tile slot
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // this thread's staged nodes: their ids are loaded before the problem
   // state is checked, so both round trips overlap
@@ -263,6 +262,8 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
     const int ln = tid + j * THREADS;
     gid[j] = ln < tm.n_node ? B.tile_nodes[tm.node_begin + ln] : -1;
   }
+  grid_dependency_wait();
+  if (pidx < 0) return;  // free tile slot
   const DevProbState st = B.pstate[pidx];
   if (st.iter >= B.target[pidx] || st.status != FM_OK) return;
   const DevProb& P = B.probs[pidx];
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
     }
     return;
   }
+  launch_dependents();  // here, not at the start: see launch_overlapped
   int32_t status = FM_OK;
   const VmsConsts PC = vms_consts(P);
 #pragma unroll
@@ -495,12 +497,20 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
 }
 
 __global__ void vms_iface_kernel(DevBatch B) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B.n_iface; i += gridDim.x * blockDim.x) {
-    // the entry's fields load together with its problem id (a free entry's
-    // are read but not used), so they do not wait for the state check
-    const int pidx = B.iface_prob[i];
-    const int g = B.iface_node[i];
-    const int k0 = B.iface_slot_beg[i], k1 = k0 + B.iface_slot_cnt[i];
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // the entry's fields load together with its problem id (a free entry's
+  // are read but not used), so they do not wait for the state check
+  int pidx = -1, g = 0, k0 = 0, k1 = 0;
+  auto entry = [&]() {
+    pidx = B.iface_prob[i];
+    g = B.iface_node[i];
+    k0 = B.iface_slot_beg[i];
+    k1 = k0 + B.iface_slot_cnt[i];
+  };
+  if (i < B.n_iface) entry();
+  grid_dependency_wait();
+  for (bool first = true; i < B.n_iface; i += gridDim.x * blockDim.x, first = false) {
+    if (!first) entry();
     if (pidx < 0) continue;  // free interface entry
     // the partials are loaded before the state check (an active entry's
     // slots are valid whatever the problem's state)
@@ -694,21 +704,24 @@ cudaError_t launch_vms_iteration(const DevBatch& B, int tn_max, int threads, int
   if (ctas <= 0) ctas = vms_default_ctas(threads, mixed);
   if (ev) cudaEventRecord(ev[0], s);
   bool launched = false;
+  cudaError_t e = cudaSuccess;
 #define FM_VMS_LAUNCH(T, M, C)                                                       \
   if (!launched && threads == T && mixed == M && ctas == C) {                        \
-    vms_tile_kernel<T, M, C><<<B.n_tiles, T, smem, s>>>(B, tn_max);         \
+    e = launch_overlapped(vms_tile_kernel<T, M, C>, B.n_tiles, T, smem, s, B, tn_max); \
     launched = true;                                                                 \
   }
   FM_VMS_VARIANTS(FM_VMS_LAUNCH)
 #undef FM_VMS_LAUNCH
   if (!launched) return cudaErrorInvalidValue;
+  if (e != cudaSuccess) return e;
   if (ev) cudaEventRecord(ev[1], s);
   if (xpack)
     vms_xpack_kernel<<<iface_blocks, 256, 0, s>>>(B);
   else
-    vms_iface_kernel<<<iface_blocks, 256, 0, s>>>(B);
+    e = launch_overlapped(vms_iface_kernel, iface_blocks, 256, (size_t)0, s, B);
   if (ev) cudaEventRecord(ev[2], s);
-  return cudaGetLastError();
+  const cudaError_t le = cudaGetLastError();
+  return e != cudaSuccess ? e : le;
 }
 
 cudaError_t launch_vms_xupdate(const DevBatch& B, int blocks, cudaStream_t s) {
