@@ -295,15 +295,42 @@ __device__ __forceinline__ void apply_bc(const DevBatch& B, int32_t rec, double 
   }
 }
 
+// What placement wrote of an interface entry: an interface kernel's first
+// entry is loaded before it waits for the tile kernel (a free entry's fields
+// are read too, but not used), so that the partials and the state are the only
+// round trip behind the wait: an iteration of 1.05 M hexa8 353 -> 348 us, of 48^3
+// VMS cells 71.5 -> 70.9, of 20^3 SUPG tets 18.5 -> 17.9.  One block a 256 entries
+// instead of at most eight an SM gave nothing more (96^3 493 -> 495.5).
+struct IfaceEntry {
+  int pidx, g, k0, k1;
+  int slot[4];  // the first slots (the first one again past k1)
+  int32_t rec;
+  double m;
+  __device__ __forceinline__ void load(const DevBatch& B, int i) {
+    pidx = B.iface_prob[i];
+    g = B.iface_node[i];
+    k0 = B.iface_slot_beg[i];
+    k1 = k0 + B.iface_slot_cnt[i];
+    if (pidx < 0) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) slot[q] = B.iface_slots[k0 + q < k1 ? k0 + q : k0];
+    rec = B.node_bc[g];
+    m = B.mass[g];
+  }
+};
+
 // Adds the tile partials of interface slots [k0, k1) to acc in slot (tile)
 // order.  The slot ids, and then the partials, are loaded four at a time
 // (past k1 the first id is loaded again and not added), so that their round
-// trips overlap instead of following one another slot by slot.
-__device__ __forceinline__ void sum_partials(const DevBatch& B, int k0, int k1, double acc[4]) {
+// trips overlap instead of following one another slot by slot.  first: the
+// first four ids, already loaded (or null).
+__device__ __forceinline__ void sum_partials(const DevBatch& B, int k0, int k1, double acc[4],
+                                             const int* first = nullptr) {
   for (int k = k0; k < k1; k += 4) {
     int s[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) s[i] = B.iface_slots[k + i < k1 ? k + i : k];
+    for (int i = 0; i < 4; ++i)
+      s[i] = first && k == k0 ? first[i] : B.iface_slots[k + i < k1 ? k + i : k];
     double2 q[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {

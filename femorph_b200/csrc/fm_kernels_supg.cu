@@ -28,11 +28,10 @@ __device__ __forceinline__ void mask_fixed(int gf, double& u, double& v, double&
 }
 
 __device__ __forceinline__ void supg_node_update(const DevBatch& B, const DevProb& P, double time, int64_t g,
-                                                 const double old[3], const double acc[3], int32_t* status,
-                                                 double* max_u2) {
-  const double im = 1.0 / B.mass[g];
+                                                 int32_t rec, double m, const double old[3], const double acc[3],
+                                                 int32_t* status, double* max_u2) {
+  const double im = 1.0 / m;
   double s[4] = {old[0] + im * acc[0], old[1] + im * acc[1], old[2] + im * acc[2], 0.0};
-  const int32_t rec = B.node_bc[g];
   if (rec >= 0) apply_bc(B, rec, time, s, status);
   B.su[g] = s[0];
   B.sv[g] = s[1];
@@ -290,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED &
     if (l2 < tm.n_int) {
       const int g = B.tile_nodes[tm.node_begin + l2];
       const double old[3] = {s_u[l2], s_v[l2], s_w[l2]};
-      supg_node_update(B, P, st.time, g, old, acc, &status, &max_u2);
+      supg_node_update(B, P, st.time, g, B.node_bc[g], B.mass[g], old, acc, &status, &max_u2);
     } else {
       const int s = tm.slot_base + (l2 - tm.n_int);
       B.part[2 * s] = make_double2(acc[0], acc[1]);
@@ -351,33 +350,27 @@ __global__ void supg_geo_kernel(DevBatch B, int tile0) {
   }
 }
 
-__global__ void supg_iface_kernel(DevBatch B) {
+__global__ void __launch_bounds__(256, 4) supg_iface_kernel(DevBatch B) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  // entry fields load together with the problem id (see vms_iface_kernel)
-  int pidx = -1, g = 0, k0 = 0, k1 = 0;
-  auto entry = [&]() {
-    pidx = B.iface_prob[i];
-    g = B.iface_node[i];
-    k0 = B.iface_slot_beg[i];
-    k1 = k0 + B.iface_slot_cnt[i];
-  };
-  if (i < B.n_iface) entry();
+  IfaceEntry en;
+  if (i < B.n_iface) en.load(B, i);
   grid_dependency_wait();
   for (bool first = true; i < B.n_iface; i += gridDim.x * blockDim.x, first = false) {
-    if (!first) entry();
-    if (pidx < 0) continue;  // free interface entry
-    // partials loaded before the state check (see vms_iface_kernel); the
-    // fourth component is not used
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    sum_partials(B, k0, k1, acc);
+    if (!first) en.load(B, i);
+    if (en.pidx < 0) continue;  // free interface entry
+    const int pidx = en.pidx, g = en.g;
+    // state and partials loaded before the state check (see vms_iface_kernel);
+    // the fourth component is not used
+    double old[3] = {B.su[g], B.sv[g], B.sw[g]};
     const DevProbState st = B.pstate[pidx];
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    sum_partials(B, en.k0, en.k1, acc, en.slot);
     if (st.iter >= B.target[pidx] || st.status != FM_OK) continue;
     const DevProb& P = B.probs[pidx];
-    double old[3] = {B.su[g], B.sv[g], B.sw[g]};
     mask_fixed(P.glob_fixed, old[0], old[1], old[2]);
     int32_t status = FM_OK;
     double max_u2 = 0.0;
-    supg_node_update(B, P, st.time, g, old, acc, &status, &max_u2);
+    supg_node_update(B, P, st.time, g, en.rec, en.m, old, acc, &status, &max_u2);
     check_exit(B, P, pidx, max_u2, status);
   }
   finish_iteration(B);
@@ -405,7 +398,7 @@ __global__ void supg_xpack_kernel(DevBatch B) {
     mask_fixed(P.glob_fixed, old[0], old[1], old[2]);
     int32_t status = FM_OK;
     double max_u2 = 0.0;
-    supg_node_update(B, P, st.time, g, old, acc, &status, &max_u2);
+    supg_node_update(B, P, st.time, g, B.node_bc[g], B.mass[g], old, acc, &status, &max_u2);
     check_exit(B, P, pidx, max_u2, status);
   }
 }
@@ -425,7 +418,7 @@ __global__ void supg_xupdate_kernel(DevBatch B) {
     mask_fixed(P.glob_fixed, old[0], old[1], old[2]);
     int32_t status = FM_OK;
     double max_u2 = 0.0;
-    supg_node_update(B, P, st.time, g, old, acc, &status, &max_u2);
+    supg_node_update(B, P, st.time, g, B.node_bc[g], B.mass[g], old, acc, &status, &max_u2);
     check_exit(B, P, pidx, max_u2, status);
   }
   finish_iteration(B);

@@ -52,16 +52,14 @@ __device__ __forceinline__ VmsConsts vms_consts(const DevProb& P) {
 
 template <class PROB>  // DevProb or VmsConsts: reads ds and q1[]
 __device__ __forceinline__ void vms_node_update(const DevBatch& B, const PROB& P, int pidx, int iter, double time,
-                                                int64_t g, const double post[4], const double acc[4], bool first_dual,
-                                                int32_t* status) {
-  const int32_t rec = B.node_bc[g];
+                                                int64_t g, int32_t rec, double m, const double post[4],
+                                                const double acc[4], bool first_dual, int32_t* status) {
   double s[4];
   if (!first_dual && rec >= 0) {
     s[0] = B.pu[g]; s[1] = B.pv[g]; s[2] = B.pw[g]; s[3] = B.pp[g];
   } else {
     s[0] = post[0]; s[1] = post[1]; s[2] = post[2]; s[3] = post[3];
   }
-  const double m = B.mass[g];
 #pragma unroll
   for (int d = 0; d < 4; ++d) s[d] = __dsub_rn(s[d], __ddiv_rn(__dmul_rn(P.ds, acc[d]), m));
   if (!(isfinite(s[0]) && isfinite(s[1]) && isfinite(s[2]) && isfinite(s[3]))) *status = FM_ERR_DIVERGED;
@@ -486,7 +484,7 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
       const double2 r1 = s_rec[rec_index(ln2, 1)], r2 = s_rec[rec_index(ln2, 2)], r3 = s_rec[rec_index(ln2, 3)];
       const int g = (int)(__double_as_longlong(r3.y) & 0x7fffffffll);
       const double post[4] = {r1.y, r2.x, r2.y, r3.x};
-      vms_node_update(B, PC, pidx, st.iter, st.time, g, post, acc, first_dual, &status);
+      vms_node_update(B, PC, pidx, st.iter, st.time, g, B.node_bc[g], B.mass[g], post, acc, first_dual, &status);
     } else {
       const int s = tm.slot_base + (ln2 - tm.n_int);
       B.part[2 * s] = a0;
@@ -496,33 +494,26 @@ __global__ void __launch_bounds__(THREADS, MINB) vms_tile_kernel(DevBatch B, int
   if (status != FM_OK) B.pstate[pidx].status = status;
 }
 
-__global__ void vms_iface_kernel(DevBatch B) {
+__global__ void __launch_bounds__(256, 4) vms_iface_kernel(DevBatch B) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  // the entry's fields load together with its problem id (a free entry's
-  // are read but not used), so they do not wait for the state check
-  int pidx = -1, g = 0, k0 = 0, k1 = 0;
-  auto entry = [&]() {
-    pidx = B.iface_prob[i];
-    g = B.iface_node[i];
-    k0 = B.iface_slot_beg[i];
-    k1 = k0 + B.iface_slot_cnt[i];
-  };
-  if (i < B.n_iface) entry();
+  IfaceEntry en;
+  if (i < B.n_iface) en.load(B, i);
   grid_dependency_wait();
   for (bool first = true; i < B.n_iface; i += gridDim.x * blockDim.x, first = false) {
-    if (!first) entry();
-    if (pidx < 0) continue;  // free interface entry
-    // the partials are loaded before the state check (an active entry's
+    if (!first) en.load(B, i);
+    if (en.pidx < 0) continue;  // free interface entry
+    const int pidx = en.pidx, g = en.g;
+    // state and partials are loaded before the state check (an active entry's
     // slots are valid whatever the problem's state)
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    sum_partials(B, k0, k1, acc);
+    const double post[4] = {B.su[g], B.sv[g], B.sw[g], B.sp[g]};
     const DevProbState st = B.pstate[pidx];
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    sum_partials(B, en.k0, en.k1, acc, en.slot);
     if (st.iter >= B.target[pidx] || st.status != FM_OK) continue;
     const DevProb& P = B.probs[pidx];
     const bool first_dual = (st.iter % (P.ndual + 1)) == 0;
-    const double post[4] = {B.su[g], B.sv[g], B.sw[g], B.sp[g]};
     int32_t status = FM_OK;
-    vms_node_update(B, P, pidx, st.iter, st.time, g, post, acc, first_dual, &status);
+    vms_node_update(B, P, pidx, st.iter, st.time, g, en.rec, en.m, post, acc, first_dual, &status);
     if (status != FM_OK) B.pstate[pidx].status = status;
   }
   finish_iteration(B);
@@ -550,7 +541,7 @@ __global__ void vms_xpack_kernel(DevBatch B) {
     const int g = B.iface_node[i];
     const double post[4] = {B.su[g], B.sv[g], B.sw[g], B.sp[g]};
     int32_t status = FM_OK;
-    vms_node_update(B, P, pidx, st.iter, st.time, g, post, acc, first_dual, &status);
+    vms_node_update(B, P, pidx, st.iter, st.time, g, B.node_bc[g], B.mass[g], post, acc, first_dual, &status);
     if (status != FM_OK) B.pstate[pidx].status = status;
   }
 }
@@ -571,7 +562,7 @@ __global__ void vms_xupdate_kernel(DevBatch B) {
     const int g = B.iface_node[i];
     const double post[4] = {B.su[g], B.sv[g], B.sw[g], B.sp[g]};
     int32_t status = FM_OK;
-    vms_node_update(B, P, pidx, st.iter, st.time, g, post, acc, first_dual, &status);
+    vms_node_update(B, P, pidx, st.iter, st.time, g, B.node_bc[g], B.mass[g], post, acc, first_dual, &status);
     if (status != FM_OK) B.pstate[pidx].status = status;
   }
   finish_iteration(B);
