@@ -509,6 +509,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
   for (int pi = 0; pi < n; ++pi) {
     fm_problem* p = probs[pi];
     const int npe = p->etype;
+    const bool vms = p->params.solver == FM_SOLVER_VMS;
     const int64_t E = p->E, N = p->N;
     L.node_begin.push_back(node_base);
     L.elem_begin.push_back(elem_base);
@@ -655,9 +656,14 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             // many colours) spreads its elements over as many colours as it
             // has warps, always to the emptiest one that fits: 36 colour runs
             // in the 32 warps of a 1024-tet tile, against 60 of the smallest
-            // colour that fits
+            // colour that fits.
+            // (SUPG mixed: the smallest colour that fits, whatever its size, in
+            // order.  Its FP32 element work turns the last bit of a nodal sum
+            // into an FP32 rounding now and then, which travels to the pressure
+            // as 1e-8 of it: the sums keep this one order.)
+            const bool ordered = !vms && p->params.precision == FM_MIXED;
             const int nwarp = (int)((ne + 31) / 32);
-            const int even = nwarp >= (npe == 4 ? 26 : 10) && nwarp <= 64 ? nwarp : 0;
+            const int even = !ordered && nwarp >= (npe == 4 ? 26 : 10) && nwarp <= 64 ? nwarp : 0;
             uint64_t level[33] = {0};  // colours below `even` by their size
             level[0] = even == 64 ? ~0ULL : (1ULL << even) - 1;
             int csize[128] = {0};
@@ -694,13 +700,13 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
                   break;
                 }
               }
-              if (++csize[k] >= 32) (k < 64 ? full0 : full1) |= 1ULL << (k & 63);
+              if (++csize[k] >= 32 && !ordered) (k < 64 ? full0 : full1) |= 1ULL << (k & 63);
               col[i] = k;
               ncol = std::max(ncol, k + 1);
               for (int a = 0; a < npe; ++a) used[2 * local[c[a]] + (k >> 6)] |= (1ULL << (k & 63));
             }
             if (W.err) continue;
-            {
+            if (!ordered) {
               // the largest colours first: they fill whole warps
               int by[128], at[128], n = 0;
               for (int k = 0; k < ncol; ++k)

@@ -62,12 +62,13 @@ __device__ __forceinline__ void check_exit(const DevBatch& B, const DevProb& P, 
 //
 // Accumulation of the element contributions into the tile's nodes: in turn, as
 // in vms_tile_kernel (rings of warps, colour run by colour run), in an order
-// fixed by the tile.  tet4 has two rings; hexa8 one of four warps, for want of
-// shared memory.  Before, every thread staged its contributions and the
+// fixed by the tile.  FP64 tet4 has two rings; hexa8 one of four warps, for want
+// of shared memory, and mixed tet4 one, so that its sums keep the tile's element
+// order (build_layout).  Before, every thread staged its contributions and the
 // node's owner thread walked a list of its corners between two barriers a
 // chunk (tet4), or colours followed each other with a barrier each (hexa8):
-// 145 against 117 us a step on 1.57 M tets FP64, 135 against 111 mixed, and
-// 372 against 339 on 1.05 M hexa8 FP64, 330 against 295 mixed.
+// 145 against 117 us a step on 1.57 M tets FP64, 135 against 116 mixed, and
+// 372 against 339 on 1.05 M hexa8 FP64, 330 against 297 mixed.
 //
 // The hexa8 kernels (GEO) read each Gauss point's inverse Jacobian and det J
 // from the geometry stored at placement (supg_geo_kernel; FP64, or rounded
@@ -76,7 +77,7 @@ __device__ __forceinline__ void check_exit(const DevBatch& B, const DevProb& P, 
 template <int NPE, int THREADS, bool MIXED, bool HISTORY>
 __global__ void __launch_bounds__(THREADS, THREADS == 128 ? (NPE == 4 && MIXED && !HISTORY ? 4 : 3) : 1)
     supg_tile_kernel(DevBatch B, int tn_max) {
-  constexpr int WARPS = THREADS / 32, SETS = supg_acc_sets(NPE), RING = WARPS / SETS;
+  constexpr int WARPS = THREADS / 32, SETS = supg_acc_sets(NPE, MIXED), RING = WARPS / SETS;
   constexpr bool GEO = NPE == 8;
   extern __shared__ double sm[];
   double* s_x = sm;  // coordinates: tet4 only
@@ -467,7 +468,7 @@ __global__ void supg_pressure_kernel(DevBatch B, int tn_max, double* pres) {
 }
 
 size_t supg_smem_bytes(int tn_max, int npe, int threads, bool mixed) {
-  return ((size_t)tn_max * ((npe == 4 ? 6 : 3) + 3 * supg_acc_sets(npe)) + supg_stage_doubles(npe, mixed, threads)) *
+  return ((size_t)tn_max * ((npe == 4 ? 6 : 3) + 3 * supg_acc_sets(npe, mixed)) + supg_stage_doubles(npe, mixed, threads)) *
          sizeof(double);
 }
 

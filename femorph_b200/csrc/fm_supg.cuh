@@ -221,7 +221,7 @@ __host__ __device__ constexpr size_t supg_stage_doubles(int npe, bool mixed, int
                   : (size_t)threads * (mixed ? FM_GEO_ROWS32 * FM_GEO_PER_GP / 2 : 24 + FM_GEO_ROWS64 * FM_GEO_PER_GP);
 }
 // Sets of accumulators (rings of warps).
-__host__ __device__ constexpr int supg_acc_sets(int npe) { return npe == 4 ? 2 : 1; }
+__host__ __device__ constexpr int supg_acc_sets(int npe, bool mixed) { return npe == 4 && !mixed ? 2 : 1; }
 
 // Inverse (cofactors, femUtils.cpp:716-770) and determinant of a 3x3 matrix.
 __device__ __forceinline__ double inverse3(const double J[3][3], double inv[3][3]) {
