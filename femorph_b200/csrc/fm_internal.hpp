@@ -120,7 +120,7 @@ struct TileMeta {
   int32_t slot_base;            // partial slot of local node n_int
   int32_t col_begin, n_col;     // colour offsets in the layout's tile_cols[col_begin .. +n_col] (host)
   int32_t problem;
-  int32_t node0;                // batch id of local node 0 when the interior nodes are
+  int32_t node0;                // lowest batch id of the interior nodes when they are
                                 // consecutive batch ids from it (-1 otherwise); set at placement
 };
 

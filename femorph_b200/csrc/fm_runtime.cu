@@ -770,13 +770,14 @@ static int place(fm_batch* b, fm_problem* p, const std::shared_ptr<Layout>& Lp) 
       tm.node_begin += (int32_t)pl.off[P_TNODE];
       tm.slot_base += (int32_t)soff;
       // the look-ahead prefetch reads node0 .. node0 + n_int - 1: checked to
-      // be the tile's interior nodes (consecutive by construction), else -1
+      // be the tile's interior nodes (consecutive ids by construction, in any
+      // order), else -1
       // (no node prefetch for the tile)
       {
         const int32_t* tn = L.tile_nodes.data() + (tm.node_begin - (int32_t)pl.off[P_TNODE]);
-        bool consecutive = tm.n_int > 0;
-        for (int32_t j = 1; j < tm.n_int && consecutive; ++j) consecutive = tn[j] == tn[0] + j;
-        tm.node0 = consecutive ? tn[0] + (int32_t)noff : -1;
+        int32_t first = tm.n_int > 0 ? tn[0] : 0, last = first;
+        for (int32_t j = 1; j < tm.n_int; ++j) first = std::min(first, tn[j]), last = std::max(last, tn[j]);
+        tm.node0 = tm.n_int > 0 && last - first == tm.n_int - 1 ? first + (int32_t)noff : -1;
       }
       tm.problem = ps;
       pl.tn_max = std::max(pl.tn_max, tm.n_node);
