@@ -472,8 +472,9 @@ struct fm_poisson {
   // coordinates, the fixed connectivity, the diffusivity rows and the source,
   // Neumann and Dirichlet markers of femModel::ExportToVTKLegacy
   fm::PoissonHostView view{};
-  std::vector<double> h_coords, h_diff, h_src, h_neu, h_dir;
-  std::vector<int32_t> h_conn;
+  fm::hvec<double> h_coords, h_diff, h_src;
+  std::vector<double> h_neu, h_dir;
+  fm::hvec<int32_t> h_conn;
 };
 
 #define PCK(x)                                                                                         \
@@ -498,6 +499,48 @@ FM_API int fm_poisson_destroy(fm_poisson* s) {
   delete s;
   return FM_OK;
 }
+
+// The solver's stream, events and pinned words, made by a thread of their own
+// while the host assembles the system: 2 to 3 ms, as much as the resident
+// kernel's plan adds to it (a small hexa wall distance: 11 to 12.5 ms without the
+// plan, 16 with both in turn, 10.2 to 10.7 now).  What the solver does not take is
+// given back.
+struct PoissonSetup {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  int32_t* h_ctl = nullptr;
+  double* h_scal = nullptr;
+  cudaError_t e = cudaSuccess;
+  std::thread th;
+  explicit PoissonSetup(int device) : th([this, device] { make(device); }) {}
+  void make(int device) {
+    int n = 0;
+    if (cudaGetDeviceCount(&n) != cudaSuccess || device < 0 || device >= n) return;  // the caller's to report
+    e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreate(&ev0);
+    if (e == cudaSuccess) e = cudaEventCreate(&ev1);
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&h_ctl, 8 * sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&h_scal, 8 * sizeof(double));
+  }
+  cudaError_t give(fm_poisson* s) {
+    th.join();
+    std::swap(s->stream, stream);
+    std::swap(s->ev0, ev0);
+    std::swap(s->ev1, ev1);
+    std::swap(s->h_ctl, h_ctl);
+    std::swap(s->h_scal, h_scal);
+    return e;
+  }
+  ~PoissonSetup() {
+    if (th.joinable()) th.join();
+    if (stream) cudaStreamDestroy(stream);
+    if (ev0) cudaEventDestroy(ev0);
+    if (ev1) cudaEventDestroy(ev1);
+    if (h_ctl) cudaFreeHost(h_ctl);
+    if (h_scal) cudaFreeHost(h_scal);
+  }
+};
 
 static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson** out) {
   if (!d || !out) return fail(FM_ERR_INVALID, "null argument");
@@ -531,6 +574,7 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   // an element whose smallest Jacobian determinant over the irSecondOrder
   // points is <= 0 gets one swap, tet4 nodes 0 / 1 (femTetra4.cpp:160-170),
   // hexa8 nodes 2 / 3 and 6 / 7 (femHexa8.cpp:93-103)
+  PoissonSetup setup(device);
   Rule rule;
   make_rule(npe, rule);
   fm::hvec<int32_t> cfix((size_t)(E * npe));
@@ -552,7 +596,7 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
         }
       }
     }
-  }, 4096);
+  }, 1024);
   const int32_t* conn = cfix.data();
   // element matrices, in parallel over elements
   const int m2 = npe * npe;
@@ -624,7 +668,7 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
           for (int q = 0; q < 3; ++q) xe[a][q] = d->coords[3 * (int64_t)conn[e * npe + a] + q];
         element_source(npe, rule, xe, d->source_value[k], &fs[(size_t)k * npe]);
       }
-    }, 4096);
+    }, 1024);
     for (int64_t k = 0; k < d->n_sources; ++k) {
       const int64_t e = d->source_elem[k];
       for (int a = 0; a < npe; ++a) rhs[conn[e * npe + a]] += fs[(size_t)k * npe + a];
@@ -648,7 +692,7 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   std::vector<int32_t> rowp(N + 1, 0);
   fm::hvec<int32_t> rowlen(N);
   std::vector<double> bvec(N), dinv(N);
-  const int64_t nblk = std::min<int64_t>(hwt, std::max<int64_t>(1, N / 2048));
+  const int64_t nblk = std::min<int64_t>(hwt, std::max<int64_t>(1, N / 1024));
   std::vector<std::vector<int32_t>> bcol(nblk);
   std::vector<std::vector<double>> bval(nblk);
   auto rows = [&](int64_t kb) {
@@ -828,10 +872,19 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   // the exporter's fields (femModel.cpp:1400-1500): Dirichlet nodes 1,
   // Neumann face nodes their row's value, source elements their value (a
   // later row wins in each)
-  s->h_coords.assign(d->coords, d->coords + N * 3);
-  s->h_conn.assign(cfix.begin(), cfix.end());
-  s->h_diff.assign(d->diffusivity, d->diffusivity + E * 3);
-  s->h_src.assign(E, 0.0);
+  s->h_conn = std::move(cfix);  // conn stays valid
+  s->h_coords.resize(N * 3);
+  s->h_diff.resize(E * 3);
+  s->h_src.resize(E);
+  // (fresh pages: one thread takes 35 ms for 1.57 M tets; the whole of create
+  // 133 -> 102 ms, 125 before it formed the resident kernel's plan)
+  fm::parallel_blocks(N, [&](int64_t b, int64_t e, int) {
+    std::copy(d->coords + 3 * b, d->coords + 3 * e, s->h_coords.begin() + 3 * b);
+  }, 1 << 15);
+  fm::parallel_blocks(E, [&](int64_t b, int64_t e, int) {
+    std::copy(d->diffusivity + 3 * b, d->diffusivity + 3 * e, s->h_diff.begin() + 3 * b);
+    std::fill(s->h_src.begin() + b, s->h_src.begin() + e, 0.0);
+  }, 1 << 15);
   for (int64_t k = 0; k < d->n_sources; ++k) s->h_src[d->source_elem[k]] = d->source_value[k];
   s->h_neu.assign(N, 0.0);
   for (int64_t k = 0; k < d->n_neumann; ++k)
@@ -902,11 +955,7 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
     fm_poisson_destroy(s);
     return fail(FM_ERR_CUDA, m);
   };
-  cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreate(&s->ev0);
-  if (e == cudaSuccess) e = cudaEventCreate(&s->ev1);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&s->h_ctl, 8 * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&s->h_scal, 8 * sizeof(double));
+  cudaError_t e = setup.give(s);
   if (e != cudaSuccess) return fail_free("stream / event / pinned buffer", e);
   const cudaStream_t st = s->stream;
   auto up = [&](void* dst, const void* src, size_t bytes) {

@@ -367,38 +367,53 @@ void build_resident(const double* coords, int64_t N, const std::vector<int32_t>&
       return q;
     };
     int64_t entries = 0;
+    for (int32_t i = a; i < b; ++i) entries += len(H.node_of[i]);
+    std::vector<uint16_t>& lc = local[g];
+    lc.resize(entries);
+    // halo columns by their first occurrence, then in order
+    uint16_t* out = lc.data();
     for (int32_t i = a; i < b; ++i) {
       const int64_t v = H.node_of[i];
-      if ((i - a) % 32 == 0) width[g].push_back(len(v));
+      const int n = len(v);
+      if ((i - a) % 32 == 0) width[g].push_back(n);
       const int32_t* col = row(v).first;
-      for (int32_t k = 0; k < len(v); ++k) {
+      for (int32_t k = 0; k < n; ++k) {
         const int32_t w = H.row_of[col[k]];
-        if (w >= a && w < b) continue;
-        const uint32_t q = slot(w);
-        if (key[q] >= 0) continue;
-        key[q] = w;
-        h.push_back(w);
-        if (2 * h.size() > mask) {
-          mask = 2 * mask + 1;
-          key.assign(mask + 1, -1);
-          id.resize(mask + 1);
-          for (int32_t u : h) key[slot(u)] = u;
+        if (w >= a && w < b) {
+          *out++ = (uint16_t)(w - a);
+          continue;
         }
+        uint32_t q = slot(w);
+        if (key[q] < 0) {
+          if (b - a + (int64_t)h.size() >= 65536) {  // does not fit (below)
+            h.push_back(w);
+            return;
+          }
+          if (2 * (h.size() + 1) > mask) {
+            mask = 2 * mask + 1;
+            key.assign(mask + 1, -1);
+            id.resize(mask + 1);
+            for (size_t j = 0; j < h.size(); ++j) {
+              const uint32_t r = slot(h[j]);
+              key[r] = h[j];
+              id[r] = (int32_t)j;
+            }
+            q = slot(w);
+          }
+          key[q] = w;
+          id[q] = (int32_t)h.size();
+          h.push_back(w);
+        }
+        *out++ = (uint16_t)(b - a + id[q]);
       }
-      entries += len(v);
     }
-    if (b - a + (int64_t)h.size() > 65536) return;  // does not fit (below)
+    std::vector<uint16_t> rank(h.size());
+    std::vector<int32_t> first(h);
     std::sort(h.begin(), h.end());
-    for (size_t i = 0; i < h.size(); ++i) id[slot(h[i])] = b - a + (int32_t)i;
-    local[g].reserve(entries);
-    for (int32_t i = a; i < b; ++i) {
-      const int64_t v = H.node_of[i];
-      const int32_t* col = row(v).first;
-      for (int32_t k = 0; k < len(v); ++k) {
-        const int32_t w = H.row_of[col[k]];
-        local[g].push_back((uint16_t)(w >= a && w < b ? w - a : id[slot(w)]));
-      }
-    }
+    for (size_t i = 0; i < h.size(); ++i) id[slot(h[i])] = (int32_t)i;
+    for (size_t j = 0; j < first.size(); ++j) rank[j] = (uint16_t)(b - a + id[slot(first[j])]);
+    for (uint16_t& c : lc)
+      if (c >= b - a) c = rank[c - (b - a)];
   });
   H.halo0.assign(G + 1, 0);
   H.slice0.assign(G + 1, 0);

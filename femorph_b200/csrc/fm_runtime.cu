@@ -279,7 +279,7 @@ static int put(T* dev_base, int64_t off, const T* src, int64_t n, cudaStream_t s
 // iteration; 24^3: 256, 24.6 against 41.4; 30^3: 384, 29.4 against 47.3;
 // 36^3: 640, 39.3 (512: 47.6); 44^3: 576, 63.7 against 78.9; 64^3: 896, 160.7
 // against 167.6; mixed 24^3: 256 against 512 24.2 against 28.7; hexa
-// 93x37x29 FP64: 256 against 384 50 against 58.  Not below 256, where a batch of
+// 93x37x29 FP64: 256 against 384 43.8 against 48.1.  Not below 256, where a batch of
 // many small problems would pay for the extra interface nodes (32 cavities of
 // 8..24 cells a side: 256 at least 148.7 us, 128 at least 170.3, full tiles
 // 157.7, measured before the warps took turns).  It depends on the problem
