@@ -134,9 +134,9 @@ def stored_geometry_bytes(E: int, precision: str, config: str) -> int:
 
 # FP64 operations of one SUPG element-step (matrix-free K u over the Gauss
 # points, counting an FMA as two), from the ncu FP64 instruction counts of
-# the tile kernels (profiles/supg_tile_kernel_*.md); the hexa8 count is that
+# the tile kernels (profiles/supg_tile_kernel_fp64_counts.md); the hexa8 count is that
 # of the kernel reading the stored Gauss-point geometry.
-SUPG_FLOPS = {"channel": 6419, "supg": 1676}
+SUPG_FLOPS = {"channel": 3480, "supg": 790}
 
 CONFIG_DEFAULT_N = {"cavity": 96, "supg": 96, "channel": 64, "io": 96}
 
