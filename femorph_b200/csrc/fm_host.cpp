@@ -495,7 +495,8 @@ void morton_order(const fm_problem* p, hvec<int64_t>& order) {
 //     interior nodes contiguous), interface nodes after them;
 //  4. inside a tile, elements are coloured greedily (no two elements of a
 //     colour share a node) and sorted by colour, which fixes the order in
-//     which contributions reach every node;
+//     which contributions reach every node; the order of the interior nodes
+//     and of the interface nodes is chosen for the shared-memory banks;
 //  5. each (tile, interface node) pair gets a partial-sum slot; the slots of
 //     an interface node are listed in tile order.
 // Nodes of a partition part that are shared with other parts (p->xidx >= 0)
@@ -635,7 +636,8 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
               }
             }
             // interior nodes in their (contiguous) batch order, then interface
-            // nodes by id.  The interior nodes and those this tile touches first
+            // nodes by id (reordered for the shared-memory banks below).  The
+            // interior nodes and the interface nodes this tile touches first
             // were numbered in this same first-touch walk, so they arrive in
             // id order; only the interface nodes of earlier tiles (all with
             // smaller ids) are sorted
@@ -792,7 +794,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             // element of a colour (the tile kernel's warps add up one colour
             // after another)
             for (int k = 0; k < ncol; ++k)
-                if (W.colcnt[k] < ne) W.conn[(size_t)W.colcnt[k] * npe + 1] |= 0x8000;
+              if (W.colcnt[k] < ne) W.conn[(size_t)W.colcnt[k] * npe + 1] |= 0x8000;
             // and of a hexa's third one that its corners repeat a node (a
             // collapsed hexa), so that they are added one by one
             if (npe == 8)
