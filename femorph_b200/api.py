@@ -36,7 +36,7 @@ SYMBOLS = [
     "fm_batch_exchange_end", "fm_batch_iterations_per_step", "fm_problem_checkpoint", "fm_problem_restore",
     "fm_batch_set_diagnostics", "fm_problem_vms_log", "fm_problem_vms_residuals",
     "fm_poisson_create", "fm_poisson_destroy", "fm_poisson_solve", "fm_poisson_get_solution", "fm_poisson_info", "fm_poisson_model",
-    "fm_poisson_read_dat", "fm_poisson_write_vtk", "fm_problem_check_layout",
+    "fm_poisson_read_dat", "fm_poisson_write_vtk", "fm_problem_check_layout", "fm_poisson_set_wait_limit",
 ]
 
 FM_POISSON_CLASSIC, FM_POISSON_PPE, FM_POISSON_DISTANCE = 0, 1, 2
@@ -149,6 +149,7 @@ def lib():
         L.fm_poisson_create.argtypes = [P, C.c_int32, P]
         L.fm_poisson_destroy.argtypes = [P]
         L.fm_poisson_solve.argtypes = [P, C.c_double, C.c_int32, P, P, P]
+        L.fm_poisson_set_wait_limit.argtypes = [P, C.c_uint32]
         L.fm_poisson_get_solution.argtypes = [P, P, P]
         L.fm_poisson_info.argtypes = [P, P, P]
         L.fm_poisson_model.argtypes = [P, P, P, P, P]
@@ -552,6 +553,10 @@ class GpuPoisson:
         it, rr, ms = C.c_int32(), C.c_double(), C.c_double()
         check(lib().fm_poisson_solve(self.h, float(rel_tol), int(max_iter), C.byref(it), C.byref(rr), C.byref(ms)))
         return int(it.value), float(rr.value), float(ms.value)
+
+    def set_wait_limit(self, polls: int) -> None:
+        """Polls of the resident solver's bounded waits before FM_ERR_TIMEOUT."""
+        check(lib().fm_poisson_set_wait_limit(self.h, int(polls)))
 
     @classmethod
     def read_dat(cls, path: str, device: int = 0):

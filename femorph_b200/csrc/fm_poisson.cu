@@ -939,6 +939,7 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   s->dist = reinterpret_cast<double*>(base + o_dist);
   if (H.fits) {
     s->R = H.R;
+    s->R.polls = kResPolls;
     s->row_of = reinterpret_cast<int32_t*>(base + o_row_of);
     s->R.row0 = reinterpret_cast<int32_t*>(base + o_row0);
     s->R.halo0 = reinterpret_cast<int32_t*>(base + o_halo0);
@@ -1023,6 +1024,7 @@ FM_API int fm_poisson_solve(fm_poisson* s, double rel_tol, int32_t max_iter, int
   const cudaStream_t st = s->stream;
   const Cg& c = s->c;
   const int G = s->blocks;
+  s->has_result = false;  // this solve writes over an earlier one's
   // stopping test r.r <= tol^2 b.b (scal[5] = b.b, scal[6] = the threshold)
   const int32_t ctl_init[8] = {0, 0, 0, max_iter, 0, 0, 0, 0};
   const double sc[2] = {s->bb, rel_tol * rel_tol * s->bb};
@@ -1072,21 +1074,29 @@ FM_API int fm_poisson_solve(fm_poisson* s, double rel_tol, int32_t max_iter, int
   PCK(cudaMemcpyAsync(s->h_ctl, c.ctl, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   PCK(cudaMemcpyAsync(s->h_scal, c.scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
   PCK(cudaStreamSynchronize(st));
+  // blocks that gave up stopped in different places: neither a result nor a
+  // count or residual of one
+  if (s->h_ctl[2] == 2) return fail(FM_ERR_TIMEOUT, "CG: an exchange between the resident blocks did not complete");
   float ms = 0.0f;
   PCK(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
   if (device_ms) *device_ms = ms;
   if (iterations) *iterations = s->h_ctl[1];
   const double bb = s->bb;
   if (rel_residual) *rel_residual = bb > 0.0 ? std::sqrt(s->h_scal[4] / bb) : 0.0;
-  if (s->h_ctl[2] == 2) return fail(FM_ERR_TIMEOUT, "CG: an exchange between the resident blocks did not complete");
   s->has_result = true;
   if (s->h_ctl[2]) return fail(FM_ERR_DIVERGED, "CG breakdown (matrix not positive definite on the search direction, or NaN)");
   return FM_OK;
 }
 
+FM_API int fm_poisson_set_wait_limit(fm_poisson* s, uint32_t polls) {
+  if (!s) return fail(FM_ERR_INVALID, "null solver");
+  s->R.polls = polls;
+  return FM_OK;
+}
+
 FM_API int fm_poisson_get_solution(fm_poisson* s, double* x, double* cell_distance) {
   if (!s) return fail(FM_ERR_INVALID, "null solver");
-  if (!s->has_result) return fail(FM_ERR_INVALID, "fm_poisson_solve has not run");
+  if (!s->has_result) return fail(FM_ERR_INVALID, "no solution: fm_poisson_solve has not run, or gave none");
   if (cell_distance && s->problem != FM_POISSON_DISTANCE)
     return fail(FM_ERR_INVALID, "cell distances exist for FM_POISSON_DISTANCE only");
   DeviceRestore restore;

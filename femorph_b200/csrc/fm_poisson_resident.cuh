@@ -23,8 +23,8 @@
 // of lines that are being written).  The table is double buffered: a CTA that
 // writes for exchange k + 2 has seen all arrive at k + 1, hence all have read
 // k.  The launch is cooperative (all CTAs are resident), the poll loop is
-// bounded, and a CTA that gives up returns with a time-out in the control
-// word.
+// bounded (CgResident::polls), and a CTA that gives up returns with a time-out
+// in the control word, which no other CTA's verdict replaces.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -42,7 +42,7 @@ constexpr int kResWide = 1024;
 // Loads a thread has in flight: matrix entries, and rows of the vector loops.
 constexpr int res_batch(int threads) { return threads == 1024 ? 8 : 16; }
 constexpr int kResRowsAhead = 4;
-constexpr uint32_t kResPolls = 1u << 22;  // a few seconds
+constexpr uint32_t kResPolls = 1u << 22;  // default limit of an exchange's wait: a few seconds
 
 // Device view.  CTA c owns rows row0[c] .. row0[c+1] of the reordered system.
 // Its local columns: first its own rows, then halo[halo0[c] ..] (row numbers).
@@ -58,6 +58,7 @@ struct CgResident {
   const uint16_t* col;
   double2* partials;   // [2][ctas]
   unsigned long long* arrived;
+  uint32_t polls;                         // an exchange's wait gives up after this many (kResPolls)
   size_t smem;
 };
 
@@ -106,11 +107,9 @@ __device__ __forceinline__ bool grid_wait(const CgResident& R, uint64_t number, 
   if (warp == 0 && R.ctas > 1) {
     if (lane == 0) {
       const uint64_t all = number * (uint64_t)R.ctas;
-      uint64_t n;
-      uint32_t polls = 0;
-      do {
+      uint64_t n = 0;
+      for (uint32_t polls = 0; n < all && polls < R.polls; ++polls)
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(n) : "l"(R.arrived) : "memory");
-      } while (n < all && ++polls < kResPolls);
       if (n < all) *failed = 1;
     }
     __syncwarp();
@@ -298,7 +297,7 @@ __global__ void __launch_bounds__(THREADS, 1) cg_resident_kernel(Cg c, CgResiden
     c.scal[4] = rr;
     c.ctl[0] = 1;
     c.ctl[1] = it;
-    if (error) c.ctl[2] = 1;
+    if (error) atomicMax(c.ctl + 2, 1);  // a time-out (2) of another CTA stays
   }
 }
 

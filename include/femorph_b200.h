@@ -487,10 +487,18 @@ FM_API int fm_poisson_destroy(fm_poisson* s);
 /* Preconditioned CG from x = 0 until ||r|| <= rel_tol ||b|| or max_iter
  * iterations; every reduction is summed in a fixed order, so the iterates
  * are the same from run to run.  FM_ERR_DIVERGED if the iteration breaks down
- * (a non-positive curvature or a NaN).  Device time of the solve in
- * *device_ms (may be NULL). */
+ * (a non-positive curvature or a NaN); the iterate it stopped at can be read.
+ * FM_ERR_TIMEOUT if a wait of the resident solver's blocks for one another
+ * gave up: the outputs are not written and there is no solution to read until
+ * another solve has run.  Device time of the solve in *device_ms (may be
+ * NULL). */
 FM_API int fm_poisson_solve(fm_poisson* s, double rel_tol, int32_t max_iter, int32_t* iterations,
                             double* rel_residual, double* device_ms);
+/* Polls after which such a wait gives up (default 4,194,304, a few seconds).
+ * A small limit (0: give up at once) makes the timeout path run on demand,
+ * which is how it is tested; 0 is not for production use.  Systems solved by
+ * one block, and those too large for the resident solver, have no such wait. */
+FM_API int fm_poisson_set_wait_limit(fm_poisson* s, uint32_t polls);
 /* The result fields: x (n_nodes; the average subtracted for
  * FM_POISSON_PPE) and, when cell_distance is non-NULL and the problem is
  * FM_POISSON_DISTANCE, the element wall distance (n_elems). */
