@@ -37,6 +37,7 @@ SYMBOLS = [
     "fm_batch_set_diagnostics", "fm_problem_vms_log", "fm_problem_vms_residuals",
     "fm_poisson_create", "fm_poisson_destroy", "fm_poisson_solve", "fm_poisson_get_solution", "fm_poisson_info", "fm_poisson_model",
     "fm_poisson_read_dat", "fm_poisson_write_vtk", "fm_problem_check_layout", "fm_poisson_set_wait_limit",
+    "fm_poisson_check_direction",
 ]
 
 FM_POISSON_CLASSIC, FM_POISSON_PPE, FM_POISSON_DISTANCE = 0, 1, 2
@@ -150,6 +151,7 @@ def lib():
         L.fm_poisson_destroy.argtypes = [P]
         L.fm_poisson_solve.argtypes = [P, C.c_double, C.c_int32, P, P, P]
         L.fm_poisson_set_wait_limit.argtypes = [P, C.c_uint32]
+        L.fm_poisson_check_direction.argtypes = [P, C.c_int32, P, P]
         L.fm_poisson_get_solution.argtypes = [P, P, P]
         L.fm_poisson_info.argtypes = [P, P, P]
         L.fm_poisson_model.argtypes = [P, P, P, P, P]
@@ -557,6 +559,12 @@ class GpuPoisson:
     def set_wait_limit(self, polls: int) -> None:
         """Polls of the resident solver's bounded waits before FM_ERR_TIMEOUT."""
         check(lib().fm_poisson_set_wait_limit(self.h, int(polls)))
+
+    def check_direction(self, iterations: int):
+        """(copies, differing) of the direction's halo copies (fm_poisson_check_direction)."""
+        n, d = C.c_int64(), C.c_int64()
+        check(lib().fm_poisson_check_direction(self.h, int(iterations), C.byref(n), C.byref(d)))
+        return int(n.value), int(d.value)
 
     @classmethod
     def read_dat(cls, path: str, device: int = 0):

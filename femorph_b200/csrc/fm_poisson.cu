@@ -457,6 +457,7 @@ struct fm_poisson {
   Cg c{};
   bool resident = false;  // solved by cg_resident_kernel over R (rows reordered)
   CgResident R{};
+  int64_t n_halo = 0;     // halo copies of all its blocks
   int32_t* row_of = nullptr;
   double* coords = nullptr;
   int32_t* conn = nullptr;
@@ -940,6 +941,7 @@ static int poisson_create(const fm_poisson_desc* d, int32_t device, fm_poisson**
   if (H.fits) {
     s->R = H.R;
     s->R.polls = kResPolls;
+    s->n_halo = (int64_t)H.halo.size();
     s->row_of = reinterpret_cast<int32_t*>(base + o_row_of);
     s->R.row0 = reinterpret_cast<int32_t*>(base + o_row0);
     s->R.halo0 = reinterpret_cast<int32_t*>(base + o_halo0);
@@ -1091,6 +1093,28 @@ FM_API int fm_poisson_solve(fm_poisson* s, double rel_tol, int32_t max_iter, int
 FM_API int fm_poisson_set_wait_limit(fm_poisson* s, uint32_t polls) {
   if (!s) return fail(FM_ERR_INVALID, "null solver");
   s->R.polls = polls;
+  return FM_OK;
+}
+
+FM_API int fm_poisson_check_direction(fm_poisson* s, int32_t iterations, int64_t* copies, int64_t* differing) {
+  if (!s || !copies || !differing || iterations < 1) return fail(FM_ERR_INVALID, "null argument or no iterations");
+  *copies = *differing = 0;
+  if (!s->resident || s->n_halo == 0) return FM_OK;
+  DeviceRestore restore;
+  PCK(cudaSetDevice(s->device));
+  const int64_t n = s->N + s->n_halo;
+  std::vector<double> seen(n);
+  std::vector<int32_t> halo(s->n_halo);
+  PCK(cudaMalloc(&s->R.seen, n * sizeof(double)));
+  int r = fm_poisson_solve(s, 0.0, iterations, nullptr, nullptr, nullptr);
+  cudaError_t e = cudaMemcpy(seen.data(), s->R.seen, n * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(halo.data(), s->R.halo, s->n_halo * sizeof(int32_t), cudaMemcpyDeviceToHost);
+  cudaFree(s->R.seen);
+  s->R.seen = nullptr;
+  if (r) return r;
+  PCK(e);
+  *copies = s->n_halo;
+  for (int64_t i = 0; i < s->n_halo; ++i) *differing += memcmp(&seen[s->N + i], &seen[halo[i]], sizeof(double)) != 0;
   return FM_OK;
 }
 

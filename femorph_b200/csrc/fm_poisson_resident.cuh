@@ -12,7 +12,10 @@
 // block as fits stays there too; two exchanges over the grid remain in an
 // iteration.  Each halo copy of the direction is updated with the same
 // arithmetic as its owner's, from the preconditioned residual z that the
-// owners write out, so z is all that crosses CTAs.
+// owners write out, so z is all that crosses CTAs.  (residual_z and
+// next_direction fix the roundings: left to the compiler, an owner's
+// D^-1 r + beta p may round beta p where a copy's z + beta p rounds z, and the
+// copies drift from their owners.)
 //
 // An exchange: every CTA writes its two partial sums into a table and adds
 // one to an arrival counter (release, which covers its z), one thread polls
@@ -59,6 +62,7 @@ struct CgResident {
   double2* partials;   // [2][ctas]
   unsigned long long* arrived;
   uint32_t polls;                         // an exchange's wait gives up after this many (kResPolls)
+  double* seen;                           // null, or where the last direction goes: the rows', then the halos' copies
   size_t smem;
 };
 
@@ -168,6 +172,9 @@ __device__ __forceinline__ void ahead(int n, LOAD load, USE use) {
   }
 }
 
+__device__ __forceinline__ double residual_z(double dinv, double r) { return __dmul_rn(dinv, r); }
+__device__ __forceinline__ double next_direction(double z, double beta, double p) { return __fma_rn(beta, p, z); }
+
 // VECTORS: how many of q, r, x, D^-1 (in this order) live in shared memory
 // beside p: 4, 2 or 0 (known at compile time, so that their accesses are
 // plain shared-memory ones).
@@ -204,7 +211,7 @@ __global__ void __launch_bounds__(THREADS, 1) cg_resident_kernel(Cg c, CgResiden
   // x = x0, r = b, z = D^-1 r
   double rz = 0.0, rr = 0.0;
   for (int i = tid; i < rows; i += THREADS) {
-    const double ri = c.b[r0 + i], di = c.dinv[r0 + i], zi = di * ri;
+    const double ri = c.b[r0 + i], di = c.dinv[r0 + i], zi = residual_z(di, ri);
     x[i] = c.xinit[r0 + i];
     r[i] = ri;
     if (VECTORS >= 4) dinv[i] = di;
@@ -223,16 +230,18 @@ __global__ void __launch_bounds__(THREADS, 1) cg_resident_kernel(Cg c, CgResiden
   while (!done) {
     // p = z + beta p, own rows and halo
     if (it == 0) {
-      for (int i = tid; i < rows; i += THREADS) p[i] = dinv[i] * r[i];
+      for (int i = tid; i < rows; i += THREADS) p[i] = residual_z(dinv[i], r[i]);
       for (int i = tid; i < nh; i += THREADS) p[rows + i] = __ldcg(c.z + halo[i]);
     } else {
       ahead<THREADS>(
-          nh, [&](int i) { return __ldcg(c.z + halo[i]); }, [&](int i, double z) { p[rows + i] = z + beta * p[rows + i]; });
+          nh, [&](int i) { return __ldcg(c.z + halo[i]); },
+          [&](int i, double z) { p[rows + i] = next_direction(z, beta, p[rows + i]); });
       if constexpr (VECTORS >= 4) {
-        for (int i = tid; i < rows; i += THREADS) p[i] = dinv[i] * r[i] + beta * p[i];
+        for (int i = tid; i < rows; i += THREADS) p[i] = next_direction(residual_z(dinv[i], r[i]), beta, p[i]);
       } else {
         ahead<THREADS>(
-            rows, [&](int i) { return dinv[i]; }, [&](int i, double d) { p[i] = d * r[i] + beta * p[i]; });
+            rows, [&](int i) { return dinv[i]; },
+            [&](int i, double d) { p[i] = next_direction(residual_z(d, r[i]), beta, p[i]); });
       }
     }
     __syncthreads();
@@ -260,7 +269,7 @@ __global__ void __launch_bounds__(THREADS, 1) cg_resident_kernel(Cg c, CgResiden
     rr = 0.0;
     auto update = [&](int i, double d) {
       const double ri = r[i] - alpha * q[i];
-      const double zi = d * ri;
+      const double zi = residual_z(d, ri);
       r[i] = ri;
       c.z[r0 + i] = zi;
       nrz += ri * zi;
@@ -292,6 +301,10 @@ __global__ void __launch_bounds__(THREADS, 1) cg_resident_kernel(Cg c, CgResiden
   }
   if (VECTORS >= 4)
     for (int i = tid; i < rows; i += THREADS) c.x[r0 + i] = x[i];
+  if (R.seen && it > 0) {
+    for (int i = tid; i < rows; i += THREADS) R.seen[r0 + i] = p[i];
+    for (int i = tid; i < nh; i += THREADS) R.seen[c.n + R.halo0[cta] + i] = p[rows + i];
+  }
   if (!ok && tid == 0) c.ctl[2] = 2;
   if (ok && cta == 0 && tid == 0) {
     c.scal[4] = rr;

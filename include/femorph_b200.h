@@ -499,6 +499,12 @@ FM_API int fm_poisson_solve(fm_poisson* s, double rel_tol, int32_t max_iter, int
  * which is how it is tested; 0 is not for production use.  Systems solved by
  * one block, and those too large for the resident solver, have no such wait. */
 FM_API int fm_poisson_set_wait_limit(fm_poisson* s, uint32_t polls);
+/* Self-check of the resident solver: runs `iterations` iterations, then
+ * counts the blocks' copies of other blocks' direction entries (*copies) and
+ * those whose bits are not the owner's (*differing: 0, as the product K p and
+ * p.K p are of one vector only then).  No copies for one block or a system
+ * too large for the resident solver.  Allocates; for tests. */
+FM_API int fm_poisson_check_direction(fm_poisson* s, int32_t iterations, int64_t* copies, int64_t* differing);
 /* The result fields: x (n_nodes; the average subtracted for
  * FM_POISSON_PPE) and, when cell_distance is non-NULL and the problem is
  * FM_POISSON_DISTANCE, the element wall distance (n_elems). */
