@@ -145,9 +145,11 @@ struct fm_problem {
   std::vector<double> tab_rows;    // rows x 4
   // Lumped mass (problem numbering): VMS N, SUPG N*3
   std::vector<double> mass;
-  // Prepared tile layout (fm_problem_prepare) and the tile sizes it was built for
+  // Prepared tile layout (fm_problem_prepare), the tile sizes it was asked for
+  // with, the most nodes a tile has under these, and the lower node limit it
+  // was cut by to fit the kernels' shared memory (0: none)
   std::shared_ptr<fm::Layout> layout;
-  int32_t layout_te = 0, layout_tn = 0;
+  int32_t layout_te = 0, layout_tn = 0, layout_most = 0, layout_cut = 0;
   // Partition part (fm_problem_partition): its index among n_parts, the
   // global node / element of each local one, and per local node its index
   // in the partition's exchange list (-1: the node is not shared)

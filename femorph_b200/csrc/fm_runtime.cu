@@ -327,31 +327,39 @@ static void default_tuning(int solver, int npe, int precision, fm_tuning& t) {
 static int prepare(fm_problem* p, const fm_tuning& t, std::shared_ptr<Layout>* out) {
   const int te = t.tile_elems > 0 ? t.tile_elems
                                   : auto_tile_elems(p->params.solver, p->etype, p->params.precision, t.threads, p->E);
-  int tn = t.tile_nodes;
-  if (p->layout && p->layout_te == te && p->layout_tn == tn) {
+  const int tn = t.tile_nodes;
+  // A caller's node limit may give tiles that the SUPG kernels' shared
+  // memory does not hold (tet4 2400 nodes, FP64 hexa8 with 256 threads
+  // 2943): those of up to 3200 nodes are cut smaller, larger ones are left
+  // to be refused when the batch is formed.
+  int fit = INT32_MAX;
+  if (p->params.solver == FM_SOLVER_SUPG) {
+    const bool mixed = p->params.precision == FM_MIXED;
+    const size_t base = supg_smem_bytes(0, p->etype, t.threads, mixed);
+    fit = (int)((227 * 1024 - 1024 - base) / (supg_smem_bytes(1, p->etype, t.threads, mixed) - base));
+  }
+  auto cut_for = [&](int most) { return most > fit && most <= 3200 ? fit : 0; };
+  // a layout asked for with the same sizes is kept where these threads would
+  // cut it the same way
+  const bool known = p->layout && p->layout_te == te && p->layout_tn == tn;
+  if (known && p->layout_cut == cut_for(p->layout_most)) {
     *out = p->layout;
     return FM_OK;
   }
   std::shared_ptr<Layout> L = std::make_shared<Layout>();
   fm_problem* arr[1] = {p};
-  int r = build_layout(arr, 1, te, tn, *L);
-  if (r) return r;
-  if (p->params.solver == FM_SOLVER_SUPG) {
-    // A caller's node limit may give tiles that the SUPG kernels' shared
-    // memory does not hold (tet4 2400 nodes, FP64 hexa8 with 256 threads
-    // 2943): those of up to 3200 nodes are cut smaller, larger ones are left
-    // to be refused when the batch is formed.
-    const bool mixed = p->params.precision == FM_MIXED;
-    const size_t base = supg_smem_bytes(0, p->etype, t.threads, mixed);
-    const int fit = (int)((227 * 1024 - 1024 - base) / (supg_smem_bytes(1, p->etype, t.threads, mixed) - base));
-    int most = 0;
+  int r = FM_OK, most = known ? p->layout_most : 0, cut = cut_for(most);
+  if (!cut) {
+    r = build_layout(arr, 1, te, tn, *L);
+    if (r) return r;
+    most = 0;
     for (const TileMeta& tm : L->tiles) most = std::max<int>(most, tm.n_node);
-    if (most > fit && most <= 3200) {
-      tn = fit;
-      L = std::make_shared<Layout>();
-      r = build_layout(arr, 1, te, tn, *L);
-      if (r) return r;
-    }
+    cut = cut_for(most);
+  }
+  if (cut) {
+    L = std::make_shared<Layout>();
+    r = build_layout(arr, 1, te, cut, *L);
+    if (r) return r;
   }
   if (p->params.precision == FM_MIXED) {
     // mixed form: elements whose Jacobian inverse stays in FP64 (aspect ratio
@@ -377,6 +385,8 @@ static int prepare(fm_problem* p, const fm_tuning& t, std::shared_ptr<Layout>* o
   p->layout = L;
   p->layout_te = te;
   p->layout_tn = tn;
+  p->layout_most = most;
+  p->layout_cut = cut;
   *out = L;
   return FM_OK;
 }
