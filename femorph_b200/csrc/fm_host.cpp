@@ -974,7 +974,8 @@ namespace fm {
 // (one problem, built by build_layout): local connectivity inside the tile's
 // node list; distinct nodes in a tile, interior ones touched by this tile
 // only; elements of one colour sharing no node (a warp adds up a colour
-// without ordering) and the marks of the colours' first elements; each
+// without ordering), the marks of the colours' first elements and those of
+// the hexas that repeat a node (their corners are added one by one); each
 // interface node's partial slots, one per touching tile, in tile order; every
 // element and node of the problem once.
 int check_layout(const fm_problem* p, const Layout& L) {
@@ -1035,12 +1036,22 @@ int check_layout(const fm_problem* p, const Layout& L) {
     if (co[0] != 0 || co[tm.n_col] != ne) return bad("tile " + std::to_string(t) + ": colour offsets");
     colour_stamp.assign(nl, -1);
     for (int32_t c = 0; c < tm.n_col; ++c)
-      for (int32_t i = co[c]; i < co[c + 1]; ++i)
+      for (int32_t i = co[c]; i < co[c + 1]; ++i) {
+        bool repeats = false;  // a node of this element
         for (int a = 0; a < npe; ++a) {
           const int32_t ln = cl[i * npe + a] & 0x7fff;
+          bool own = false;
+          for (int b = 0; b < a; ++b) own |= (cl[i * npe + b] & 0x7fff) == ln;
+          if (npe == 8 && own) {
+            repeats = true;
+            continue;
+          }
           if (colour_stamp[ln] == c) return bad("tile " + std::to_string(t) + ": two elements of a colour share a node");
           colour_stamp[ln] = c;
         }
+        if (npe == 8 && repeats != ((cl[i * npe + 2] & 0x8000) != 0))
+          return bad("tile " + std::to_string(t) + ": mark of a collapsed hexa");
+      }
     {
       // the marks of the colours' first elements (not needed on the tile's first)
       std::vector<char> first(ne, 0);

@@ -182,7 +182,8 @@ FM_API int fm_problem_prepare(fm_problem* p, const fm_tuning* tuning);
  * checks the invariants the tile kernels rely on: local connectivity inside
  * each tile's node list, interior nodes touched by one tile only, no two
  * elements of a colour sharing a node, the marks of the colours' first
- * elements, one partial slot per (tile, interface node) listed in tile order, every element and node once; for a
+ * elements and of the hexas that repeat a node, one partial slot per (tile,
+ * interface node) listed in tile order, every element and node once; for a
  * partition part (fm_problem_partition) also that shared nodes are interface
  * nodes carrying their exchange index.
  * FM_ERR_INVALID names the first broken one.  Host only.  No counterpart in
