@@ -649,9 +649,8 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             const int32_t n_node = li;
             // colouring (greedy, up to 128 colours)
             const int64_t ne = tile_start[t + 1] - tile_start[t];
-            used.assign(2 * (size_t)n_node, 0);
             col.resize(ne);
-            int ncol = 0;
+            int ncol = 0, csize[128];
             // A warp of the tile kernel adds up its 32 elements one colour
             // after another, so colours hold at most 32 elements, and a tile
             // of enough warps (a node has up to 24 tets or 8 hexa, hence as
@@ -663,51 +662,64 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             // order.  Its FP32 element work turns the last bit of a nodal sum
             // into an FP32 rounding now and then, which travels to the pressure
             // as 1e-8 of it: the sums keep this one order.)
-            const bool ordered = !vms && p->params.precision == FM_MIXED;
+            bool ordered = !vms && p->params.precision == FM_MIXED;
             const int nwarp = (int)((ne + 31) / 32);
-            const int even = !ordered && nwarp >= (npe == 4 ? 26 : 10) && nwarp <= 64 ? nwarp : 0;
-            uint64_t level[33] = {0};  // colours below `even` by their size
-            level[0] = even == 64 ? ~0ULL : (1ULL << even) - 1;
-            int csize[128] = {0};
-            uint64_t full0 = 0, full1 = 0;  // colours with 32 elements
-            for (int64_t i = 0; i < ne; ++i) {
-              const int32_t* c = &cs[(size_t)(tile_start[t] + i) * npe];
-              uint64_t m0 = full0, m1 = full1;
-              for (int a = 0; a < npe; ++a) {
-                m0 |= used[2 * local[c[a]]];
-                m1 |= used[2 * local[c[a]] + 1];
-              }
-              int k = -1;
-              for (int q = 0; even && q < 32; ++q)
-                if (level[q] & ~m0) {
-                  k = __builtin_ctzll(level[q] & ~m0);
-                  level[q] &= ~(1ULL << k);
-                  level[q + 1] |= 1ULL << k;
-                  break;
-                }
-              if (k >= 0) {
-              } else if (~m0) k = __builtin_ctzll(~m0);
-              else if (~m1) k = 64 + __builtin_ctzll(~m1);
-              else {
-                // every colour full or taken: past the limit of 32 instead
-                m0 = m1 = 0;
+            auto colour = [&]() -> bool {
+              used.assign(2 * (size_t)n_node, 0);
+              std::fill(csize, csize + 128, 0);
+              ncol = 0;
+              const int even = !ordered && nwarp >= (npe == 4 ? 26 : 10) && nwarp <= 64 ? nwarp : 0;
+              uint64_t level[33] = {0};  // colours below `even` by their size
+              level[0] = even == 64 ? ~0ULL : (1ULL << even) - 1;
+              uint64_t full0 = 0, full1 = 0;  // colours with 32 elements
+              for (int64_t i = 0; i < ne; ++i) {
+                const int32_t* c = &cs[(size_t)(tile_start[t] + i) * npe];
+                uint64_t m0 = full0, m1 = full1;
                 for (int a = 0; a < npe; ++a) {
                   m0 |= used[2 * local[c[a]]];
                   m1 |= used[2 * local[c[a]] + 1];
                 }
-                if (~m0) k = __builtin_ctzll(~m0);
+                int k = -1;
+                for (int q = 0; even && q < 32; ++q)
+                  if (level[q] & ~m0) {
+                    k = __builtin_ctzll(level[q] & ~m0);
+                    level[q] &= ~(1ULL << k);
+                    level[q + 1] |= 1ULL << k;
+                    break;
+                  }
+                if (k >= 0) {
+                } else if (~m0) k = __builtin_ctzll(~m0);
                 else if (~m1) k = 64 + __builtin_ctzll(~m1);
                 else {
-                  W.err = 1;
-                  break;
+                  // every colour full or taken: past the limit of 32 instead
+                  m0 = m1 = 0;
+                  for (int a = 0; a < npe; ++a) {
+                    m0 |= used[2 * local[c[a]]];
+                    m1 |= used[2 * local[c[a]] + 1];
+                  }
+                  if (~m0) k = __builtin_ctzll(~m0);
+                  else if (~m1) k = 64 + __builtin_ctzll(~m1);
+                  else return false;
                 }
+                if (++csize[k] >= 32 && !ordered) (k < 64 ? full0 : full1) |= 1ULL << (k & 63);
+                col[i] = k;
+                ncol = std::max(ncol, k + 1);
+                for (int a = 0; a < npe; ++a) used[2 * local[c[a]] + (k >> 6)] |= (1ULL << (k & 63));
               }
-              if (++csize[k] >= 32 && !ordered) (k < 64 ? full0 : full1) |= 1ULL << (k & 63);
-              col[i] = k;
-              ncol = std::max(ncol, k + 1);
-              for (int a = 0; a < npe; ++a) used[2 * local[c[a]] + (k >> 6)] |= (1ULL << (k & 63));
+              return true;
+            };
+            // Spread over many colours, the elements around a few nodes of a
+            // hundred tets each can leave none for the last of them: such a
+            // tile takes the smallest colour that fits throughout.
+            bool fits = colour();
+            if (!fits && !ordered) {
+              ordered = true;
+              fits = colour();
             }
-            if (W.err) continue;
+            if (!fits) {
+              W.err = 1;
+              continue;
+            }
             if (!ordered) {
               // the largest colours first: they fill whole warps
               int by[128], at[128], n = 0;
