@@ -150,6 +150,8 @@ struct fm_problem {
   // was cut by to fit the kernels' shared memory (0: none)
   std::shared_ptr<fm::Layout> layout;
   int32_t layout_te = 0, layout_tn = 0, layout_most = 0, layout_cut = 0;
+  // Layout of full tiles (fm_vms_solve_static, where the prepared one is too large)
+  std::shared_ptr<fm::Layout> layout_full;
   // Partition part (fm_problem_partition): its index among n_parts, the
   // global node / element of each local one, and per local node its index
   // in the partition's exchange list (-1: the node is not shared)

@@ -203,15 +203,19 @@ extern "C" int fm_vms_solve_static(fm_problem* p, int32_t nsteps, int32_t device
   if (!p->layout) return fail(FM_ERR_INVALID, "call fm_problem_prepare before fm_vms_solve_static");
   if (p->part >= 0) return fail(FM_ERR_INVALID, "fm_vms_solve_static does not run partition parts");
   // the prepared layout, or full tiles where its small ones (more interface
-  // partials) would not fit
-  std::shared_ptr<Layout> full;
+  // partials) would not fit: built once and kept with the problem, and not
+  // for one whose nodes and elements alone are too large
   const Layout* pl = p->layout.get();
-  if (plan(p, *pl).total > (size_t)FM_STATIC_SCRATCH_BYTES) {
-    fm_problem* arr[1] = {p};
-    full = std::make_shared<Layout>();
-    const int lr = build_layout(arr, 1, 1024, FM_MAX_TILE_NODES, *full);
-    if (lr) return lr;
-    if (plan(p, *full).total < plan(p, *pl).total) pl = full.get();
+  const size_t least = (size_t)p->N * 12 * sizeof(double) + (size_t)p->E * (12 * sizeof(double) + 4 * sizeof(uint16_t));
+  if (plan(p, *pl).total > (size_t)FM_STATIC_SCRATCH_BYTES && least <= (size_t)FM_STATIC_SCRATCH_BYTES) {
+    if (!p->layout_full) {
+      fm_problem* arr[1] = {p};
+      std::shared_ptr<Layout> full = std::make_shared<Layout>();
+      const int lr = build_layout(arr, 1, 1024, FM_MAX_TILE_NODES, *full);
+      if (lr) return lr;
+      p->layout_full = full;
+    }
+    if (plan(p, *p->layout_full).total < plan(p, *pl).total) pl = p->layout_full.get();
   }
   const Layout& L = *pl;
   const Offsets o = plan(p, L);
