@@ -529,6 +529,10 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
     greedy_tiles(cs.data(), npe, E, TE, TN, tile_start);
     tile_start.push_back(E);
     const int ntile = (int)tile_start.size() - 1;
+    // host threads of the short passes by the work, in full tiles (24,576 tets
+    // in tiles of 256: starting more of them took 0.7 of 5.4 ms)
+    const int64_t full = std::max<int64_t>(1, std::min<int64_t>(ntile, E / (npe == 8 ? 384 : 1024)));
+    auto grain = [&](int64_t tiles) { return (tiles * ntile + full - 1) / full; };
     // 3. node tile counts and first tile (shared partition nodes count as
     // touched by two tiles), tiles split over the host threads
     std::vector<int32_t> ntiles(N, 0), first_tile(N, INT32_MAX);
@@ -550,7 +554,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
         }
         set.clear();
       }
-    }, 64);
+    }, grain(64));
     if (!p->xidx.empty())
       for (int64_t i = 0; i < N; ++i)
         if (p->xidx[i] >= 0 && ntiles[i] == 1) ntiles[i] = 2;
@@ -558,7 +562,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
     // them, each group in order of first touch along the sorted elements
     // (per-tile first-touch lists in parallel, then prefix offsets)
     const int64_t hwt = std::max<int64_t>(1, std::min<int64_t>(32, std::thread::hardware_concurrency()));
-    const int64_t nwk = std::min<int64_t>(hwt, std::max<int64_t>(1, ntile / 4));
+    const int64_t nwk = std::min<int64_t>(hwt, std::max<int64_t>(1, full / 4));
     std::vector<std::vector<int32_t>> first_int(ntile), first_ifc(ntile);
     {
       std::vector<std::thread> th;
@@ -595,7 +599,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
         k = node_base + iface_begin + ifc_at[t];
         for (int32_t v : first_ifc[t]) nn[v] = (int32_t)k++;
       }
-    }, 16);
+    }, grain(16));
     std::vector<std::vector<int32_t>>().swap(first_int);
     std::vector<std::vector<int32_t>>().swap(first_ifc);
     int64_t next = iface_begin + ifc_at[ntile];
@@ -671,6 +675,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
               const int even = !ordered && nwarp >= (npe == 4 ? 26 : 10) && nwarp <= 64 ? nwarp : 0;
               uint64_t level[33] = {0};  // colours below `even` by their size
               level[0] = even == 64 ? ~0ULL : (1ULL << even) - 1;
+              int low = 0;  // no colour is smaller (sizes only grow)
               uint64_t full0 = 0, full1 = 0;  // colours with 32 elements
               for (int64_t i = 0; i < ne; ++i) {
                 const int32_t* c = &cs[(size_t)(tile_start[t] + i) * npe];
@@ -680,7 +685,8 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
                   m1 |= used[2 * local[c[a]] + 1];
                 }
                 int k = -1;
-                for (int q = 0; even && q < 32; ++q)
+                while (low < 32 && !level[low]) ++low;
+                for (int q = even ? low : 32; q < 32; ++q)
                   if (level[q] & ~m0) {
                     k = __builtin_ctzll(level[q] & ~m0);
                     level[q] &= ~(1ULL << k);
@@ -761,9 +767,10 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             // 119 -> 116, 1.05 M hexas 348 -> 337, 1.57 M SUPG tets 119.5 ->
             // 117.2.  (The nodes with the most elements first: fewer conflicts,
             // but the lists of interface nodes lose their order, 475 and 341.)
-            // taken: 4 bits a bank group.
+            // taken: a byte a bank group, one or two words a lane group and
+            // corner, so that a node's counts are sums of whole words.
             {
-              const int G = vms ? 8 : 16;
+              const int G = vms ? 8 : 16, lg = vms ? 3 : 4, words = G / 8;
               const int n_int = (int)W.inter.size();
               cnt.assign(n_node + 1, 0);
               for (int64_t i = 0; i < ne * npe; ++i) cnt[W.conn[i] + 1]++;
@@ -771,25 +778,46 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
               inc.resize((size_t)ne * npe);
               pos.assign(cnt.begin(), cnt.end() - 1);
               for (int64_t i = 0; i < ne; ++i)
-                for (int a = 0; a < npe; ++a) inc[pos[W.conn[i * npe + a]]++] = (int32_t)(i / G * npe + a);
-              taken.assign((size_t)((ne + G - 1) / G) * npe, 0);
+                for (int a = 0; a < npe; ++a) inc[pos[W.conn[i * npe + a]]++] = (int32_t)(((i >> lg) * npe + a) * words);
+              taken.assign((size_t)((ne + G - 1) / G) * npe * words, 0);
               place.resize(n_node);
               moved.resize(n_node);
               for (int part = 0; part < 2; ++part) {
                 const int lo = part ? n_int : 0, hi = part ? n_node : n_int;
-                int next[16];  // the next free local id of each bank group
-                for (int k = 0; k < G; ++k) next[k] = lo + ((k - lo) % G + G) % G;
+                uint32_t next[16];  // the next free local id of each bank group, or kNone
+                constexpr uint32_t kNone = 1u << 31;
+                for (int k = 0; k < G; ++k) {
+                  next[k] = (uint32_t)(lo + ((k - lo) % G + G) % G);
+                  if ((int)next[k] >= hi) next[k] = kNone;
+                }
                 for (int v = lo; v < hi; ++v) {
-                  int hits[16] = {0};
-                  for (int32_t q = cnt[v]; q < cnt[v + 1]; ++q)
-                    for (int k = 0; k < G; ++k) hits[k] += (int)((taken[inc[q]] >> (4 * k)) & 15);
-                  int best = -1;
-                  for (int k = 0; k < G; ++k)
-                    if (next[k] < hi && (best < 0 || hits[k] < hits[best] || (hits[k] == hits[best] && next[k] < next[best])))
-                      best = k;
-                  place[v] = next[best];
-                  next[best] += G;
-                  for (int32_t q = cnt[v]; q < cnt[v + 1]; ++q) taken[inc[q]] += 1ULL << (4 * best);
+                  uint32_t hits[16] = {0};
+                  for (int32_t q = cnt[v]; q < cnt[v + 1];) {
+                    // at most G lanes a byte: 15 entries stay below 256
+                    const int32_t to = std::min(q + 15, cnt[v + 1]);
+                    uint64_t w0 = 0, w1 = 0;
+                    for (; q < to; ++q) {
+                      w0 += taken[inc[q]];
+                      if (words == 2) w1 += taken[inc[q] + 1];
+                    }
+                    for (int k = 0; k < 8; ++k) hits[k] += (uint32_t)((w0 >> (8 * k)) & 255);
+                    if (words == 2)
+                      for (int k = 0; k < 8; ++k) hits[8 + k] += (uint32_t)((w1 >> (8 * k)) & 255);
+                  }
+                  // the fewest hits, of those the lowest id: a node has at
+                  // most 128 elements here (a colour each), eight corners
+                  // each, hence fewer than 2^15 hits; ids are below 2^16
+                  uint32_t key = UINT32_MAX;
+                  int best = 0;
+                  for (int k = 0; k < G; ++k) {
+                    const uint32_t kk = (hits[k] << 16) + next[k];
+                    best = kk < key ? k : best;
+                    key = kk < key ? kk : key;
+                  }
+                  place[v] = (int32_t)next[best];
+                  next[best] += (uint32_t)G;
+                  if ((int)next[best] >= hi) next[best] = kNone;
+                  for (int32_t q = cnt[v]; q < cnt[v + 1]; ++q) taken[inc[q] + (best >> 3)] += 1ULL << (8 * (best & 7));
                 }
                 std::vector<int32_t>& list = part ? W.ifc : W.inter;
                 for (int v = lo; v < hi; ++v) moved[place[v] - lo] = list[v - lo];
@@ -812,6 +840,9 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             if (npe == 8)
               for (int64_t i = 0; i < ne; ++i) {
                 const uint16_t* c = &W.conn[(size_t)i * 8];
+                uint64_t seen = 0;  // eight bits: eight nodes
+                for (int a = 0; a < 8; ++a) seen |= 1ULL << (c[a] & 63);
+                if (__builtin_popcountll(seen) == 8) continue;
                 bool same = false;
                 for (int a = 0; a < 8; ++a)
                   for (int b = 0; b < a; ++b) same |= (c[a] & 0x7fff) == (c[b] & 0x7fff);
@@ -884,7 +915,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
         std::copy(W.eo.begin(), W.eo.end(), eo.begin() + (tm.elem_begin - elem_base));
         std::fill(eo.begin() + (tm.elem_begin - elem_base) + tm.n_elem, eo.begin() + eo_next, -1);
       }
-    }, 8);
+    }, grain(8));
     if (ntile == 0) {
       std::fill(L.conn_local.begin() + (size_t)elem_base * npe, L.conn_local.end(), 0);
       std::fill(eo.begin(), eo.end(), -1);
@@ -896,7 +927,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
     {
       const int64_t NI = N - iface_begin;
       const int64_t hw2 = std::max<int64_t>(1, std::min<int64_t>(32, std::thread::hardware_concurrency()));
-      const int64_t nw = std::min<int64_t>(hw2, std::max<int64_t>(1, ntile / 64));
+      const int64_t nw = std::min<int64_t>(hw2, std::max<int64_t>(1, full / 64));
       std::vector<std::vector<int32_t>> wc(nw);
       auto node_of = [&](int32_t v) { return (int64_t)nn[v] - node_base - iface_begin; };
       {
