@@ -416,11 +416,14 @@ FM_API int fm_batch_profile(fm_batch* b, int32_t nsteps, double* kernel_ms, int6
 
 /* Autotuner: times the tile/interface kernels of these problems (as one
  * batch, `steps` steps per candidate, per-kernel CUDA events) over the
- * candidate launch shapes (tile elements x threads per CTA) and writes the
- * fastest to *best.  With cache_path non-NULL the result is looked up first
- * and stored afterwards, keyed by GPU name, solver, element type, precision
- * and the batch's element count (rounded to a power of two).  The problems
- * must not be in a batch; their host data is not modified. */
+ * candidate launch shapes (the default, then tile elements x threads per
+ * CTA) and writes the fastest to *best (tile_elems 0 and tile_nodes 0: the
+ * default by each problem's size).  With cache_path non-NULL the result is
+ * looked up first and stored afterwards, keyed by GPU name, solver, element
+ * type, precision and the batch's element count (rounded to a power of two).
+ * A line of an earlier build is taken as it is, though this build's fastest
+ * shape may be another: delete the file to time anew.  The problems must not
+ * be in a batch; their host data is not modified. */
 FM_API int fm_autotune(fm_problem* const* problems, int32_t n, int32_t device, int32_t steps, const char* cache_path,
                        fm_tuning* best);
 
