@@ -118,6 +118,7 @@ def lib():
         L.fm_batch_set_diagnostics.argtypes = [P, C.c_int32]
         L.fm_batch_set_wait_limit.argtypes = [P, C.c_uint32]
         L.fm_math_check.argtypes = [P, C.c_int64, P]
+        L.fm_math_check_rsqrt.argtypes = [P, C.c_int64, P]
         L.fm_problem_vms_log.argtypes = [P, P, C.c_int32, P]
         L.fm_problem_vms_residuals.argtypes = [P, P, P]
         L.fm_problem_restore.argtypes = [P, C.c_char_p]

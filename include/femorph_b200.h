@@ -342,6 +342,8 @@ FM_API int fm_batch_set_wait_limit(fm_batch* b, uint32_t polls);
  * sqrt(x), rcbrt_nr((float)x), rcbrtf((float)x), computed on device 0
  * (allocates; for tests). */
 FM_API int fm_math_check(const double* x, int64_t n, double* out);
+/* The same for the SUPG kernels' inverse square root: out[i] = rsqrt_nr(x[i]). */
+FM_API int fm_math_check_rsqrt(const double* x, int64_t n, double* out);
 FM_API int fm_problem_vms_log(fm_problem* p, double* rows, int32_t max_rows, int32_t* n_rows);
 FM_API int fm_problem_vms_residuals(fm_problem* p, double* res_u, double* res_p);
 
