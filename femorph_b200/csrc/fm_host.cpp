@@ -613,7 +613,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
       std::vector<uint16_t> conn;       // ne x npe tile-local ids
       std::vector<int32_t> colcnt;      // colour offsets (ncol + 1)
       int ncol = 0;
-      int err = 0;                      // 1: > 128 colours, 2: 16-bit corner count overflow
+      int err = 0;                      // 1: > 128 colours, 2: > FM_MAX_TILE_CORNERS
     };
     std::vector<TileWork> tw(ntile);
     {
@@ -653,6 +653,10 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
             const int32_t n_node = li;
             // colouring (greedy, up to 128 colours)
             const int64_t ne = tile_start[t + 1] - tile_start[t];
+            if (ne * npe > FM_MAX_TILE_CORNERS) {
+              W.err = 2;
+              continue;
+            }
             col.resize(ne);
             int ncol = 0, csize[128];
             // A warp of the tile kernel adds up its 32 elements one colour
@@ -825,11 +829,6 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
               }
               for (int64_t i = 0; i < ne * npe; ++i) W.conn[i] = (uint16_t)place[W.conn[i]];
             }
-            // entries of a tile are counted in 16 bits
-            if (ne * npe > 65535) {
-              W.err = 2;
-              continue;
-            }
             // bit 15 of an element's second node id marks the first
             // element of a colour (the tile kernel's warps add up one colour
             // after another)
@@ -854,7 +853,7 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
     }
     for (int t = 0; t < ntile; ++t) {
       if (tw[t].err == 1) return fail(FM_ERR_INVALID, "element colouring needs more than 128 colours in one tile");
-      if (tw[t].err == 2) return fail(FM_ERR_INVALID, "tile_elems too large for 16-bit incidence entries");
+      if (tw[t].err == 2) return fail(FM_ERR_INVALID, "tile_elems too large: more than 65535 corners in a tile");
     }
     // placement: every tile starts at a multiple of ELEM_ALIGN element slots
     // (padding slots in between are never processed, so each chunk of a
@@ -883,7 +882,6 @@ int build_layout(fm_problem* const* probs, int n, int TE, int TN, Layout& L) {
         sb += (int64_t)W.ifc.size();
         col_off += (int64_t)W.colcnt.size();
         L.max_colors = std::max(L.max_colors, W.ncol);
-        L.max_tile_elems = std::max<int32_t>(L.max_tile_elems, tm.n_elem);
       }
       // final sizes at once (the last problem includes the trailing
       // padding: chunk copies round their length up to 16 bytes); the new

@@ -198,7 +198,6 @@ struct Layout {
   std::vector<TileMeta> tiles;
   hvec<int32_t> tile_nodes;
   std::vector<int32_t> tile_cols;
-  int32_t max_tile_elems = 0;
   hvec<uint16_t> conn_local;          // n_elems x npe
   std::vector<int32_t> iface_node, iface_slot_beg, iface_slots, iface_prob;
   std::vector<int32_t> iface_xidx;    // exchange index of each interface node (-1: none); partition parts only
@@ -216,6 +215,10 @@ constexpr int ELEM_ALIGN = 32;
 // SUPG hexa8 FP64: stored geometry values per Gauss point (inverse Jacobian
 // and det J), 8 points an element.
 constexpr int FM_GEO_PER_GP = 10;
+// A tile's elements x corners.  No kernel depends on it (their limit is the
+// nodes that shared memory holds); shapes beyond it have always been refused
+// and stay so.
+constexpr int64_t FM_MAX_TILE_CORNERS = 65535;
 // VMS tiles: at most this many nodes (the shared memory of a CTA's
 // accumulators).
 #define FM_MAX_TILE_NODES 512

@@ -447,7 +447,7 @@ __global__ void supg_pressure_kernel(DevBatch B, int tn_max, double* pres) {
   for (int le = threadIdx.x; le < tm.n_elem; le += blockDim.x) {
     const int64_t e = tm.elem_begin + le;
     int ln[NPE];
-    for (int a = 0; a < NPE; ++a) ln[a] = B.conn[e * NPE + a] & 0x7fff;  // bit 15: mixed-form flag
+    for (int a = 0; a < NPE; ++a) ln[a] = B.conn[e * NPE + a] & 0x7fff;  // bit 15 of the first three: marks (supg_geo_kernel)
     double num = 0.0, den = 0.0;
     for (int g = 0; g < GaussRule<NPE>::n; ++g) {
       double q[3], Nf[NPE], dN[NPE][3], inv[3][3];
@@ -506,12 +506,11 @@ static cudaError_t raise_tile_smem(int optin) {
 // maximum (the attribute is per kernel and process-wide, so a batch with
 // small tiles must not lower it below what another batch launches with; the
 // shared-memory carve-out still follows each launch's actual size).
-cudaError_t supg_configure(size_t smem, int npe) {
+cudaError_t supg_configure(int npe) {
   int dev = 0, optin = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  (void)smem;  // checked against the limit by the caller
   if (npe == 4) {
     e = raise_tile_smem<4>(optin);
     if (e == cudaSuccess) e = raise_dyn_smem(supg_pressure_kernel<4>, optin);

@@ -40,7 +40,7 @@ cudaError_t launch_vms_diagnostics(const DevBatch& B, const double* cres_buf, co
                                    int32_t n_nodes, const int32_t* eo, int64_t eb, int64_t ec, int64_t nb,
                                    double* el, double* out, int blocks, cudaStream_t s);
 size_t supg_smem_bytes(int tn_max, int npe, int threads, bool mixed);
-cudaError_t supg_configure(size_t smem, int npe);
+cudaError_t supg_configure(int npe);
 cudaError_t launch_supg_step(const DevBatch& B, int tn_max, int threads, int iface_blocks, int npe, bool mixed,
                              bool xpack, cudaStream_t s, cudaEvent_t* ev);
 cudaError_t launch_supg_xupdate(const DevBatch& B, int blocks, cudaStream_t s);
@@ -548,7 +548,7 @@ static int configure(fm_batch* b) {
                                            : supg_smem_bytes(tn, b->npe, b->threads, b->precision == FM_MIXED);
   // 227 KB opt-in limit per block, less room for the kernels' static shared memory
   if (smem + 1024 > 227 * 1024) return fail(FM_ERR_INVALID, "tile too large for shared memory; lower tile_nodes");
-  cudaError_t ce = b->solver == FM_SOLVER_VMS ? vms_configure() : supg_configure(smem, b->npe);
+  cudaError_t ce = b->solver == FM_SOLVER_VMS ? vms_configure() : supg_configure(b->npe);
   if (ce != cudaSuccess) return fail(FM_ERR_CUDA, std::string("kernel attribute: ") + cudaGetErrorString(ce));
   b->configured_tn = tn;
   return FM_OK;
