@@ -345,6 +345,7 @@ void build_resident(const double* coords, int64_t N, const std::vector<int32_t>&
                     size_t smem_limit, ResidentHost& H) {
   CgResident& R = H.R;
   const int G = N <= kResOne ? 1 : (int)std::min<int64_t>(sms, N / kResRows);
+  if ((size_t)(N / G) * 8 > smem_limit) return;
   R.ctas = G;
   R.threads = N / G > kResWide ? 1024 : 512;
   fm::morton_order_nodes(coords, N, H.node_of);
@@ -366,9 +367,12 @@ void build_resident(const double* coords, int64_t N, const std::vector<int32_t>&
     for (int64_t i = H.row0[g]; i < H.row0[g + 1]; ++i) H.row_of[H.node_of[i]] = (int32_t)i;
   });
   // each block's halo (its columns outside it, through a small open-addressing
-  // map) and its entries' local columns
+  // map) and its entries' local columns; once a block does not fit, the others
+  // are not formed
   std::vector<std::vector<uint16_t>> local(G);
+  std::atomic<bool> over_limit{false};
   over([&](int g) {
+    if (over_limit) return;
     const int32_t a = H.row0[g], b = H.row0[g + 1];
     std::vector<int32_t>& h = hal[g];
     std::vector<int32_t> key(1024, -1), id(1024);
@@ -397,8 +401,9 @@ void build_resident(const double* coords, int64_t N, const std::vector<int32_t>&
         }
         uint32_t q = slot(w);
         if (key[q] < 0) {
-          if (b - a + (int64_t)h.size() >= 65536) {  // does not fit (below)
-            h.push_back(w);
+          const size_t m = h.size() + 1;  // the direction and the halo's row numbers
+          if (b - a + m > 65536 || (b - a + m) * 8 + m * 4 > smem_limit) {
+            over_limit = true;
             return;
           }
           if (2 * (h.size() + 1) > mask) {
@@ -427,6 +432,7 @@ void build_resident(const double* coords, int64_t N, const std::vector<int32_t>&
     for (uint16_t& c : lc)
       if (c >= b - a) c = rank[c - (b - a)];
   });
+  if (over_limit) return;
   H.halo0.assign(G + 1, 0);
   H.slice0.assign(G + 1, 0);
   int64_t hsum = 0;
