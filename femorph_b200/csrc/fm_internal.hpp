@@ -4,6 +4,7 @@
 #include <memory>
 #include <new>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <type_traits>
 #include <utility>
@@ -62,8 +63,15 @@ inline void parallel_blocks(int64_t n, F f, int64_t grain = 4096) {
     return;
   }
   std::vector<std::thread> th;
-  for (int64_t t = 0; t < nt; ++t)
-    th.emplace_back([&, t] { f(n * t / nt, n * (t + 1) / nt, (int)t); });
+  th.reserve(nt);
+  for (int64_t t = 0; t < nt; ++t) {
+    auto part = [&f, n, nt, t] { f(n * t / nt, n * (t + 1) / nt, (int)t); };
+    try {
+      th.emplace_back(part);
+    } catch (const std::system_error&) {  // no thread to be had: on this one
+      part();
+    }
+  }
   for (auto& x : th) x.join();
 }
 

@@ -942,13 +942,10 @@ static void touch_pages(void* p, size_t bytes) {
   constexpr size_t page = 4096, each = 1 << 21;
   const size_t nt = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), bytes / each});
   if (nt < 2) return;
-  std::vector<std::thread> th;
-  for (size_t t = 0; t < nt; ++t)
-    th.emplace_back([=] {
-      volatile char* q = static_cast<char*>(p);
-      for (size_t i = bytes * t / nt; i < bytes * (t + 1) / nt; i += page) q[i] = q[i];
-    });
-  for (auto& x : th) x.join();
+  parallel_blocks((int64_t)nt, [&](int64_t t0, int64_t t1, int) {
+    volatile char* q = static_cast<char*>(p);
+    for (size_t i = bytes * t0 / nt; i < bytes * t1 / nt; i += page) q[i] = q[i];
+  }, 1);
 }
 
 extern "C" {
