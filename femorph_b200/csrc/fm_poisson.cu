@@ -1104,8 +1104,14 @@ FM_API int fm_poisson_check_direction(fm_poisson* s, int32_t iterations, int64_t
   DeviceRestore restore;
   PCK(cudaSetDevice(s->device));
   const int64_t n = s->N + s->n_halo;
-  std::vector<double> seen(n);
-  std::vector<int32_t> halo(s->n_halo);
+  std::vector<double> seen;
+  std::vector<int32_t> halo;
+  try {
+    seen.resize(n);
+    halo.resize(s->n_halo);
+  } catch (const std::bad_alloc&) {
+    return fail(FM_ERR_OOM, "host allocation failed");
+  }
   PCK(cudaMalloc(&s->R.seen, n * sizeof(double)));
   int r = fm_poisson_solve(s, 0.0, iterations, nullptr, nullptr, nullptr);
   cudaError_t e = cudaMemcpy(seen.data(), s->R.seen, n * sizeof(double), cudaMemcpyDeviceToHost);

@@ -209,11 +209,15 @@ extern "C" int fm_vms_solve_static(fm_problem* p, int32_t nsteps, int32_t device
   const size_t least = (size_t)p->N * 12 * sizeof(double) + (size_t)p->E * (12 * sizeof(double) + 4 * sizeof(uint16_t));
   if (plan(p, *pl).total > (size_t)FM_STATIC_SCRATCH_BYTES && least <= (size_t)FM_STATIC_SCRATCH_BYTES) {
     if (!p->layout_full) {
-      fm_problem* arr[1] = {p};
-      std::shared_ptr<Layout> full = std::make_shared<Layout>();
-      const int lr = build_layout(arr, 1, 1024, FM_MAX_TILE_NODES, *full);
-      if (lr) return lr;
-      p->layout_full = full;
+      try {
+        fm_problem* arr[1] = {p};
+        std::shared_ptr<Layout> full = std::make_shared<Layout>();
+        const int lr = build_layout(arr, 1, 1024, FM_MAX_TILE_NODES, *full);
+        if (lr) return lr;
+        p->layout_full = full;
+      } catch (const std::bad_alloc&) {
+        return fail(FM_ERR_OOM, "host allocation failed while building the tile layout");
+      }
     }
     if (plan(p, *p->layout_full).total < plan(p, *pl).total) pl = p->layout_full.get();
   }
